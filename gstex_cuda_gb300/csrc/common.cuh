@@ -146,38 +146,58 @@ struct RecCold {  // the backward's ray terms and the blur adjoint
 };
 constexpr int kRecBytes = sizeof(RecHot) + sizeof(RecWarm) + sizeof(RecCold);
 
-// The four edges of the projected alpha >= 1/255 rectangle (a convex quad
-// inside the screen box): a pixel centre (x, y) can only meet the splat where
-// A.k x + B.k y + C.k >= 0 for every edge k (pixel units, with a margin).
-// Used by the backward's candidate lists; all-pass (A = B = 0, C = 1) where
-// the box is infinite, with blur, or for a degenerate edge.
-struct RecEdge {
-    float4 A, B, C;
+// The alpha >= 1/255 region of a splat as pixel rows see it: at height y, with
+// u = (y - yc) / hy, the region lies inside xc + m (y - yc) +- s sqrt(1 - u^2)
+// (an ellipse) or xc +- s (a box), and only rows with |u| <= 1 meet it.  The
+// image of the ellipse sigma <= ln(255 opacity) is an ellipse when the splat's
+// rectangle is in front of the camera; where that form does not apply (an
+// infinite screen box, blur, a strong perspective) the screen box takes its
+// place, and a region that no pixel meets has s < 0.  16 bytes, one load: s
+// and 1 / hy are rounded to bfloat16 such that the region only grows; m, whose
+// error would move a sliver's ends sideways, keeps all but its last bit.
+struct RecCull {
+    float xc, yc;
+    uint32_t ms;  // m (upper half), s
+    uint32_t hk;  // 1 / hy, m (lower half but for its last bit), 1 for an ellipse
 };
-constexpr int kEdgeBytes = sizeof(RecEdge);
 
-// One (view, Gaussian) record as the batched path stores it in device memory:
-// built once per view by the record kernel (where the near-edge-on solve runs
-// in double), then copied into shared memory by every tile the splat touches.
-struct __align__(16) RecAll {
-    RecHot h;
-    RecWarm w;
-    RecCold c;
-    RecEdge e;
+// One (view, Gaussian) record as it is stored in device memory: built once per
+// view by the record kernel (where the near-edge-on solve runs in double), then
+// read by every tile the splat touches.  224 bytes, in 16-byte chunks ordered
+// by who reads them, so that each reader takes whole 32-byte sectors: the cull
+// test chunk 0, the block kernels' forward 2-8 and backward 2-9.
+enum RecChunk {
+    kChunkCull = 0,   // RecCull (chunk 1 is unused)
+    kChunkOrg = 2,    // px0, py0, g (NaN: direct form only), tvn
+    kChunkLc = 3,     // p1u, p1v, p2u, p2v
+    kChunkNop = 4,    // nu, nv, opacity, chart start (int)
+    kChunkUvm = 5,    // texture uv numerators
+    kChunkUvs = 6,    // uv0.x, uv0.y, chart h, w (ints)
+    kChunkCol = 7,    // colour, 1 / (scale_x glob)
+    kChunkNrm = 8,    // world normal, 1 / (scale_y glob)
+    kChunkRay = 9,    // a1.mu / s1, a2.mu / s2, umap.mu, vmap.mu (camera space)
+    kChunkMisc = 10,  // blur centre x, y, flags, Gaussian id (ints)
+    kChunkBox = 11,   // screen box
+    kChunkMu = 12,    // camera-space mean, a1 . mean
+    kChunkDt = 13,    // a2 . mean, umap . mean, vmap . mean
+    kRecChunks = 14
 };
-static_assert(sizeof(RecAll) == kRecBytes + kEdgeBytes, "record layout");
+struct __align__(16) RecAll {
+    float4 c[kRecChunks];
+};
+static_assert(sizeof(RecAll) == 224, "record layout");
 
 struct Recs {
     RecHot* hot;
     RecWarm* warm;
     RecCold* cold;
-    RecEdge* edge;  // null when the kernel does not stage edges
-    __device__ __forceinline__ static Recs carve(unsigned char* smem, int n, bool with_edges) {
+    RecCull* cull;  // null when the kernel does not stage it
+    __device__ __forceinline__ static Recs carve(unsigned char* smem, int n, bool with_cull) {
         Recs r;
         r.hot = reinterpret_cast<RecHot*>(smem);
         r.warm = reinterpret_cast<RecWarm*>(smem + sizeof(RecHot) * n);
         r.cold = reinterpret_cast<RecCold*>(smem + (sizeof(RecHot) + sizeof(RecWarm)) * n);
-        r.edge = with_edges ? reinterpret_cast<RecEdge*>(smem + (size_t)kRecBytes * n) : nullptr;
+        r.cull = with_cull ? reinterpret_cast<RecCull*>(smem + (size_t)kRecBytes * n) : nullptr;
         return r;
     }
 };
@@ -243,56 +263,84 @@ __device__ __forceinline__ void edge_on_solve(RecHot& H, RecWarm& Wm, const View
                          (float)(mz * (g * vmc.x - vmd * nc.x) * ifx), (float)(mz * (g * vmc.y - vmd * nc.y) * ify));
 }
 
-// Edges of the convex quad with corners k = 0 (+,+), 1 (-,+), 3 (-,-), 2 (+,-)
-// in cyclic order, oriented so that the quad's centroid is inside, normalised
-// to pixel distances and widened by a margin; a degenerate edge passes all.
-__device__ __forceinline__ void quad_edges(const float (&qx)[4], const float (&qy)[4], RecEdge& E) {
-    const int cyc[5] = { 0, 1, 3, 2, 0 };
-    const float gx = 0.25f * (qx[0] + qx[1] + qx[2] + qx[3]), gy = 0.25f * (qy[0] + qy[1] + qy[2] + qy[3]);
-    const float margin = 0.05f + 1e-5f * (fabsf(gx) + fabsf(gy));
-    float A[4], B[4], C[4];
-    float side = 0.f;
-#pragma unroll
-    for (int e = 0; e < 4; e++) {
-        const int i = cyc[e], j = cyc[e + 1];
-        const float ax = -(qy[j] - qy[i]), by = qx[j] - qx[i];
-        const float len = sqrtf(ax * ax + by * by);
-        if (len > 1e-3f) {
-            const float il = 1.f / len;
-            A[e] = ax * il;
-            B[e] = by * il;
-            C[e] = -(A[e] * qx[i] + B[e] * qy[i]);
-            side += A[e] * gx + B[e] * gy + C[e];
-        } else {
-            A[e] = B[e] = 0.f;
-            C[e] = 1.f;
-        }
-    }
-    if (fabsf(side) < 1e-3f) {  // a quad of (near) zero width: no usable orientation
-        E.A = E.B = make_float4(0.f, 0.f, 0.f, 0.f);
-        E.C = make_float4(1.f, 1.f, 1.f, 1.f);
-        return;
-    }
-    const float sg = side < 0.f ? -1.f : 1.f;
-    // a flipped edge keeps C = 1 for the degenerate (all-pass) case
-#pragma unroll
-    for (int e = 0; e < 4; e++) {
-        if (A[e] != 0.f || B[e] != 0.f) {
-            A[e] *= sg;
-            B[e] *= sg;
-            C[e] = C[e] * sg + margin;
-        }
-    }
-    E.A = make_float4(A[0], A[1], A[2], A[3]);
-    E.B = make_float4(B[0], B[1], B[2], B[3]);
-    E.C = make_float4(C[0], C[1], C[2], C[3]);
+// s rounded away from zero, ih towards zero.
+__device__ __forceinline__ RecCull pack_cull(float xc, float yc, float m, float s, float ih, bool ellipse) {
+    RecCull c;
+    c.xc = xc;
+    c.yc = yc;
+    c.ms = (__float_as_uint(m) & 0xffff0000u) | ((__float_as_uint(s) + 0xffffu) >> 16);
+    c.hk = (__float_as_uint(ih) & 0xffff0000u) | (__float_as_uint(m) & 0xfffeu) | (ellipse ? 1u : 0u);
+    return c;
+}
+
+// Rows of the screen box x0..x1, y0..y1 (infinite or empty ones included).
+__device__ __forceinline__ RecCull cull_box(float x0, float x1, float y0, float y1) {
+    if (x0 > x1) return pack_cull(0.f, 0.f, 0.f, -1.f, 0.f, false);
+    if (!(fabsf(x0) < 1e30f && fabsf(x1) < 1e30f && fabsf(y0) < 1e30f && fabsf(y1) < 1e30f))
+        return pack_cull(0.f, 0.f, 0.f, INFINITY, 0.f, false);
+    // (the half sizes cover the rounding of the middle)
+    const float mx = 1e-3f + 1e-6f * (fabsf(x0) + fabsf(x1)), my = 1e-3f + 1e-6f * (fabsf(y0) + fabsf(y1));
+    return pack_cull(0.5f * (x0 + x1), 0.5f * (y0 + y1), 0.f, 0.5f * (x1 - x0) + mx, 0.99999f / (0.5f * (y1 - y0) + my),
+                     false);
+}
+
+// Image of the plane ellipse mu + e1 cos(t) a1 + e2 sin(t) a2.  With u_i the
+// homogeneous images of the axes relative to the projected centre (px0, py0),
+// its tangent lines satisfy l^T D l = 0, D = e1^2 u1 u1^T + e2^2 u2 u2^T -
+// u0 u0^T, u0 = (0, 0, z); scaled to D_zz = -1, D is [S - c c^T, -c; -c^T, -1]
+// with the ellipse's centre c and its second moments S, sums of squares
+// without cancellation.  S is widened so that the region grows by at least
+// `eps` pixels on every side: the per-pixel evaluation rounds the projected
+// centre to single precision, a thin sliver's half width may be less.
+// Returns false where a corner comes near the camera plane (D_zz cancels).
+__device__ __forceinline__ bool cull_ellipse(RecCull& c, const View& V, float3 mc, float u0, float v0, float3 a1,
+                                             float3 a2, float e1, float e2) {
+    const float x1 = e1 * V.fx * (a1.x - u0 * a1.z), y1 = e1 * V.fy * (a1.y - v0 * a1.z), z1 = e1 * a1.z;
+    const float x2 = e2 * V.fx * (a2.x - u0 * a2.z), y2 = e2 * V.fy * (a2.y - v0 * a2.z), z2 = e2 * a2.z;
+    const float k = mc.z * mc.z - (z1 * z1 + z2 * z2);
+    if (!(k > 0.05f * mc.z * mc.z)) return false;
+    const float ik = 1.f / k;
+    const float cx = -(x1 * z1 + x2 * z2) * ik, cy = -(y1 * z1 + y2 * z2) * ik;
+    float sxx = (x1 * x1 + x2 * x2) * ik + cx * cx, syy = (y1 * y1 + y2 * y2) * ik + cy * cy;
+    const float sxy = (x1 * y1 + x2 * y2) * ik + cx * cy;
+    const float px0 = V.fx * u0 + V.cx, py0 = V.fy * v0 + V.cy;
+    const float reach = sqrtf(sxx + syy);
+    const float eps = 5e-4f + 5e-7f * (fabsf(px0) + fabsf(py0)) + 2e-6f * reach;
+    const float grow = 2.f * reach * eps + eps * eps;
+    sxx += grow;
+    syy += grow;
+    const float m = sxy / syy, w = sxx - sxy * m, hy = sqrtf(syy);
+    if (!(w > 0.f && sxx < 1e12f && syy < 1e12f)) return false;
+    c = pack_cull(px0 + cx, py0 + cy, m, sqrtf(w) * 1.0001f, 0.9999f / hy, true);
+    return true;
+}
+
+// One row of a region: its middle and half width there; false if the region
+// does not meet the row.
+__device__ __forceinline__ bool cull_span(const RecCull& c, float y, float& mid, float& half) {
+    const float dy = y - c.yc, u = dy * __uint_as_float(c.hk & 0xffff0000u);
+    const float q = 1.f - u * u;
+    mid = c.xc + __uint_as_float((c.ms & 0xffff0000u) | (c.hk & 0xfffeu)) * dy;
+    half = __uint_as_float(c.ms << 16) * sqrtf((c.hk & 1u) ? fmaxf(q, 0.f) : 1.f) + 1e-3f;
+    return q >= 0.f;
+}
+
+// Columns [0, 8) of one row that a region can reach, as a bit mask: x0 is the
+// centre of column 0, y the row's centre.
+__device__ __forceinline__ unsigned cull_row(const RecCull& c, float x0, float y) {
+    float mid, half;
+    const bool meets = cull_span(c, y, mid, half);
+    mid -= x0;
+    const int lo = min(max(__float2int_ru(mid - half), 0), 8), hi = min(max(__float2int_rd(mid + half), -1), 7) + 1;
+    const unsigned bits = ((1u << hi) - 1u) & ~((1u << lo) - 1u);
+    return meets ? bits : 0u;
 }
 
 __device__ __forceinline__ bool make_record(RecHot& H, RecWarm& Wm, RecCold& Cd, int gid, const View& V,
                                             const float3 mean, const float4 quat, const float2 scale,
                                             float glob_scale, float opac, float3 color, float2 uv0, float3 umap,
                                             float3 vmap, int3 dims, bool use_blur, bool allow_double = true,
-                                            RecEdge* E = nullptr, bool cull = true) {
+                                            RecCull* E = nullptr, bool cull = true) {
     const Axes A = quat_axes(quat);
     const float3 mc = V.xform(mean);
     const float3 a1c = V.rot(A.a1), a2c = V.rot(A.a2), nc = V.rot(A.a3);
@@ -314,15 +362,11 @@ __device__ __forceinline__ bool make_record(RecHot& H, RecWarm& Wm, RecCold& Cd,
     const float smax = __logf(255.f * opac);
     int flags = 0;
     if (!(mc.z > kTNear)) flags = 1;
-    if (E) {
-        E->A = E->B = make_float4(0.f, 0.f, 0.f, 0.f);
-        E->C = make_float4(1.f, 1.f, 1.f, 1.f);
-    }
+    bool oval = false;
     if (smax > 0.f) {
         const float a = sqrtf(2.f * smax + 1e-3f) * 1.002f;
         const float e1 = a / is1, e2 = a / is2;
         bool front = !flags;
-        float qx[4], qy[4];
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             const float s1 = (k & 1) ? -e1 : e1, s2 = (k & 2) ? -e2 : e2;
@@ -331,15 +375,13 @@ __device__ __forceinline__ bool make_record(RecHot& H, RecWarm& Wm, RecCold& Cd,
             front = front && c.z > 1e-3f;
             const float iz = 1.f / c.z;
             const float px = V.fx * c.x * iz + V.cx, py = V.fy * c.y * iz + V.cy;
-            qx[k] = px;
-            qy[k] = py;
             x0 = fminf(x0, px); x1 = fmaxf(x1, px);
             y0 = fminf(y0, py); y1 = fmaxf(y1, py);
         }
         if (front) {
             const float mx = 1e-2f + 1e-5f * (fabsf(x0) + fabsf(x1)), my = 1e-2f + 1e-5f * (fabsf(y0) + fabsf(y1));
             x0 -= mx; x1 += mx; y0 -= my; y1 += my;
-            if (E && !use_blur) quad_edges(qx, qy, *E);
+            if (E && !use_blur && cull) oval = cull_ellipse(*E, V, mc, mc.x / mc.z, mc.y / mc.z, a1c, a2c, e1, e2);
         } else {
             x0 = y0 = -INFINITY;
             x1 = y1 = INFINITY;
@@ -358,11 +400,8 @@ __device__ __forceinline__ bool make_record(RecHot& H, RecWarm& Wm, RecCold& Cd,
         // alpha-visualisation mode sets alpha without the opacity: no box
         x0 = y0 = -INFINITY;
         x1 = y1 = INFINITY;
-        if (E) {
-            E->A = E->B = make_float4(0.f, 0.f, 0.f, 0.f);
-            E->C = make_float4(1.f, 1.f, 1.f, 1.f);
-        }
     }
+    if (E && !oval) *E = cull_box(x0, x1, y0, y1);
 
     H.box = make_float4(x0, x1, y0, y1);
     if (flags) {
@@ -392,6 +431,36 @@ __device__ __forceinline__ bool make_record(RecHot& H, RecWarm& Wm, RecCold& Cd,
     H.nop.z = opac;
     H.nop.w = __int_as_float(flags);
     return edge_on && !allow_double;
+}
+
+__device__ __forceinline__ RecCull unpack_cull(float4 c) {
+    RecCull e;
+    e.xc = c.x;
+    e.yc = c.y;
+    e.ms = __float_as_uint(c.z);
+    e.hk = __float_as_uint(c.w);
+    return e;
+}
+
+// A record as it is stored (RecChunk).  The block kernels read "direct form
+// only" from a NaN in g, which makes the plane denominator NaN.
+__device__ __forceinline__ void pack_record(RecAll& r, const RecHot& h, const RecWarm& w, const RecCold& c,
+                                            const RecCull& e) {
+    const int flags = __float_as_int(h.nop.w);
+    r.c[kChunkCull] = make_float4(e.xc, e.yc, __uint_as_float(e.ms), __uint_as_float(e.hk));
+    r.c[kChunkCull + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
+    r.c[kChunkOrg] = make_float4(h.org.x, h.org.y, flags ? __int_as_float(0x7fffffff) : h.org.z, h.org.w);
+    r.c[kChunkLc] = h.lc;
+    r.c[kChunkNop] = make_float4(h.nop.x, h.nop.y, h.nop.z, __int_as_float(w.tex.z));
+    r.c[kChunkUvm] = w.uvm;
+    r.c[kChunkUvs] = make_float4(w.uvs.x, w.uvs.y, __int_as_float(w.tex.x), __int_as_float(w.tex.y));
+    r.c[kChunkCol] = w.col;
+    r.c[kChunkNrm] = w.nrm;
+    r.c[kChunkRay] = make_float4(w.col.w * c.mu.w, w.nrm.w * c.dt.x, c.dt.y, c.dt.z);
+    r.c[kChunkMisc] = make_float4(w.uvs.z, w.uvs.w, h.nop.w, __int_as_float(w.tex.w));
+    r.c[kChunkBox] = h.box;
+    r.c[kChunkMu] = c.mu;
+    r.c[kChunkDt] = c.dt;
 }
 
 // Per-pixel constants: pixel centre, camera direction d = (u, v, 1), |d|.

@@ -19,6 +19,7 @@
 // view (the reference's texture_forward/backward), and a persistent kernel
 // that pulls tiles of many views from one global queue (batched rendering).
 #include "common.cuh"
+#include "pixel.cuh"
 #include "raster.cuh"
 
 namespace gstex {
@@ -28,7 +29,7 @@ __device__ __forceinline__ void stage(const Recs& R, int slot, const SceneArgs& 
     make_record(R.hot[slot], R.warm[slot], R.cold[slot], gid, V, a.means[gid], a.quats[gid],
                 make_float2(a.scales[3 * gid], a.scales[3 * gid + 1]), a.glob, a.opac[gid],
                 colors ? colors[gid] : make_float3(0.f, 0.f, 0.f), a.uv0[gid],
-                a.umap[gid], a.vmap[gid], a.dims[gid], use_blur, true, R.edge ? R.edge + slot : nullptr,
+                a.umap[gid], a.vmap[gid], a.dims[gid], use_blur, true, R.cull ? R.cull + slot : nullptr,
                 !(a.settings & (1 << 16)));
 }
 
@@ -37,24 +38,24 @@ __device__ __forceinline__ void stage(const Recs& R, int slot, const SceneArgs& 
 __device__ __forceinline__ void stage_job(const Recs& R, int slot, const SceneArgs& a, const TileJob& J, int gid,
                                           bool use_blur) {
     if (J.recs) {
-        const uint4* src = reinterpret_cast<const uint4*>(J.recs + gid);
-        uint4 v[kRecBytes / 16];
-#pragma unroll
-        for (int q = 0; q < kRecBytes / 16; q++) v[q] = __ldg(src + q);
-        uint4* hot = reinterpret_cast<uint4*>(R.hot + slot);
-        uint4* warm = reinterpret_cast<uint4*>(R.warm + slot);
-        uint4* cold = reinterpret_cast<uint4*>(R.cold + slot);
-        constexpr int nh = sizeof(RecHot) / 16, nw = sizeof(RecWarm) / 16, nc = sizeof(RecCold) / 16;
-#pragma unroll
-        for (int q = 0; q < nh; q++) hot[q] = v[q];
-#pragma unroll
-        for (int q = 0; q < nw; q++) warm[q] = v[nh + q];
-#pragma unroll
-        for (int q = 0; q < nc; q++) cold[q] = v[nh + nw + q];
-        if (R.edge) {
-            uint4* edge = reinterpret_cast<uint4*>(R.edge + slot);
-#pragma unroll
-            for (int q = 0; q < kEdgeBytes / 16; q++) edge[q] = __ldg(src + kRecBytes / 16 + q);
+        const float4* src = J.recs[gid].c;
+        const float4 nop = __ldg(src + kChunkNop), uvs = __ldg(src + kChunkUvs), misc = __ldg(src + kChunkMisc);
+        RecHot& h = R.hot[slot];
+        RecWarm& w = R.warm[slot];
+        RecCold& c = R.cold[slot];
+        h.box = __ldg(src + kChunkBox);
+        h.org = __ldg(src + kChunkOrg);
+        h.lc = __ldg(src + kChunkLc);
+        h.nop = make_float4(nop.x, nop.y, nop.z, misc.z);
+        w.uvm = __ldg(src + kChunkUvm);
+        w.uvs = make_float4(uvs.x, uvs.y, misc.x, misc.y);
+        w.col = __ldg(src + kChunkCol);
+        w.nrm = __ldg(src + kChunkNrm);
+        w.tex = make_int4(__float_as_int(uvs.z), __float_as_int(uvs.w), __float_as_int(nop.w), __float_as_int(misc.w));
+        c.mu = __ldg(src + kChunkMu);
+        c.dt = __ldg(src + kChunkDt);
+        if (R.cull) {
+            R.cull[slot] = unpack_cull(__ldg(src + kChunkCull));
         }
     } else {
         stage(R, slot, a, J.V, J.colors, gid, use_blur);
@@ -65,21 +66,6 @@ __device__ __forceinline__ void stage_job(const Recs& R, int slot, const SceneAr
 // threads of the CTA, which stage one each), else one per thread.
 __device__ __forceinline__ int batch_of(const SceneArgs& a, int nthr) {
     return (a.batch > 0 && a.batch < nthr) ? a.batch : nthr;
-}
-
-// Completes a Hit in the direct form, rebuilding the Gaussian's camera-space
-// frame from its parameters (rare: splats at the camera plane and pixels within
-// the reference's denominator clamp).
-__device__ __forceinline__ void direct_hit(Hit& H, const float4* __restrict__ quats, const float3* __restrict__ means,
-                                           const float* __restrict__ scales, float glob, const float2* __restrict__ uv0s,
-                                           const float3* __restrict__ umaps, const float3* __restrict__ vmaps,
-                                           const View& V, int gid, const PixelRay& P, float tvn) {
-    const Axes A = quat_axes(quats[gid]);
-    const float3 mc = V.xform(means[gid]);
-    const float is1 = 1.f / (scales[3 * gid] * glob), is2 = 1.f / (scales[3 * gid + 1] * glob);
-    const float2 uv0 = uv0s[gid];
-    intersect_direct(H, P, tvn, mc, V.rot(A.a1), V.rot(A.a2), V.rot(A.a3), V.rot(umaps[gid]), V.rot(vmaps[gid]), is1,
-                     is2, uv0.x, uv0.y);
 }
 
 __device__ __forceinline__ Hit hit_pixel(const RecHot& Hr, const Recs& R, int k, const SceneArgs& a, const View& V,
@@ -105,32 +91,6 @@ __device__ __noinline__ float local_outline(const RecHot& Hr, const Recs& R, int
         }
     }
     return best;
-}
-
-// All channels of the 4 bilinear corners (C == 3 fast path).
-template <int TEXMODE>
-__device__ __forceinline__ void fetch3(const void* tex, const Bilerp& B, float c[4][3]) {
-    const int rows[4] = { B.i00, B.i01, B.i10, B.i11 };
-    if (TEXMODE == 1) {
-        const uint2* t = (const uint2*)tex;
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const uint2 raw = __ldg(t + rows[q]);
-            const __nv_bfloat162 lo = *reinterpret_cast<const __nv_bfloat162*>(&raw.x);
-            const __nv_bfloat162 hi = *reinterpret_cast<const __nv_bfloat162*>(&raw.y);
-            c[q][0] = __low2float(lo);
-            c[q][1] = __high2float(lo);
-            c[q][2] = __low2float(hi);
-        }
-    } else {
-        const float* t = (const float*)tex;
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            c[q][0] = __ldg(t + 3 * rows[q] + 0);
-            c[q][1] = __ldg(t + 3 * rows[q] + 1);
-            c[q][2] = __ldg(t + 3 * rows[q] + 2);
-        }
-    }
 }
 
 // Local (row, column) of a thread's first pixel.  When the tile width is a
@@ -189,15 +149,16 @@ __device__ __forceinline__ int group_min(int v) {
 __device__ __forceinline__ bool splat_meets_rect(const Recs& R, int kk, float rx0, float rx1, float ry0, float ry1) {
     const float4 bx = R.hot[kk].box;
     bool hit = !(bx.y < rx0 || bx.x > rx1 || bx.w < ry0 || bx.z > ry1);
-    if (hit && R.edge) {
-        // separating axes of the splat's quad: the rectangle's corner
-        // furthest inside each edge must be inside it
-        const RecEdge e = R.edge[kk];
-        const float ea[4] = { e.A.x, e.A.y, e.A.z, e.A.w }, eb[4] = { e.B.x, e.B.y, e.B.z, e.B.w };
-        const float ec[4] = { e.C.x, e.C.y, e.C.z, e.C.w };
-#pragma unroll
-        for (int q = 0; q < 4; q++)
-            hit = hit && ea[q] * (ea[q] > 0.f ? rx1 : rx0) + eb[q] * (eb[q] > 0.f ? ry1 : ry0) + ec[q] >= 0.f;
+    if (hit && R.cull) {
+        // some row of pixel centres (a subset of y = ry0, ry0 + 1, ...) must
+        // meet the region inside [rx0, rx1]
+        const RecCull c = R.cull[kk];
+        bool any = false;
+        for (float y = ry0; y <= ry1; y += 1.f) {
+            float mid, half;
+            any = any || (cull_span(c, y, mid, half) && mid - half <= rx1 && mid + half >= rx0);
+        }
+        hit = any;
     }
     return hit;
 }
@@ -475,11 +436,6 @@ struct Ragged<N, 0> {
     static __device__ __forceinline__ int slot(unsigned, int j = 0) { return j; }
 };
 static_assert(Ragged<23, 16>::OUT == 1, "a full warp reduces 23 moments to one per lane");
-
-template <typename T>
-__device__ __forceinline__ T ld_or(const T* p, size_t i, T z) {
-    return p ? p[i] : z;
-}
 
 // Per-pixel state of the backward walk.
 template <int CA>
@@ -1024,9 +980,9 @@ __global__ void BWD_BOUNDS(PPT) bwd_view_kernel(SceneArgs a, ViewArgs va, BwdArg
     J.vcolors = va.vcolors;
     J.vc_stride = 3;
     J.recs = va.recs;
-    uint8_t* lists = smem + (size_t)(kRecBytes + kEdgeBytes + kMomSlot * sizeof(float)) * nthr;
+    uint8_t* lists = smem + (size_t)(kRecBytes + (int)sizeof(RecCull) + kMomSlot * sizeof(float)) * nthr;
     bwd_tile<TEXMODE, CT, PPT, GS>(a, J, g, Recs::carve(smem, nthr, true),
-                                   reinterpret_cast<float*>(smem + (size_t)(kRecBytes + kEdgeBytes) * nthr), lists,
+                                   reinterpret_cast<float*>(smem + (size_t)(kRecBytes + (int)sizeof(RecCull)) * nthr), lists,
                                    lists + ((size_t)ceil_div(nthr, 32) + (GS < 32 ? ceil_div(nthr, GS) : 0)) * nthr);
 }
 
@@ -1071,8 +1027,8 @@ __device__ __forceinline__ void bwd_batch_body(const SceneArgs& a, const BatchAr
     const int slots = batch_of(a, nthr);
     TileJob J;
     const Recs R = Recs::carve(smem, slots, true);
-    float* smom = reinterpret_cast<float*>(smem + (size_t)(kRecBytes + kEdgeBytes) * slots);
-    uint8_t* lists = smem + (size_t)(kRecBytes + kEdgeBytes + kMomSlot * sizeof(float)) * slots;
+    float* smom = reinterpret_cast<float*>(smem + (size_t)(kRecBytes + (int)sizeof(RecCull)) * slots);
+    uint8_t* lists = smem + (size_t)(kRecBytes + (int)sizeof(RecCull) + kMomSlot * sizeof(float)) * slots;
     uint8_t* touched = lists + ((size_t)ceil_div(nthr, 32) + (GS < 32 ? ceil_div(nthr, GS) : 0)) * slots;
     while (next_job(ba, &s_tile, J)) bwd_tile<TEXMODE, CT, PPT, GS, FIX>(a, J, g, R, smom, lists, touched);
 }
@@ -1131,11 +1087,15 @@ __global__ void __launch_bounds__(128) records_kernel(SceneArgs a, BatchArgs ba,
     const bool live = i < ba.num_points && (i == 0 || counts[j] > 0);
     if (live) {
         const View V = ba.views[v].V;
-        RecAll& r = srec[threadIdx.x];
-        const bool defer = make_record(r.h, r.w, r.c, i, V, a.means[i], a.quats[i],
+        RecHot h;
+        RecWarm w;
+        RecCold c;
+        RecCull e;
+        const bool defer = make_record(h, w, c, i, V, a.means[i], a.quats[i],
                                        make_float2(a.scales[3 * i], a.scales[3 * i + 1]), a.glob, a.opac[i],
                                        ba.colors[j], a.uv0[i], a.umap[i], a.vmap[i], a.dims[i],
-                                       a.settings & (1 << 9), false, &r.e, !(a.settings & (1 << 16)));
+                                       a.settings & (1 << 9), false, &e, !(a.settings & (1 << 16)));
+        pack_record(srec[threadIdx.x], h, w, c, e);
         if (defer) fix[atomicAdd(fix_count, 1)] = (uint32_t)j;
     }
     const unsigned lane = threadIdx.x & 31;
@@ -1150,11 +1110,14 @@ __device__ __forceinline__ void fix_record(const SceneArgs& a, const View& V, in
     const float3 a1c = V.rot(A.a1), a2c = V.rot(A.a2), nc = V.rot(A.a3);
     const float3 umc = V.rot(a.umap[i]), vmc = V.rot(a.vmap[i]);
     const float is1 = 1.f / (a.scales[3 * i] * a.glob), is2 = 1.f / (a.scales[3 * i + 1] * a.glob);
-    RecHot h = rec->h;
-    RecWarm w = rec->w;
+    RecHot h;
+    RecWarm w;
     edge_on_solve(h, w, V, mc, a1c, a2c, nc, umc, vmc, is1, is2, dot3(nc, mc));
-    rec->h = h;
-    rec->w.uvm = w.uvm;
+    rec->c[kChunkOrg] = h.org;
+    rec->c[kChunkLc] = h.lc;
+    rec->c[kChunkNop].x = h.nop.x;
+    rec->c[kChunkNop].y = h.nop.y;
+    rec->c[kChunkUvm] = w.uvm;
 }
 
 // The double solve of the deferred near-edge-on records, densely.
@@ -1179,11 +1142,15 @@ __global__ void __launch_bounds__(128) view_records_kernel(SceneArgs a, ViewArgs
     const bool live = i < a.N;
     if (live) {
         const View V = load_view(va.viewmat, va.fx, va.fy, va.cx, va.cy);
-        RecAll& r = srec[threadIdx.x];
-        const bool defer = make_record(r.h, r.w, r.c, i, V, a.means[i], a.quats[i],
+        RecHot h;
+        RecWarm w;
+        RecCold c;
+        RecCull e;
+        const bool defer = make_record(h, w, c, i, V, a.means[i], a.quats[i],
                                        make_float2(a.scales[3 * i], a.scales[3 * i + 1]), a.glob, a.opac[i],
                                        va.colors[i], a.uv0[i], a.umap[i], a.vmap[i], a.dims[i], a.settings & (1 << 9),
-                                       false, &r.e, !(a.settings & (1 << 16)));
+                                       false, &e, !(a.settings & (1 << 16)));
+        pack_record(srec[threadIdx.x], h, w, c, e);
         if (defer) fix[atomicAdd(fix_count, 1)] = (uint32_t)i;
     }
     const unsigned lane = threadIdx.x & 31;
@@ -1395,7 +1362,7 @@ static size_t list_bytes(int bw, int ppt, int gs, int batch) {
 size_t fwd_smem(int bw, int ppt, int batch) { return (size_t)kRecBytes * slots_of(bw, ppt, batch); }
 size_t bwd_smem(int bw, int ppt, int gs, int batch) {
     // ... then one "touched" flag per slot
-    return ((size_t)kRecBytes + kEdgeBytes + kMomSlot * sizeof(float) + 1) * slots_of(bw, ppt, batch) +
+    return ((size_t)kRecBytes + (int)sizeof(RecCull) + kMomSlot * sizeof(float) + 1) * slots_of(bw, ppt, batch) +
            list_bytes(bw, ppt, gs, batch);
 }
 
@@ -1418,8 +1385,39 @@ static FwdBatch<0, 0, 1>::type pick_fwd_batch(int C, int texmode, int& ppt, int 
     return pick_fwd<FwdBatch>(C, texmode, ppt, settings);
 }
 
+static BlockArgs block_args(const BatchArgs& ba, int bw) {
+    BlockArgs b{};
+    b.total_tiles = ba.total_tiles;
+    b.bw = bw;
+    b.num_points = ba.num_points;
+    b.views = ba.views;
+    b.tile_view = ba.tile_view;
+    b.order = ba.order;
+    b.bins = ba.bins;
+    b.recs = ba.recs;
+    b.vcolors = ba.vcolors;
+    b.vc_stride = 4;
+    return b;
+}
+
+static BlockArgs block_args(const ViewArgs& va, int bw, int n) {
+    BlockArgs b{};
+    b.total_tiles = va.tiles_x * ceil_div(va.H, bw);
+    b.bw = bw;
+    b.num_points = n;
+    b.bins = va.bins;
+    b.recs = va.recs;
+    b.vcolors = va.vcolors;
+    b.vc_stride = 3;
+    b.viewmat = va.viewmat;
+    b.fx = va.fx; b.fy = va.fy; b.cx = va.cx; b.cy = va.cy;
+    b.W = va.W; b.H = va.H; b.tiles_x = va.tiles_x;
+    return b;
+}
+
 int launch_fwd_batch(const SceneArgs& a, const BatchArgs& ba, const FwdOut& o, int bw, int texmode, int ppt, int grid,
                      cudaStream_t stream) {
+    if (blocks_apply(bw, a.C, a.settings, ba.recs)) return launch_fwd_blocks(a, block_args(ba, bw), o, texmode, stream);
     ppt = ppt_of(bw, ppt);
     auto k = pick_fwd_batch(a.C, texmode, ppt, a.settings);
     const size_t smem = fwd_smem(bw, ppt, a.batch);
@@ -1551,6 +1549,8 @@ extern "C" int gstex_texture_forward(const gstex_raster_inputs* in, const gstex_
     const int bw = in->block_width;
     ViewArgs va = view_args(in);
     cudaStream_t stream = (cudaStream_t)s;
+    if (blocks_apply(bw, a.C, a.settings, va.recs))
+        return launch_fwd_blocks(a, block_args(va, bw, a.N), o, in->texture_dtype, stream);
     const dim3 grid(va.tiles_x, ceil_div(va.H, bw));
     int ppt = ppt_of(bw, in->pixels_per_thread);
     auto k = pick_fwd<FwdView>(a.C, in->texture_dtype, ppt, a.settings);

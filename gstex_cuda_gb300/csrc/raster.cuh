@@ -73,6 +73,22 @@ struct TileJob {
     const RecAll* recs;   // the view's prebuilt records, or null
 };
 
+// Launch of the block kernels (composite.cu): the tiles of the views of a
+// batch, or of one view (views == nullptr).
+struct BlockArgs {
+    int total_tiles, bw, num_points;
+    const BatchView* views;
+    const int32_t* tile_view;
+    const int32_t* order;      // optional order of the tiles
+    const int2* bins;
+    const RecAll* recs;        // [V, N]
+    float* vcolors;            // [V, N, vc_stride] colour gradients (backward)
+    int vc_stride;
+    const float* viewmat;      // one view
+    float fx, fy, cx, cy;
+    int W, H, tiles_x;
+};
+
 struct FwdOut {
     float3* img;
     float* depth;
@@ -136,6 +152,8 @@ constexpr int kFixedBwdSettings = 1 << 8;
 // (bilinear off, blur, NDC depth, flipped normals, alpha visualisation): the
 // kernel compiled for fixed settings applies when all are off.
 constexpr int kFixedFwdMask = (1 << 2) | (1 << 9) | (1 << 10) | (1 << 15) | (1 << 16);
+bool blocks_apply(int bw, int C, int settings, const RecAll* recs);
+int launch_fwd_blocks(const SceneArgs& a, const BlockArgs& ba, const FwdOut& o, int texmode, cudaStream_t stream);
 int launch_records(const SceneArgs& a, const BatchArgs& ba, int num_views, const int32_t* counts, RecAll* recs,
                    int* fix_count, uint32_t* fix, cudaStream_t stream);
 
