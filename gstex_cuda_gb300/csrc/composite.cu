@@ -1,7 +1,7 @@
-// Block compositor: the textured 2D-Gaussian forward with one warp per 8x4
-// block of pixels.
+// Block compositor: the textured 2D-Gaussian forward and backward with one
+// warp per 8x4 block of pixels.
 //
-// Reference: csrc/texture.cu:11-329.  A splat reaches about a tenth of
+// Reference: csrc/texture.cu:11-329 and 331-760.  A splat reaches about a tenth of
 // the pixels of a tile that lists it, so a warp that walks its tile's list
 // splat by splat has few of its lanes at work.  Here a warp first turns the
 // list into one list per pixel and then every lane walks its own:
@@ -251,6 +251,9 @@ __device__ __forceinline__ float block_alpha(const Hit& H, float opac, bool use_
     return fminf(kAlphaMax, opac * (nbf * e + bf * eb));
 }
 
+__device__ __forceinline__ int chart_start(float4 nop) { return (int)(__float_as_uint(nop.w) & ~kCoarseChart); }
+__device__ __forceinline__ bool is_coarse(float4 nop) { return (__float_as_uint(nop.w) & kCoarseChart) != 0u; }
+
 // uv of the hit before clamping (hit_uv on the stored chunks).
 __device__ __forceinline__ float2 block_uv(const Hit& H, float4 uvm, float2 uv0) {
     if (H.direct) return make_float2(H.tu, H.tv);
@@ -294,7 +297,7 @@ __device__ __forceinline__ void blend(FwdPix<CT>& S, const SceneArgs& a, const R
     if (CT == 3) {
         const float4 uvs = rec(kChunkUvs);
         const float2 uv = block_uv(H, rec(kChunkUvm), make_float2(uvs.x, uvs.y));
-        const Bilerp B = bilerp(__float_as_int(uvs.z), __float_as_int(uvs.w), __float_as_int(rec(kChunkNop).w),
+        const Bilerp B = bilerp(__float_as_int(uvs.z), __float_as_int(uvs.w), chart_start(rec(kChunkNop)),
                                 clamp01(uv.x), clamp01(uv.y), FIX || !(a.settings & (1 << 2)));
         float c[4][3];
         fetch3<TM>(a.tex, B, c);
@@ -459,6 +462,427 @@ __global__ void __launch_bounds__(32 * kBlockWarps, kFwdCtas)
 }
 
 // ---------------------------------------------------------------------------
+// Backward.  The walk is the forward's, back to front; a splat's gradients are
+// sums over pixels (finalize_kernel turns 21 of them into the parameters'
+// gradients), and the pixels of a step are at different splats.  So every lane
+// first steps back over up to kRounds of its pixel's pairs and leaves eight
+// numbers per pair in shared memory; then the roles turn (one more transpose):
+// every lane takes a splat and sums the pairs of its pixels in registers,
+// without the shuffles and shared-memory atomics of a reduction over the warp,
+// and adds the sums to the splat's row with 16-byte atomics.
+//
+// What bounds it: the L1 data path (71% of its cycles; a 16-byte reduction
+// takes about a cycle per lane there) and the latency of its chains at 16 warps
+// per SM.  Of 23.6 ms on 32 views (36.6 ms with the list walk, its moment
+// reduction by shuffles and 8-lane groups) the scan, staging and ray-plane
+// solves take 6 ms, the adjoint 4, texel reads 3.5, texel atomics 4 and the
+// sums 6.  8 clustered full-HD views: 22.3 -> 14.4 ms; one 800x800 view of 1x1
+// charts 254 -> 111 us; one full-HD view of large splats 36.0 -> 8.7 ms (where
+// the list walk also staged every splat behind the last contributor).
+// ---------------------------------------------------------------------------
+constexpr int kBwdChunks = 8;
+// Pairs per pixel between two summations, and CTAs per SM (at most 128
+// registers): 7 rounds are what fits 8 CTAs' shared memory.  6 and 8: 2% slower;
+// 5 and 9: 16%; 9 and 7: 9% (32 views).
+constexpr int kRounds = 7;
+constexpr int kBwdCtas = 8;
+struct BwdMem {
+    Staged<kBwdChunks> rec;
+    float4 pair[2][kRounds][33];  // (vis, e v_alpha, v_sigma, v_t / (n . r)), (v_u, v_v, l1s, l2s) of a pixel's pairs
+    float4 pix[3][32];            // upstream colour, normal and texture gradients of the pixels (w: centre x, y)
+    unsigned valid[32];           // staged splats of a pixel's pairs
+    uint8_t slot[32];             // splats with pairs
+    Queue q;
+};
+
+template <int CT>
+struct BwdState {
+    float T, vT_run;
+    float3 sfin, vout, vnorm;
+    int dfin, bfin;
+    float vdepth, vreg;
+    float vtex[CT > 0 ? CT : 1];
+};
+
+// Texel gradients of one pair: gv = vis * upstream texture gradient.
+template <int TM>
+__device__ __forceinline__ void add_texel_grads(float* __restrict__ v_texgrad, const Bilerp& B, float2 gv01, float gv2) {
+    if (gv01.x == 0.f && gv01.y == 0.f && gv2 == 0.f) return;
+    const int rows[4] = { B.i00, B.i01, B.i10, B.i11 };
+    float wts[4] = { B.w00, B.w01, B.w10, B.w11 };
+    // beyond a chart's last row or column two texels are one: add once
+    if (B.i10 == B.i00) {
+        wts[0] += wts[2]; wts[1] += wts[3];
+        wts[2] = wts[3] = 0.f;
+    }
+    if (B.i01 == B.i00) {
+        wts[0] += wts[1]; wts[2] += wts[3];
+        wts[1] = wts[3] = 0.f;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        if (wts[q] == 0.f) continue;
+        const float2 g01 = mul2(dup2(wts[q]), gv01);
+        if (TM == 1) {
+            atomicAdd(reinterpret_cast<float4*>(v_texgrad) + rows[q], make_float4(g01.x, g01.y, wts[q] * gv2, 0.f));
+        } else {
+            float* dst = v_texgrad + 3 * (size_t)rows[q];
+            atomicAdd(dst + 0, g01.x);
+            atomicAdd(dst + 1, g01.y);
+            atomicAdd(dst + 2, wts[q] * gv2);
+        }
+    }
+}
+
+// Adjoint of one contributing pair (csrc/texture.cu:577-708): steps the pixel's
+// recurrences back over it, adds its texel gradients and returns what the
+// per-splat sums need of it.
+template <int TM, int CT, int FIX>
+__device__ __forceinline__ void pair_adjoint(BwdState<CT>& S, const SceneArgs& a, const BwdArgs& g,
+                                             const StagedRec<kBwdChunks>& rec, const Hit& H, const PixelRay& P, int idx,
+                                             float opac, float alpha, float nbf, float bf, float e, float eb, float4& q0,
+                                             float4& q1) {
+    const bool use_ndc = !FIX && (a.settings & (1 << 10)), prop_uv = FIX || (a.settings & (1 << 8));
+    const bool bilinear = FIX || !(a.settings & (1 << 2));
+    const float4 col = rec(kChunkCol), nw = rec(kChunkNrm), ray = rec(kChunkRay);
+    S.T = __fdividef(S.T, 1.f - alpha);
+    const float T = S.T;
+    const float vis = alpha * T;
+    float v_vis = col.x * S.vout.x + col.y * S.vout.y + col.z * S.vout.z + nw.x * S.vnorm.x + nw.y * S.vnorm.y +
+                  nw.z * S.vnorm.z;
+    float v_u = 0.f, v_v = 0.f;
+    float2 duv = make_float2(0.f, 0.f);  // uv of the hit, relative to uv0
+    if (CT == 3) {
+        const float4 uvs = rec(kChunkUvs);
+        const float2 uv = block_uv(H, rec(kChunkUvm), make_float2(uvs.x, uvs.y));
+        duv = sub2(uv, make_float2(uvs.x, uvs.y));
+        const int h = __float_as_int(uvs.z), w = __float_as_int(uvs.w);
+        const float4 nop = rec(kChunkNop);
+        const Bilerp B = bilerp(h, w, chart_start(nop), clamp01(uv.x), clamp01(uv.y), bilinear);
+        float c[4][3];
+        fetch3<TM>(a.tex, B, c);
+        // channels 0 and 1 as f32x2 pairs, channel 2 alone
+        const float2 c0 = make_float2(c[0][0], c[0][1]), c1 = make_float2(c[1][0], c[1][1]);
+        const float2 c2 = make_float2(c[2][0], c[2][1]), c3 = make_float2(c[3][0], c[3][1]);
+        const float2 vt = make_float2(S.vtex[0], S.vtex[1]);
+        float2 val = mul2(dup2(B.w00), c0);
+        val = fma2(dup2(B.w01), c1, val);
+        val = fma2(dup2(B.w10), c2, val);
+        val = fma2(dup2(B.w11), c3, val);
+        const float val2 = B.w00 * c[0][2] + B.w01 * c[1][2] + B.w10 * c[2][2] + B.w11 * c[3][2];
+        const float2 gv01 = mul2(dup2(vis), vt);
+        const float gv2 = vis * S.vtex[2];
+        if (bilinear && prop_uv) {
+            // d(val)/d(tcx) = (1 - fy)(c10 - c00) + fy (c11 - c01),
+            // d(val)/d(tcy) = (1 - fx)(c01 - c00) + fx (c11 - c10)
+            const float2 du = fma2(dup2(B.fy), sub2(c3, c1), mul2(dup2(1.f - B.fy), sub2(c2, c0)));
+            const float2 dv = fma2(dup2(B.fx), sub2(c3, c2), mul2(dup2(1.f - B.fx), sub2(c1, c0)));
+            const float du2 = (1.f - B.fy) * (c[2][2] - c[0][2]) + B.fy * (c[3][2] - c[1][2]);
+            const float dv2 = (1.f - B.fx) * (c[1][2] - c[0][2]) + B.fx * (c[3][2] - c[2][2]);
+            const float2 pu = mul2(gv01, du), pv = mul2(gv01, dv);
+            v_u = (float)h * (pu.x + pu.y + gv2 * du2);
+            v_v = (float)w * (pv.x + pv.y + gv2 * dv2);
+        }
+        const float2 vs = mul2(val, vt);
+        v_vis += vs.x + vs.y + val2 * S.vtex[2];
+        // (a coarse chart's are summed over the pixels first)
+        if (!is_coarse(nop)) add_texel_grads<TM>(g.v_texgrad, B, gv01, gv2);
+    }
+    float v_alpha = T * v_vis - T * S.vT_run;
+    float vT_cur = alpha * v_vis + (1.f - alpha) * S.vT_run;
+    const float t_view = H.tcam;
+    float v_t = 0.f, v_t_ndc = 0.f, v_w = 0.f;
+    if (use_ndc) {
+        const float t_ndc = (kTFar * t_view - kTFar * kTNear) / ((kTFar - kTNear) * t_view);
+        v_t_ndc = 2.f * (vis * t_ndc * S.sfin.x - vis * S.sfin.y) * S.vreg;
+        v_w = (t_ndc * t_ndc * S.sfin.x - 2.f * t_ndc * S.sfin.y + S.sfin.z) * S.vreg;
+    } else {
+        v_t = 2.f * (vis * H.t * S.sfin.x - vis * S.sfin.y) * S.vreg;
+        v_w = (H.t * H.t * S.sfin.x - 2.f * H.t * S.sfin.y + S.sfin.z) * S.vreg;
+    }
+    v_alpha += v_w * T;
+    vT_cur += v_w * alpha;
+    S.vT_run = vT_cur;
+    const float v_sigma = -nbf * opac * e * v_alpha;
+    // sigma = (l1s^2 + l2s^2) / 2 with l_ks = l_k / s_k.  A point l of the
+    // plane has a . r = (l + a . mu) / t along the ray r, so dsigma/dt = sum_k
+    // l_ks (l_ks + a_k . mu / s_k) / t, and likewise for the uv
+    float v_ray = H.l1s * v_sigma * (H.l1s + ray.x) + H.l2s * v_sigma * (H.l2s + ray.y);
+    if (prop_uv) v_ray += v_u * (duv.x + ray.z) + v_v * (duv.y + ray.w);
+    v_t += v_ray * __fdividef(1.f, H.t);
+    float v_t_view = 0.f;
+    if (idx == S.dfin) v_t_view += S.vdepth;
+    if (use_ndc) v_t_view += (kTFar * kTNear) / ((kTFar - kTNear) * t_view * t_view) * v_t_ndc;
+    v_t += P.idn * v_t_view;
+    q0 = make_float4(vis, (nbf * e + bf * eb) * v_alpha, v_sigma, v_t * (P.dn * H.inv));
+    q1 = make_float4(v_u, v_v, H.l1s, H.l2s);
+}
+
+// Texel gradients of a coarse chart (kCoarseChart): atomics of 32 lanes on the
+// same texel are served one after the other, so the lane sums a staged splat's pairs over
+// its pixels (own) as long as they fall between the same four texels.  k: the
+// lane's staged splat.
+template <int TM, int FIX>
+__device__ __forceinline__ void add_coarse_texel_grads(const BwdMem& M, const SceneArgs& a, float* __restrict__ v_texgrad,
+                                                       int k, unsigned own) {
+    const StagedRec<kBwdChunks> rec(M.rec, k);
+    const float4 nop = rec(kChunkNop), uvs = rec(kChunkUvs), uvm = rec(kChunkUvm);
+    RecHot Hr;
+    Hr.org = rec(kChunkOrg);
+    Hr.lc = make_float4(0.f, 0.f, 0.f, 0.f);
+    Hr.nop = make_float4(nop.x, nop.y, nop.z, 0.f);
+    const unsigned below = (1u << k) - 1u;
+    Bilerp cell;
+    cell.i00 = -1;
+    float acc[4][3];
+    auto flush = [&]() {
+        const int rows[4] = { cell.i00, cell.i01, cell.i10, cell.i11 };
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            if (acc[q][0] == 0.f && acc[q][1] == 0.f && acc[q][2] == 0.f) continue;
+            if (TM == 1) {
+                atomicAdd(reinterpret_cast<float4*>(v_texgrad) + rows[q],
+                          make_float4(acc[q][0], acc[q][1], acc[q][2], 0.f));
+            } else {
+                float* dst = v_texgrad + 3 * (size_t)rows[q];
+                atomicAdd(dst + 0, acc[q][0]);
+                atomicAdd(dst + 1, acc[q][1]);
+                atomicAdd(dst + 2, acc[q][2]);
+            }
+        }
+    };
+    for (; own; own &= own - 1) {
+        const int p = __ffs(own) - 1;
+        const float vis = M.pair[0][__popc(M.valid[p] & below)][p].x;
+        const float4 vt = M.pix[2][p];
+        PixelRay P;
+        P.px = M.pix[0][p].w;
+        P.py = M.pix[1][p].w;
+        P.dn = 0.f;
+        const Hit H = intersect(Hr, P);
+        const float2 t = fma2(make_float2(uvm.y, uvm.w), dup2(H.dv), mul2(make_float2(uvm.x, uvm.z), dup2(H.du)));
+        const float2 uv = fma2(t, dup2(H.inv), make_float2(uvs.x, uvs.y));
+        const Bilerp B = bilerp(__float_as_int(uvs.z), __float_as_int(uvs.w), chart_start(nop), clamp01(uv.x),
+                                clamp01(uv.y), FIX || !(a.settings & (1 << 2)));
+        if (B.i00 != cell.i00) {  // (i00 fixes the other three)
+            if (cell.i00 >= 0) flush();
+            cell = B;
+#pragma unroll
+            for (int q = 0; q < 4; q++) acc[q][0] = acc[q][1] = acc[q][2] = 0.f;
+        }
+        const float gv[3] = { vis * vt.x, vis * vt.y, vis * vt.z };
+        const float wts[4] = { B.w00, B.w01, B.w10, B.w11 };
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+#pragma unroll
+            for (int c = 0; c < 3; c++) acc[q][c] += wts[q] != 0.f ? wts[q] * gv[c] : 0.f;
+    }
+    if (cell.i00 >= 0) flush();
+}
+
+// Adds the sums of one splat over the pixels of a block to its gradients (the
+// moment layout of finalize_kernel).  m: 0-2 colour, 3 opacity, 4-6 l1^2, l2^2,
+// l1 l2 times v_sigma, 7-8 l v_sigma, 9-11 (1, l1, l2) v_t / (n . r), 12-14
+// normal, 15-16 v_uv, 17-20 l v_uv, 21-22 blur; l in units of the scales.
+template <int FIX>
+__device__ __forceinline__ void flush_moments(const float* m, const SceneArgs& a, const BlockArgs& ba, const BwdArgs& g,
+                                              const Block& J, int gid, float is1, float is2, bool use_blur) {
+    if (ba.vc_stride == 4) {
+        atomicAdd(reinterpret_cast<float4*>(J.vcolors) + gid, make_float4(m[0], m[1], m[2], 0.f));
+    } else {
+        float* vc = J.vcolors + 3 * (size_t)gid;
+        atomicAdd(vc + 0, m[0]);
+        atomicAdd(vc + 1, m[1]);
+        atomicAdd(vc + 2, m[2]);
+    }
+    float3 vmb = make_float3(0.f, 0.f, 0.f);
+    if (!FIX && use_blur) {
+        // blur moments -> world-space mean gradient (helpers.cuh:155-164, 114-121)
+        const float4 p = __ldg(J.recs[gid].c + kChunkMu);
+        const float rw = 1.f / (p.z + 1e-6f);
+        const float vx = J.fx * m[21], vy = J.fy * m[22];
+        vmb = block_view(ba, J.view).rot_t(make_float3(vx * rw, vy * rw, -(vx * p.x + vy * p.y) * rw * rw));
+    }
+    const float r1 = 1.f / is1, r2 = 1.f / is2;
+    float4* dst = reinterpret_cast<float4*>(g.moments + (size_t)gid * kMomStride);
+    atomicAdd(dst + 0, make_float4(m[3], -is1 * a.glob * m[4], -is2 * a.glob * m[5], is1 * m[7]));
+    atomicAdd(dst + 1, make_float4(is2 * m[8], m[9], m[4], is1 * r2 * m[6]));
+    atomicAdd(dst + 2, make_float4(is2 * r1 * m[6], m[5], r1 * m[10], r2 * m[11]));
+    atomicAdd(dst + 3, make_float4(m[12], m[13], m[14], m[15]));
+    atomicAdd(dst + 4, make_float4(m[16], r1 * m[17], r2 * m[18], r1 * m[19]));
+    if (FIX || !use_blur)
+        atomicAdd(reinterpret_cast<float*>(dst + 5), r2 * m[20]);
+    else
+        atomicAdd(dst + 5, make_float4(r2 * m[20], vmb.x, vmb.y, vmb.z));
+}
+
+template <int TM, int CT, int FIX>
+__global__ void __launch_bounds__(32 * kBlockWarps, kBwdCtas)
+    bwd_block_kernel(const __grid_constant__ SceneArgs a, const __grid_constant__ BlockArgs ba, BwdArgs g) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const unsigned lane = threadIdx.x & 31;
+    BwdMem& M = reinterpret_cast<BwdMem*>(smem)[threadIdx.x >> 5];
+    Block J;
+    if (!load_block(ba, (int)blockIdx.x * kBlockWarps + (int)(threadIdx.x >> 5), J)) return;
+    if (J.range.x >= J.range.y) return;
+    const bool use_blur = !FIX && (a.settings & (1 << 9)) != 0;
+    const int pi = J.y0 + lane_row(lane), pj = J.x0 + lane_col(lane);
+    const bool inside = pi < J.H && pj < J.W;
+    PixelRay P;
+    {
+        View V;
+        V.fx = J.fx; V.fy = J.fy; V.cx = J.cx; V.cy = J.cy;
+        P = make_pixel(V, pi, pj);
+    }
+    const float3 z3 = make_float3(0.f, 0.f, 0.f);
+    BwdState<CT> S;
+    const size_t pix = inside ? J.pix + (size_t)pi * J.W + pj : 0;
+    S.bfin = inside ? g.final_idx[pix] : -1;
+    // splats beyond the last contributor of the block's pixels add nothing
+    int pos = min(J.range.y - 1, __reduce_max_sync(kFull, S.bfin));
+    if (pos < J.range.x) return;
+    S.T = inside ? g.final_T[pix] : 1.f;
+    S.sfin = inside ? g.reg_s[pix] : z3;
+    S.dfin = inside ? g.depth_idx[pix] : -1;
+    S.vout = inside ? ld_or(g.v_img, pix, z3) : z3;
+    S.vdepth = inside ? ld_or(g.v_depth, pix, 0.f) : 0.f;
+    S.vreg = inside ? ld_or(g.v_reg, pix, 0.f) : 0.f;
+    S.vnorm = inside ? ld_or(g.v_normal, pix, z3) : z3;
+    const float valph = inside ? ld_or(g.v_alpha, pix, 0.f) : 0.f;
+#pragma unroll
+    for (int c = 0; c < (CT > 0 ? CT : 1); c++) S.vtex[c] = (CT > 0 && inside && g.v_tex) ? g.v_tex[pix * CT + c] : 0.f;
+    S.vT_run = a.bg[0] * S.vout.x + a.bg[1] * S.vout.y + a.bg[2] * S.vout.z - valph;
+    M.pix[0][lane] = f4(S.vout, P.px);
+    M.pix[1][lane] = f4(S.vnorm, P.py);
+    if (CT == 3) M.pix[2][lane] = make_float4(S.vtex[0], S.vtex[CT > 1 ? 1 : 0], S.vtex[CT > 2 ? 2 : 0], 0.f);
+    const float fx0 = (float)J.x0 + 0.5f, fy0 = (float)J.y0 + 0.5f;
+    const unsigned live = __ballot_sync(kFull, S.bfin >= J.range.x), below = (1u << lane) - 1u;
+    int n = 0;
+    for (;;) {
+        n = fill_queue<-1>(M.q, n, pos, J.range.x - 1, a.gids, J.recs, fx0, fy0, live, lane);
+        if (n == 0) break;
+        const int ns = min(n, 32);
+        stage_records(M.rec, M.q, ns, J.recs, lane);
+        unsigned todo = transpose32((int)lane < ns ? M.q.mask[lane] : 0u, lane);
+        if (M.q.idx[0] > S.bfin) {  // skip the splats beyond this pixel's last contributor
+            int k = 0;
+#pragma unroll
+            for (int step = 32; step > 0; step >>= 1)
+                if (k + step <= ns && M.q.idx[k + step - 1] > S.bfin) k += step;
+            todo = k >= 32 ? 0u : todo & (~0u << k);
+        }
+        if (!((live >> lane) & 1u)) todo = 0;
+        cp_async_wait();
+        __syncwarp();
+        while (__any_sync(kFull, todo != 0u)) {
+            // every lane steps back over its pixel's next pairs
+            unsigned valid = 0;
+            int r = 0;
+            while (todo && r < kRounds) {
+                const int k = __ffs(todo) - 1;
+                todo &= todo - 1;
+                const StagedRec<kBwdChunks> rec(M.rec, k);
+                float opac, nbf, bf, e, eb;
+                const int gid = M.q.gid[k];
+                const Hit H = block_hit(a, ba, J.view, rec, gid, P, opac);
+                const float alpha = block_alpha<FIX>(H, opac, use_blur, J.recs + gid, P, nbf, bf, e, eb);
+                if (H.t < kTNear || H.t > kTFar || alpha < kAlphaMin) continue;
+                float4 q0, q1;
+                pair_adjoint<TM, CT, FIX>(S, a, g, rec, H, P, M.q.idx[k], opac, alpha, nbf, bf, e, eb, q0, q1);
+                M.pair[0][r][lane] = q0;
+                M.pair[1][r][lane] = q1;
+                valid |= 1u << k;
+                r++;
+            }
+            M.valid[lane] = valid;
+            __syncwarp();
+            // sum every splat's pairs over the pixels: one lane per splat, or
+            // two or four where few splats have pairs (splats that cover the
+            // block fill the rounds with few of them)
+            unsigned mine = transpose32(valid, lane);
+            const unsigned act = __ballot_sync(kFull, mine != 0u);
+            const int na = __popc(act), shift = na <= 8 ? 2 : na <= 16 ? 1 : 0, sub = (int)lane & ((1 << shift) - 1);
+            int k = (int)lane;
+            if (shift) {
+                if (mine) M.slot[__popc(act & below)] = (uint8_t)lane;
+                __syncwarp();
+                const int j = (int)lane >> shift;
+                k = j < na ? M.slot[j] : 0;
+                mine = __shfl_sync(kFull, mine, k);
+                if (j >= na) mine = 0;
+            }
+            const unsigned own = mine & ((shift == 2 ? 0x11111111u : shift == 1 ? 0x55555555u : kFull) << sub);
+            const unsigned below_k = (1u << k) - 1u;
+            float m[FIX ? 21 : 23];
+#pragma unroll
+            for (int q = 0; q < (FIX ? 21 : 23); q++) m[q] = 0.f;
+            const float4 nop = M.rec.c[kChunkNop - kChunkOrg][k];
+            for (unsigned todo_p = own; todo_p; todo_p &= todo_p - 1) {
+                const int p = __ffs(todo_p) - 1;
+                const int r2 = __popc(M.valid[p] & below_k);  // pairs are stored in list order
+                const float4 q0 = M.pair[0][r2][p], q1 = M.pair[1][r2][p];
+                const float4 vo = M.pix[0][p], vn = M.pix[1][p];
+                const float vis = q0.x, vtd = q0.w;
+                const float vsig = FIX ? q0.y : q0.z;  // (FIX: v_sigma = -opacity times this, applied below)
+                const float2 ls = make_float2(q1.z, q1.w);
+                float2 t2 = fma2(dup2(vis), make_float2(vo.x, vo.y), make_float2(m[0], m[1]));
+                m[0] = t2.x; m[1] = t2.y;
+                m[2] += vis * vo.z;
+                m[3] += q0.y;
+                const float2 pk = mul2(ls, dup2(vsig));
+                t2 = fma2(ls, pk, make_float2(m[4], m[5]));
+                m[4] = t2.x; m[5] = t2.y;
+                m[6] += ls.x * pk.y;
+                t2 = add2(make_float2(m[7], m[8]), pk);
+                m[7] = t2.x; m[8] = t2.y;
+                m[9] += vtd;
+                t2 = fma2(ls, dup2(vtd), make_float2(m[10], m[11]));
+                m[10] = t2.x; m[11] = t2.y;
+                t2 = fma2(dup2(vis), make_float2(vn.x, vn.y), make_float2(m[12], m[13]));
+                m[12] = t2.x; m[13] = t2.y;
+                m[14] += vis * vn.z;
+                if (CT > 0) {
+                    t2 = add2(make_float2(m[15], m[16]), make_float2(q1.x, q1.y));
+                    m[15] = t2.x; m[16] = t2.y;
+                    t2 = fma2(ls, dup2(q1.x), make_float2(m[17], m[18]));
+                    m[17] = t2.x; m[18] = t2.y;
+                    t2 = fma2(ls, dup2(q1.y), make_float2(m[19], m[20]));
+                    m[19] = t2.x; m[20] = t2.y;
+                }
+                if constexpr (!FIX) {
+                    // one of the two alphas is the pair's: v_sigma_blur = -opacity e v_alpha - v_sigma
+                    if (use_blur) {
+                        const float4 c = __ldg(J.recs[M.q.gid[k]].c + kChunkMisc);
+                        const float vsb = -nop.z * q0.y - q0.z;
+                        m[21] += kBlurFsq * vsb * (c.x - vo.w);
+                        m[22] += kBlurFsq * vsb * (c.y - vn.w);
+                    }
+                }
+            }
+            __syncwarp();
+            for (int o = 1; o < 1 << shift; o <<= 1) {
+#pragma unroll
+                for (int q = 0; q < (FIX ? 21 : 23); q++) m[q] += __shfl_xor_sync(kFull, m[q], o);
+            }
+            if (mine && sub == 0) {
+                if (FIX) {
+#pragma unroll
+                    for (int q = 4; q < 9; q++) m[q] *= -nop.z;
+                }
+                flush_moments<FIX>(m, a, ba, g, J, M.q.gid[k], M.rec.c[kChunkCol - kChunkOrg][k].w,
+                                   M.rec.c[kChunkNrm - kChunkOrg][k].w, use_blur);
+            }
+            if (CT == 3) {
+                const unsigned coarse = is_coarse(nop) ? own : 0u;
+                if (coarse) add_coarse_texel_grads<TM, FIX>(M, a, g.v_texgrad, k, coarse);
+            }
+            __syncwarp();
+        }
+        n = pop_queue(M.q, n, lane);
+    }
+}
+
+// ---------------------------------------------------------------------------
 // Launches
 // ---------------------------------------------------------------------------
 // The block kernels take tile widths that are multiples of 8 (8 or 16), no
@@ -479,6 +903,24 @@ int launch_fwd_blocks(const SceneArgs& a, const BlockArgs& ba, const FwdOut& o, 
     else k = fix ? fwd_block_kernel<0, 3, 1> : fwd_block_kernel<0, 3, 0>;
     k<<<(unsigned)grid, 32 * kBlockWarps, 0, stream>>>(a, ba, o);
     return check_launch("forward blocks");
+}
+
+int launch_bwd_blocks(const SceneArgs& a, const BlockArgs& ba, const BwdArgs& g, int texmode, cudaStream_t stream) {
+    const long long blocks = (long long)ba.total_tiles * ((ba.bw >> 3) * (ba.bw >> 2));
+    const long long grid = (blocks + kBlockWarps - 1) / kBlockWarps;
+    if (grid > 0x7fffffffLL) return GSTEX_ERR_UNSUPPORTED;
+    const bool fix = (a.settings & kFixedBwdMask) == kFixedBwdSettings;
+    void (*k)(const SceneArgs, const BlockArgs, BwdArgs);
+    if (a.C == 0) k = fix ? bwd_block_kernel<0, 0, 1> : bwd_block_kernel<0, 0, 0>;
+    else if (texmode == 1) k = fix ? bwd_block_kernel<1, 3, 1> : bwd_block_kernel<1, 3, 0>;
+    else k = fix ? bwd_block_kernel<0, 3, 1> : bwd_block_kernel<0, 3, 0>;
+    const size_t smem = sizeof(BwdMem) * kBlockWarps;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
+    if (e != cudaSuccess) { set_cuda_error(e, "backward blocks"); return GSTEX_ERR_CUDA; }
+    k<<<(unsigned)grid, 32 * kBlockWarps, smem, stream>>>(a, ba, g);
+    return check_launch("backward blocks");
 }
 
 }  // namespace gstex

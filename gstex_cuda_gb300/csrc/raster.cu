@@ -51,7 +51,8 @@ __device__ __forceinline__ void stage_job(const Recs& R, int slot, const SceneAr
         w.uvs = make_float4(uvs.x, uvs.y, misc.x, misc.y);
         w.col = __ldg(src + kChunkCol);
         w.nrm = __ldg(src + kChunkNrm);
-        w.tex = make_int4(__float_as_int(uvs.z), __float_as_int(uvs.w), __float_as_int(nop.w), __float_as_int(misc.w));
+        w.tex = make_int4(__float_as_int(uvs.z), __float_as_int(uvs.w), (int)(__float_as_uint(nop.w) & ~kCoarseChart),
+                           __float_as_int(misc.w));
         c.mu = __ldg(src + kChunkMu);
         c.dt = __ldg(src + kChunkDt);
         if (R.cull) {
@@ -1458,6 +1459,7 @@ static int set_bwd_smem(K k, size_t smem, const char* what) {
 
 int launch_bwd_batch(const SceneArgs& a, const BatchArgs& ba, const BwdArgs& g, int bw, int texmode, int ppt, int gs,
                      int ctas, int grid, cudaStream_t stream) {
+    if (blocks_apply(bw, a.C, a.settings, ba.recs)) return launch_bwd_blocks(a, block_args(ba, bw), g, texmode, stream);
     ppt = ppt_of(bw, ppt);
     gs = gs_of(bw, ppt, a.C, gs);
     auto k = pick_bwd_batch(bw, a.C, texmode, ppt, gs, ctas, a.settings);
@@ -1636,14 +1638,18 @@ extern "C" int gstex_texture_backward(const gstex_raster_inputs* in, const gstex
     const int bw = in->block_width;
     ViewArgs va = view_args(in);
     va.vcolors = io->v_colors;
-    const dim3 grid(va.tiles_x, ceil_div(va.H, bw));
-    const int ppt = ppt_of(bw, in->pixels_per_thread);
-    const int gs = gs_of(bw, ppt, a.C, in->group_lanes);
-    auto k = pick<BwdView>(a.C, in->texture_dtype, ppt, gs);
-    const size_t smem = bwd_smem(bw, ppt, gs, 0);
-    if ((rc = set_smem(k, smem, "texture_backward"))) return rc;
-    k<<<grid, block_of(bw, ppt), smem, stream>>>(a, va, g);
-    if ((rc = check_launch("texture_backward"))) return rc;
+    if (blocks_apply(bw, a.C, a.settings, va.recs)) {
+        if ((rc = launch_bwd_blocks(a, block_args(va, bw, a.N), g, in->texture_dtype, stream))) return rc;
+    } else {
+        const dim3 grid(va.tiles_x, ceil_div(va.H, bw));
+        const int ppt = ppt_of(bw, in->pixels_per_thread);
+        const int gs = gs_of(bw, ppt, a.C, in->group_lanes);
+        auto k = pick<BwdView>(a.C, in->texture_dtype, ppt, gs);
+        const size_t smem = bwd_smem(bw, ppt, gs, 0);
+        if ((rc = set_smem(k, smem, "texture_backward"))) return rc;
+        k<<<grid, block_of(bw, ppt), smem, stream>>>(a, va, g);
+        if ((rc = check_launch("texture_backward"))) return rc;
+    }
     return launch_finalize(a, (const float*)io->workspace, io->v_opacity, io->v_means, io->v_scales, io->v_quats,
                            io->v_uv0, io->v_umap, io->v_vmap, stream);
 }

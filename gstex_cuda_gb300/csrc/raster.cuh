@@ -154,6 +154,7 @@ constexpr int kFixedBwdSettings = 1 << 8;
 constexpr int kFixedFwdMask = (1 << 2) | (1 << 9) | (1 << 10) | (1 << 15) | (1 << 16);
 bool blocks_apply(int bw, int C, int settings, const RecAll* recs);
 int launch_fwd_blocks(const SceneArgs& a, const BlockArgs& ba, const FwdOut& o, int texmode, cudaStream_t stream);
+int launch_bwd_blocks(const SceneArgs& a, const BlockArgs& ba, const BwdArgs& g, int texmode, cudaStream_t stream);
 int launch_records(const SceneArgs& a, const BatchArgs& ba, int num_views, const int32_t* counts, RecAll* recs,
                    int* fix_count, uint32_t* fix, cudaStream_t stream);
 
