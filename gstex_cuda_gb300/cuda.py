@@ -166,6 +166,42 @@ def get_tile_bin_edges(num_intersects, isect_ids_sorted, tile_bounds):
     return bins
 
 
+def bin_view(centers, extents, depths, num_tiles_hit, tile_bounds, block_width):
+    """Depth-first binning of one view: (number of intersections,
+    gaussian_ids_sorted, tile_bins), equal to the scan, emission, sort and
+    ranges of the functions above.  Reads the number back to the host."""
+    _chk(("centers", centers), ("extents", extents), ("depths", depths), ("num_tiles_hit", num_tiles_hit))
+    _i32("num_tiles_hit", num_tiles_hit)
+    n = min(num_tiles_hit.shape[0], centers.shape[0])
+    L = _lib.lib()
+    dev = num_tiles_hit.device
+    st = _lib.stream_of(num_tiles_hit)
+    order = torch.empty((2, n), dtype=torch.int32, device=dev)  # depth order, inclusive slot sums
+    info = torch.empty(2, dtype=torch.int64, device=dev)
+    wsb = L.gstex_view_order_workspace_bytes(n)
+    ws = torch.empty(wsb, dtype=torch.uint8, device=dev)
+    check(L.gstex_view_order(n, ptr(depths), ptr(num_tiles_hit), ptr(order[0]), ptr(order[1]), ptr(info), ptr(ws), wsb,
+                             st), "view_order")
+    total, ties = info.tolist()
+    if total >= 2 ** 31:
+        raise OverflowError(f"{total} intersections exceed the int32 range of the reference's cumsum")
+    if ties:  # depths of +0: the order of the 64-bit keys
+        cum, _ = inclusive_scan(num_tiles_hit)
+        keys, ids = map_gaussian_to_intersects(n, total, centers, extents, depths, cum, tile_bounds, block_width)
+        num_tiles = int(tile_bounds[0]) * int(tile_bounds[1])
+        keys, ids = sort_pairs(keys, ids, sort_end_bit(num_tiles))
+        return total, ids, get_tile_bin_edges(total, keys, tile_bounds)
+    total = max(total, 0)
+    gids = torch.empty(total, dtype=torch.int32, device=dev)
+    bins = torch.empty((int(tile_bounds[0]) * int(tile_bounds[1]), 2), dtype=torch.int32, device=dev)
+    wsb = L.gstex_view_bins_workspace_bytes(total)
+    ws = torch.empty(wsb, dtype=torch.uint8, device=dev)
+    check(L.gstex_view_bins(n, total, ptr(centers), ptr(extents), ptr(depths), ptr(order[0]), ptr(order[1]),
+                            int(tile_bounds[0]), int(tile_bounds[1]), int(block_width), ptr(gids), ptr(bins), ptr(ws),
+                            wsb, st), "view_bins")
+    return total, gids, bins
+
+
 # ---------------------------------------------------------------------------
 # compositor (csrc/texture.cu:762-1053)
 # ---------------------------------------------------------------------------

@@ -14,7 +14,7 @@ from torch import Tensor
 from torch.autograd import Function
 
 from . import cuda as _C
-from .utils import bin_and_sort_gaussians, compute_cumulative_intersects
+from .utils import bin_view
 
 
 def texture_gaussians(texture_info: Tuple[int, int, int], texture_dims: Tensor, centers: Tensor, extents: Tensor,
@@ -56,20 +56,13 @@ class _TextureGaussians(Function):
     def forward(ctx, texture_info, texture_dims, centers, extents, depths, num_tiles_hit, colors, opacity, means,
                 scales, glob_scale, quats, uv0, umap, vmap, texture, viewmat, c2w, fx, fy, cx, cy, img_height,
                 img_width, block_width, settings, background):
-        num_points = centers.size(0)
         tile_bounds = ((img_width + block_width - 1) // block_width, (img_height + block_width - 1) // block_width, 1)
         block = (block_width, block_width, 1)
         img_size = (img_width, img_height, 1)
-        num_intersects, cum_tiles_hit = compute_cumulative_intersects(num_tiles_hit)
-        dev = centers.device
-        if num_intersects < 1:
-            # No splat touches the image.  (The reference's branch for this case,
-            # gstex_cuda/texture.py:197-205, leaves most outputs undefined.)
-            gaussian_ids_sorted = torch.zeros(0, dtype=torch.int32, device=dev)
-            tile_bins = torch.zeros(tile_bounds[0] * tile_bounds[1], 2, dtype=torch.int32, device=dev)
-        else:
-            _, _, _, gaussian_ids_sorted, tile_bins = bin_and_sort_gaussians(
-                num_points, num_intersects, centers, extents, depths, cum_tiles_hit, tile_bounds, block_width)
+        # (with no intersections the lists are empty; the reference's branch for
+        # this case, gstex_cuda/texture.py:197-205, leaves most outputs undefined)
+        num_intersects, gaussian_ids_sorted, tile_bins = bin_view(centers, extents, depths, num_tiles_hit, tile_bounds,
+                                                                  block_width)
         outs = _C.texture_forward(tile_bounds, block, img_size, texture_info, texture_dims, gaussian_ids_sorted,
                                   tile_bins, colors, opacity, means, scales, glob_scale, quats, uv0, umap, vmap,
                                   texture, viewmat, c2w, fx, fy, cx, cy, settings, background)

@@ -14,7 +14,7 @@ import torch
 from torch import Tensor
 
 from . import cuda as _C
-from .utils import bin_and_sort_gaussians, compute_cumulative_intersects
+from .utils import bin_view
 
 
 def texture_edit(texture_info: Tuple[int, int, int], texture_dims: Tensor, updated_img: Tensor,
@@ -31,16 +31,14 @@ def texture_edit(texture_info: Tuple[int, int, int], texture_dims: Tensor, updat
     assert 1 < block_width <= 16, "block_width must be between 2 and 16"
     if use_torch_impl:
         raise NotImplementedError("texture_edit has only a CUDA implementation (as in the reference)")
-    num_points = centers.size(0)
     tile_bounds = ((img_width + block_width - 1) // block_width, (img_height + block_width - 1) // block_width, 1)
     block = (block_width, block_width, 1)
     img_size = (img_width, img_height, 1)
     texture_total_size = int(torch.sum(texture_dims[:, 0].long() * texture_dims[:, 1].long()).item())
-    num_intersects, cum_tiles_hit = compute_cumulative_intersects(num_tiles_hit)
+    num_intersects, gaussian_ids_sorted, tile_bins = bin_view(centers, extents, depths, num_tiles_hit, tile_bounds,
+                                                              block_width)
     if num_intersects < 1:
         raise ValueError("texture_edit: no Gaussian intersects the image")
-    _, _, _, gaussian_ids_sorted, tile_bins = bin_and_sort_gaussians(
-        num_points, num_intersects, centers, extents, depths, cum_tiles_hit, tile_bounds, block_width)
     if background is None:
         background = torch.zeros(3, device=means.device)
     return _C.texture_edit(tile_bounds, block, img_size, texture_info, texture_total_size, texture_dims.contiguous(),

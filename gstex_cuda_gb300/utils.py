@@ -54,3 +54,14 @@ def bin_and_sort_gaussians(num_points: int, num_intersects: int, centers: Tensor
     isect_sorted, gids_sorted = _C.sort_pairs(isect_ids, gaussian_ids, _C.sort_end_bit(num_tiles))
     tile_bins = get_tile_bin_edges(num_intersects, isect_sorted, tile_bounds)
     return isect_ids, gaussian_ids, isect_sorted, gids_sorted, tile_bins
+
+
+def bin_view(centers: Tensor, extents: Tensor, depths: Tensor, num_tiles_hit: Tensor,
+             tile_bounds: Tuple[int, int, int], block_size: int) -> Tuple[int, Tensor, Tensor]:
+    """(num_intersects, gaussian_ids_sorted, tile_bins) of one view: what
+    compute_cumulative_intersects and bin_and_sort_gaussians give a renderer,
+    without the 64-bit intersection keys."""
+    counts = num_tiles_hit.contiguous()
+    if counts.dtype != torch.int32:
+        counts = counts.to(torch.int32)
+    return _C.bin_view(centers.contiguous(), extents.contiguous(), depths.contiguous(), counts, tile_bounds, block_size)

@@ -146,6 +146,25 @@ int gstex_sort_pairs32(int n, const int64_t* count, int end_bit, const uint32_t*
 int gstex_get_tile_bin_edges32_dyn(int capacity, const int64_t* count, const uint32_t* keys_sorted, int shift,
                                    int num_tiles, int32_t* tile_bins, gstex_stream_t stream);
 
+/* Depth-first binning of one view: the gaussian_ids_sorted and tile_bins of
+ * bin_and_sort_gaussians (gstex_cuda/utils.py:106-161) without its 64-bit
+ * intersection keys, bit for bit.
+ *   1. gstex_view_order: the Gaussians in (stable) depth order, the inclusive
+ *      sums of their tile counts in that order, and info[0] = their total,
+ *      info[1] = 1 if a Gaussian with tiles has depth +0 (such depths tie with
+ *      the zero entries of unwritten slots: sort 64-bit keys instead);
+ *   2. the caller reads info (the total sizes the next step's buffers);
+ *   3. gstex_view_bins: emission in that order, a stable sort by tile, ranges.
+ * Workspaces 16-byte aligned. */
+size_t gstex_view_order_workspace_bytes(int n);
+int gstex_view_order(int n, const float* depths, const int32_t* num_tiles_hit, int32_t* order, int32_t* cum,
+                     int64_t* info, void* workspace, size_t workspace_bytes, gstex_stream_t stream);
+size_t gstex_view_bins_workspace_bytes(int num_intersects);
+int gstex_view_bins(int n, int num_intersects, const float* centers, const float* extents, const float* depths,
+                    const int32_t* order, const int32_t* cum, int tiles_x, int tiles_y, int block_width,
+                    int32_t* gaussian_ids_sorted, int32_t* tile_bins, void* workspace, size_t workspace_bytes,
+                    gstex_stream_t stream);
+
 /* ---------------------------------------------------------------------
  * Textured compositor (texture_forward / texture_backward)
  * ------------------------------------------------------------------- */
