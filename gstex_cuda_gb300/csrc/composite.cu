@@ -473,24 +473,27 @@ __global__ void __launch_bounds__(32 * kBlockWarps, kFwdCtas)
 //
 // What bounds it: the L1 data path (71% of its cycles; a 16-byte reduction
 // takes about a cycle per lane there) and the latency of its chains at 16 warps
-// per SM.  Of 23.6 ms on 32 views (36.6 ms with the list walk, its moment
+// per SM.  Of 22.8 ms on 32 views (36.6 ms with the list walk, its moment
 // reduction by shuffles and 8-lane groups) the scan, staging and ray-plane
 // solves take 6 ms, the adjoint 4, texel reads 3.5, texel atomics 4 and the
-// sums 6.  8 clustered full-HD views: 22.3 -> 14.4 ms; one 800x800 view of 1x1
-// charts 254 -> 111 us; one full-HD view of large splats 36.0 -> 8.7 ms (where
+// sums 5.  8 clustered full-HD views: 22.3 -> 13.7 ms; one 800x800 view of 1x1
+// charts 254 -> 111 us; one full-HD view of large splats 36.0 -> 8.4 ms (where
 // the list walk also staged every splat behind the last contributor).
 // ---------------------------------------------------------------------------
 constexpr int kBwdChunks = 8;
-// Pairs per pixel between two summations, and CTAs per SM (at most 128
-// registers): 7 rounds are what fits 8 CTAs' shared memory.  6 and 8: 2% slower;
-// 5 and 9: 16%; 9 and 7: 9% (32 views).
-constexpr int kRounds = 7;
+// Pairs between two summations, and CTAs per SM (at most 128 registers): what
+// fits 8 CTAs' shared memory (32 staged splats have 230 pairs on average; with
+// 192, 1% slower).  Pairs are placed splat by splat, so the room is used up and
+// a splat is summed once: 7 rounds of one pair per pixel in the same room took
+// 23.6 instead of 22.8 ms on 32 views, 14.4 instead of 13.7 ms on 8 clustered
+// ones.
+constexpr int kPairs = 224;
 constexpr int kBwdCtas = 8;
 struct BwdMem {
     Staged<kBwdChunks> rec;
-    float4 pair[2][kRounds][33];  // (vis, e v_alpha, v_sigma, v_t / (n . r)), (v_u, v_v, l1s, l2s) of a pixel's pairs
+    float4 pair[2][kPairs];       // (vis, e v_alpha, v_sigma, v_t / (n . r)), (v_u, v_v, l1s, l2s), splat by splat
     float4 pix[3][32];            // upstream colour, normal and texture gradients of the pixels (w: centre x, y)
-    unsigned valid[32];           // staged splats of a pixel's pairs
+    uint2 place[32];              // first pair of a staged splat; its pixels that may have one
     uint8_t slot[32];             // splats with pairs
     Queue q;
 };
@@ -621,17 +624,16 @@ __device__ __forceinline__ void pair_adjoint(BwdState<CT>& S, const SceneArgs& a
 // Texel gradients of a coarse chart (kCoarseChart): atomics of 32 lanes on the
 // same texel are served one after the other, so the lane sums a staged splat's pairs over
 // its pixels (own) as long as they fall between the same four texels.  k: the
-// lane's staged splat.
+// lane's staged splat, whose pairs start at `first` in the order of `may`.
 template <int TM, int FIX>
 __device__ __forceinline__ void add_coarse_texel_grads(const BwdMem& M, const SceneArgs& a, float* __restrict__ v_texgrad,
-                                                       int k, unsigned own) {
+                                                       int k, unsigned own, unsigned may, int first) {
     const StagedRec<kBwdChunks> rec(M.rec, k);
     const float4 nop = rec(kChunkNop), uvs = rec(kChunkUvs), uvm = rec(kChunkUvm);
     RecHot Hr;
     Hr.org = rec(kChunkOrg);
     Hr.lc = make_float4(0.f, 0.f, 0.f, 0.f);
     Hr.nop = make_float4(nop.x, nop.y, nop.z, 0.f);
-    const unsigned below = (1u << k) - 1u;
     Bilerp cell;
     cell.i00 = -1;
     float acc[4][3];
@@ -653,7 +655,7 @@ __device__ __forceinline__ void add_coarse_texel_grads(const BwdMem& M, const Sc
     };
     for (; own; own &= own - 1) {
         const int p = __ffs(own) - 1;
-        const float vis = M.pair[0][__popc(M.valid[p] & below)][p].x;
+        const float vis = M.pair[0][first + __popc(may & ((1u << p) - 1u))].x;
         const float4 vt = M.pix[2][p];
         PixelRay P;
         P.px = M.pix[0][p].w;
@@ -774,13 +776,26 @@ __global__ void __launch_bounds__(32 * kBlockWarps, kBwdCtas)
         if (!((live >> lane) & 1u)) todo = 0;
         cp_async_wait();
         __syncwarp();
-        while (__any_sync(kFull, todo != 0u)) {
-            // every lane steps back over its pixel's next pairs
+        // room for the pairs: splat by splat, in pixel order; as many splats at
+        // a time as there is room for
+        const unsigned may = transpose32(todo, lane);
+        int last = __popc(may);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(kFull, last, o);
+            if ((int)lane >= o) last += y;
+        }
+        const int total = __shfl_sync(kFull, last, 31);
+        const int first = last - __popc(may);
+        M.place[lane] = make_uint2((unsigned)first, may);
+        for (int base = 0; base < total;) {
+            const unsigned fits = __ballot_sync(kFull, first >= base && last - base <= kPairs);
+            const int stop = __shfl_sync(kFull, last, 31 - __clz(fits));
+            __syncwarp();
+            // every lane steps back over its pixel's pairs
             unsigned valid = 0;
-            int r = 0;
-            while (todo && r < kRounds) {
-                const int k = __ffs(todo) - 1;
-                todo &= todo - 1;
+            for (unsigned bits = todo & fits; bits; bits &= bits - 1) {
+                const int k = __ffs(bits) - 1;
                 const StagedRec<kBwdChunks> rec(M.rec, k);
                 float opac, nbf, bf, e, eb;
                 const int gid = M.q.gid[k];
@@ -789,16 +804,16 @@ __global__ void __launch_bounds__(32 * kBlockWarps, kBwdCtas)
                 if (H.t < kTNear || H.t > kTFar || alpha < kAlphaMin) continue;
                 float4 q0, q1;
                 pair_adjoint<TM, CT, FIX>(S, a, g, rec, H, P, M.q.idx[k], opac, alpha, nbf, bf, e, eb, q0, q1);
-                M.pair[0][r][lane] = q0;
-                M.pair[1][r][lane] = q1;
+                const uint2 pl = M.place[k];
+                const int at = (int)pl.x - base + __popc(pl.y & below);
+                M.pair[0][at] = q0;
+                M.pair[1][at] = q1;
                 valid |= 1u << k;
-                r++;
             }
-            M.valid[lane] = valid;
             __syncwarp();
             // sum every splat's pairs over the pixels: one lane per splat, or
             // two or four where few splats have pairs (splats that cover the
-            // block fill the rounds with few of them)
+            // block fill the room with few of them)
             unsigned mine = transpose32(valid, lane);
             const unsigned act = __ballot_sync(kFull, mine != 0u);
             const int na = __popc(act), shift = na <= 8 ? 2 : na <= 16 ? 1 : 0, sub = (int)lane & ((1 << shift) - 1);
@@ -812,15 +827,15 @@ __global__ void __launch_bounds__(32 * kBlockWarps, kBwdCtas)
                 if (j >= na) mine = 0;
             }
             const unsigned own = mine & ((shift == 2 ? 0x11111111u : shift == 1 ? 0x55555555u : kFull) << sub);
-            const unsigned below_k = (1u << k) - 1u;
+            const uint2 pl = M.place[k];
             float m[FIX ? 21 : 23];
 #pragma unroll
             for (int q = 0; q < (FIX ? 21 : 23); q++) m[q] = 0.f;
             const float4 nop = M.rec.c[kChunkNop - kChunkOrg][k];
             for (unsigned todo_p = own; todo_p; todo_p &= todo_p - 1) {
                 const int p = __ffs(todo_p) - 1;
-                const int r2 = __popc(M.valid[p] & below_k);  // pairs are stored in list order
-                const float4 q0 = M.pair[0][r2][p], q1 = M.pair[1][r2][p];
+                const int at = (int)pl.x - base + __popc(pl.y & ((1u << p) - 1u));
+                const float4 q0 = M.pair[0][at], q1 = M.pair[1][at];
                 const float4 vo = M.pix[0][p], vn = M.pix[1][p];
                 const float vis = q0.x, vtd = q0.w;
                 const float vsig = FIX ? q0.y : q0.z;  // (FIX: v_sigma = -opacity times this, applied below)
@@ -874,9 +889,10 @@ __global__ void __launch_bounds__(32 * kBlockWarps, kBwdCtas)
             }
             if (CT == 3) {
                 const unsigned coarse = is_coarse(nop) ? own : 0u;
-                if (coarse) add_coarse_texel_grads<TM, FIX>(M, a, g.v_texgrad, k, coarse);
+                if (coarse) add_coarse_texel_grads<TM, FIX>(M, a, g.v_texgrad, k, coarse, pl.y, (int)pl.x - base);
             }
             __syncwarp();
+            base = stop;
         }
         n = pop_queue(M.q, n, lane);
     }
