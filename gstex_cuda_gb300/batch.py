@@ -70,6 +70,7 @@ _BATCH_SIGS = {
     "gstex_get_tile_bin_edges32_dyn": (_I, [_I, _P, _P, _I, _I, _P, _P]),
     "gstex_batch_tile_order_workspace_bytes": (ctypes.c_size_t, [_I]),
     "gstex_batch_tile_order": (_I, [_I, _P, _P, _P, _I, _P, _P, ctypes.c_size_t, _P]),
+    "gstex_batch_tile_order_small": (_I, [_I, _P, _P, _P, _P]),
     "gstex_batch_emit": (_I, [_I, _I, _P, _P, _P, _F, _P, _I, _P, _P, _LL, _P, _P, _P, _P, _P]),
     "gstex_sort_pairs_dyn": (_I, [_I, _P, _I, _P, _P, _P, _P, _P, ctypes.c_size_t, _P]),
     "gstex_get_tile_bin_edges_dyn": (_I, [_I, _P, _P, _I, _P, _P]),
@@ -275,6 +276,7 @@ class BatchRenderer:
         self.tile_order = torch.empty(self.total_tiles, **i32) if heavy_first else None
         self.order_ws = (torch.empty(L.gstex_batch_tile_order_workspace_bytes(self.total_tiles), **u8)
                          if heavy_first else None)
+        self._order_groups = self._tile_groups() if heavy_first else None
         self.queue = torch.zeros(1, **i32)
         self.bg = torch.tensor(list(background), **f32)
         # per-pixel outputs of all views
@@ -294,6 +296,23 @@ class BatchRenderer:
         self.side = torch.cuda.Stream(dev)
         self.ev_fork = torch.cuda.Event()
         self.ev_join = torch.cuda.Event()
+
+    MAX_SMALL_GROUPS = 4096  # tile groups that gstex_batch_tile_order_small takes
+
+    def _tile_groups(self):
+        """Groups of order_group^2 neighbouring tiles of a view, in tile order
+        ([n, 4]: first tile, tiles per row, width, height), with the
+        order_group they were made for; None in their place if there are too
+        many for the one-launch order."""
+        G, rows, off = self.order_group, [], 0
+        for h, w in self.sizes:
+            tx, ty = (w + self.bw - 1) // self.bw, (h + self.bw - 1) // self.bw
+            if G < 1 or len(rows) + ((tx + G - 1) // G) * ((ty + G - 1) // G) > self.MAX_SMALL_GROUPS:
+                return G, None
+            rows += [(off + y * tx + x, tx, min(G, tx - x), min(G, ty - y))
+                     for y in range(0, ty, G) for x in range(0, tx, G)]
+            off += tx * ty
+        return G, torch.tensor(rows, dtype=torch.int32).to(self.dev)
 
     def _alloc_isect(self):
         L = _L()
@@ -403,7 +422,13 @@ class BatchRenderer:
                                    self.sort_ws.numel(), st), "sort_pairs32")
         check(L.gstex_get_tile_bin_edges32_dyn(self.capacity, ptr(self.count), ptr(self.keys_sorted), 1,
                                                self.total_tiles, ptr(self.bins), st), "tile_bin_edges32_dyn")
-        if self.tile_order is not None:
+        if self.tile_order is not None and self._order_groups[0] != self.order_group:
+            self._order_groups = self._tile_groups()
+        groups = self._order_groups[1] if self.tile_order is not None else None
+        if groups is not None:
+            check(L.gstex_batch_tile_order_small(groups.shape[0], ptr(groups), ptr(self.bins), ptr(self.tile_order),
+                                                 st), "batch_tile_order_small")
+        elif self.tile_order is not None:
             check(L.gstex_batch_tile_order(self.total_tiles, ptr(self.bins), ptr(self.tile_view), ptr(self.views_dev),
                                            self.order_group, ptr(self.tile_order), ptr(self.order_ws),
                                            self.order_ws.numel(), st), "batch_tile_order")

@@ -628,6 +628,45 @@ __global__ void __launch_bounds__(kSmallThreads) view_bins_small_kernel(
     }
 }
 
+// The forward's queue order (tile_group_keys_kernel) of up to kSmallItems
+// groups of tiles in one launch.  groups[i]: first tile, tiles per row of its
+// view, width and height in tiles, in tile order.  (Sorting the tiles takes two
+// sorts, six passes or more of three launches: 96 us for 3 to 18 thousand
+// tiles, 17 to 20 here.)
+__global__ void __launch_bounds__(kSmallThreads) tile_order_small_kernel(int n, const int4* __restrict__ groups,
+                                                                         const int2* __restrict__ bins,
+                                                                         int32_t* __restrict__ order) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    SmallSort& S = *reinterpret_cast<SmallSort*>(smem);
+    for (int i = threadIdx.x; i < n; i += kSmallThreads) {
+        const int4 g = groups[i];
+        uint32_t cost = 0;
+        for (int y = 0; y < g.w; y++)
+            for (int x = 0; x < g.z; x++) {
+                const int2 b = bins[g.x + y * g.y + x];
+                cost += (uint32_t)max(b.y - b.x, 0);
+            }
+        S.key[0][i] = ~cost;
+        S.val[0][i] = (uint32_t)i;
+    }
+    __syncthreads();
+    const int at = small_sort(S, n, 32);
+    // positions of the groups' tiles: exclusive sums of their sizes in order
+    int4 g[kSmallPer];
+    uint32_t sum = 0, all;
+#pragma unroll
+    for (int r = 0; r < kSmallPer; r++) {
+        const int i = (int)threadIdx.x * kSmallPer + r;
+        g[r] = i < n ? groups[S.val[at][i]] : make_int4(0, 0, 0, 0);
+        sum += (uint32_t)(g[r].z * g[r].w);
+    }
+    uint32_t to = small_scan(sum, S.wsum, &all);
+#pragma unroll
+    for (int r = 0; r < kSmallPer; r++)
+        for (int y = 0; y < g[r].w; y++)
+            for (int x = 0; x < g[r].z; x++) order[to++] = g[r].x + y * g[r].y + x;
+}
+
 static size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 }  // namespace gstex
@@ -848,4 +887,18 @@ extern "C" int gstex_view_bins(int n, int num_isect, const float* centers, const
     bin_edges_kernel<uint32_t><<<ceil_div(num_isect, 256 * kEdgeItems), 256, 0, stream>>>(num_isect, nullptr, sorted, 1,
                                                                                           num_tiles, (int2*)bins);
     return check_launch("view_bins");
+}
+
+extern "C" int gstex_batch_tile_order_small(int num_groups, const int32_t* groups, const int32_t* tile_bins,
+                                            int32_t* order, gstex_stream_t s) {
+    GSTEX_REQUIRE(num_groups >= 0);
+    if (num_groups == 0) return GSTEX_OK;
+    GSTEX_REQUIRE(groups && ((uintptr_t)groups & 15) == 0 && tile_bins && order);
+    if (num_groups > kSmallItems) return GSTEX_ERR_UNSUPPORTED;
+    cudaError_t e = cudaFuncSetAttribute(tile_order_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)sizeof(SmallSort));
+    if (e != cudaSuccess) { set_cuda_error(e, "batch_tile_order"); return GSTEX_ERR_CUDA; }
+    tile_order_small_kernel<<<1, kSmallThreads, sizeof(SmallSort), (cudaStream_t)s>>>(
+        num_groups, (const int4*)groups, (const int2*)tile_bins, order);
+    return check_launch("batch_tile_order");
 }

@@ -383,6 +383,12 @@ size_t gstex_batch_tile_order_workspace_bytes(int total_tiles);
 int gstex_batch_tile_order(int total_tiles, const int32_t* tile_bins, const int32_t* tile_view,
                            const void* views_dev, int group, int32_t* order, void* workspace,
                            size_t workspace_bytes, gstex_stream_t stream);
+/* The same order in one launch, for up to 4096 groups given by the caller in
+ * tile order: groups [num_groups, 4] int32 (first tile, tiles per row of its
+ * view, width, height in tiles), 16-byte aligned; together they hold every
+ * tile once. */
+int gstex_batch_tile_order_small(int num_groups, const int32_t* groups, const int32_t* tile_bins, int32_t* order,
+                                 gstex_stream_t stream);
 
 typedef struct gstex_batch_inputs {
     int num_points, num_views, block_width;
