@@ -304,15 +304,17 @@ class BatchRenderer:
         ([n, 4]: first tile, tiles per row, width, height), with the
         order_group they were made for; None in their place if there are too
         many for the one-launch order."""
-        G, rows, off = self.order_group, [], 0
+        G, rows, off, n = self.order_group, [], 0, 0
         for h, w in self.sizes:
             tx, ty = (w + self.bw - 1) // self.bw, (h + self.bw - 1) // self.bw
-            if G < 1 or len(rows) + ((tx + G - 1) // G) * ((ty + G - 1) // G) > self.MAX_SMALL_GROUPS:
+            n += ((tx + G - 1) // G) * ((ty + G - 1) // G) if G >= 1 else self.MAX_SMALL_GROUPS + 1
+            if n > self.MAX_SMALL_GROUPS:
                 return G, None
-            rows += [(off + y * tx + x, tx, min(G, tx - x), min(G, ty - y))
-                     for y in range(0, ty, G) for x in range(0, tx, G)]
+            y, x = torch.meshgrid(torch.arange(0, ty, G), torch.arange(0, tx, G), indexing="ij")
+            rows.append(torch.stack([off + y * tx + x, torch.full_like(x, tx), (tx - x).clamp(max=G),
+                                     (ty - y).clamp(max=G)], -1).reshape(-1, 4))
             off += tx * ty
-        return G, torch.tensor(rows, dtype=torch.int32).to(self.dev)
+        return G, torch.cat(rows).to(torch.int32).to(self.dev)
 
     def _alloc_isect(self):
         L = _L()

@@ -119,5 +119,30 @@ __device__ __forceinline__ int sh_basis(int deg, float3 dir, float* Y) {
     return 25;
 }
 
+// Rows of R values per Gaussian (SH coefficients) between device memory and
+// one row per thread.  A thread that walks its own row of 48 values touches
+// another line with every lane of every access; the block moves its rows
+// through shared memory instead, lane after lane along the memory.  Shared rows
+// of an odd length keep a warp's own rows on different banks.
+template <int R>
+struct RowStage {
+    static constexpr int kRows = 128;  // rows of a block (threads)
+    static constexpr int kLen = R | 1;
+    float v[kRows * kLen];
+    // rows [i0, i0 + n) of g; all threads of the block, ends with a barrier
+    template <typename T>
+    __device__ __forceinline__ void load(const T* __restrict__ g, int i0, int n) {
+        const T* src = g + (size_t)i0 * R;
+        for (int k = threadIdx.x; k < n * R; k += kRows) v[k / R * kLen + k % R] = (float)src[k];
+        __syncthreads();
+    }
+    // begins with a barrier (the rows are written by their threads)
+    __device__ __forceinline__ void store(float* __restrict__ g, int i0, int n) {
+        __syncthreads();
+        float* dst = g + (size_t)i0 * R;
+        for (int k = threadIdx.x; k < n * R; k += kRows) dst[k] = v[k / R * kLen + k % R];
+    }
+    __device__ __forceinline__ float* row() { return v + threadIdx.x * kLen; }
+};
 
 }  // namespace gstex
