@@ -56,6 +56,7 @@ _SIGS = {
     "gstex_version": (ctypes.c_char_p, []),
     "gstex_launch_count": (ctypes.c_ulonglong, []),
     "gstex_get_aabb_2d": (_I, [_I, _P, _P, _F, _P, _P, _F, _F, _F, _F, _P, _P, _P]),
+    "gstex_project_points": (_I, [_I, _P, _P, _F, _F, _F, _F, _P, _P, _P]),
     "gstex_num_tiles_hit": (_I, [_I, _P, _P, _I, _I, _I, _P, _P]),
     "gstex_view_records_bytes": (ctypes.c_size_t, [_I]),
     "gstex_view_records": (_I, [_P, _P, ctypes.c_size_t, _P]),
@@ -125,6 +126,20 @@ def stream_of(t: torch.Tensor):
     if not t.is_cuda:
         raise GstexError("gstex_cuda_gb300 operators need CUDA tensors (no CPU implementation)")
     return torch.cuda.current_stream(t.device).cuda_stream
+
+
+def plain_cuda_f32(*tensors) -> bool:
+    """Whether a kernel launch can stand for torch operations on these
+    tensors: float32 CUDA tensors that no gradient, forward-mode tangent,
+    functional transform, tracer, compiler or dispatch mode looks at."""
+    grad = torch.is_grad_enabled()
+    for t in tensors:
+        if type(t) not in (torch.Tensor, torch.nn.Parameter) or not t.is_cuda or t.dtype is not torch.float32 \
+                or (grad and t.requires_grad):
+            return False
+    return (torch.autograd.forward_ad._current_level < 0 and torch._C._functorch.peek_interpreter_stack() is None
+            and torch._C._get_tracing_state() is None and not torch.compiler.is_compiling()
+            and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0)
 
 
 def require_cuda(*tensors, names=None):

@@ -94,6 +94,19 @@ def get_aabb_2d(means, scales, glob_scale, quats, viewmat, fx, fy, cx, cy):
     return centers, extents
 
 
+def project_points(points, viewmat, fx, fy, cx, cy):
+    """Pixel positions [N, 2] and camera depths [N] of points [N, 3]."""
+    _chk(("points", points), ("viewmat", viewmat))
+    _f32("points", points)
+    _f32("viewmat", viewmat)
+    n = points.shape[0]
+    pix = torch.empty((n, 2), dtype=torch.float32, device=points.device)
+    depths = torch.empty(n, dtype=torch.float32, device=points.device)
+    check(_lib.lib().gstex_project_points(n, ptr(points), ptr(viewmat), float(fx), float(fy), float(cx), float(cy),
+                                          ptr(pix), ptr(depths), _lib.stream_of(points)), "project_points")
+    return pix, depths
+
+
 def num_tiles_hit(centers, extents, img_height, img_width, block_width):
     _chk(("centers", centers), ("extents", extents))
     _f32("centers", centers)

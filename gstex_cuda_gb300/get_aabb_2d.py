@@ -3,6 +3,7 @@ from __future__ import annotations
 
 import torch
 
+from . import _lib
 from . import _torch_impl as _T
 from . import cuda as _C
 
@@ -17,6 +18,10 @@ def merge_aabbs(centers1, extents1, centers2, extents2):
 def project_points(points, viewmat, intrins, clip=False):
     """Pixel positions and camera depths of points (gstex_cuda/get_aabb_2d.py:22-32).
     The depths are the per-Gaussian sort keys of the binning stage."""
+    if not clip and _lib.plain_cuda_f32(points, viewmat) and points.ndim == 2 and points.shape[-1] == 3 \
+            and viewmat.shape == (4, 4) and all(type(x) in (int, float) for x in intrins) \
+            and points.device == viewmat.device:
+        return _C.project_points(points.detach().contiguous(), viewmat.detach().contiguous(), *intrins)
     view_points = points @ viewmat.T[:3, :3] + viewmat.T[3:, :3]
     if clip:
         with torch.no_grad():

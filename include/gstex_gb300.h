@@ -53,6 +53,11 @@ int gstex_get_aabb_2d(int n, const float* means, const float* scales, float glob
                       const float* viewmat, float fx, float fy, float cx, float cy, float* centers,
                       float* extents, gstex_stream_t stream);
 
+/* Pixel positions [n,2] and camera depths [n] of points [n,3]
+ * (project_points, gstex_cuda/get_aabb_2d.py:22-32, without its clip). */
+int gstex_project_points(int n, const float* points, const float* viewmat, float fx, float fy, float cx, float cy,
+                         float* pix, float* depths, gstex_stream_t stream);
+
 /* Per-Gaussian number of tiles hit, bit-exact with the reference's torch
  * tile counter.  Replaces get_num_tiles_hit_2d (gstex_cuda/get_aabb_2d.py:70-91). */
 int gstex_num_tiles_hit(int n, const float* centers, const float* extents, int img_height, int img_width,
