@@ -125,7 +125,7 @@ def stream_of(t: torch.Tensor):
     """Handle of the current torch stream on t's device."""
     if not t.is_cuda:
         raise GstexError("gstex_cuda_gb300 operators need CUDA tensors (no CPU implementation)")
-    return torch.cuda.current_stream(t.device).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(t.get_device())
 
 
 def plain_cuda_f32(*tensors) -> bool:

@@ -25,12 +25,13 @@ def _chk(*named):
     for name, t in named:
         if t is None:
             continue
+        if isinstance(t, torch.Tensor) and t.is_cuda and t.is_contiguous():
+            continue
         if not isinstance(t, torch.Tensor):
             raise TypeError(f"{name} must be a torch.Tensor")
         if not t.is_cuda:
             raise _lib.GstexError(f"{name} must be a CUDA tensor")
-        if not t.is_contiguous():
-            raise _lib.GstexError(f"{name} must be contiguous")
+        raise _lib.GstexError(f"{name} must be contiguous")
 
 
 def _f32(name, t):
@@ -189,12 +190,13 @@ def bin_view(centers, extents, depths, num_tiles_hit, tile_bounds, block_width):
     L = _lib.lib()
     dev = num_tiles_hit.device
     st = _lib.stream_of(num_tiles_hit)
-    order = torch.empty((2, n), dtype=torch.int32, device=dev)  # depth order, inclusive slot sums
+    order = torch.empty(2 * n, dtype=torch.int32, device=dev)  # depth order, inclusive slot sums
+    p_order, p_cum = ptr(order), ptr(order) + 4 * n
     info = torch.empty(2, dtype=torch.int64, device=dev)
     wsb = L.gstex_view_order_workspace_bytes(n)
     ws = torch.empty(wsb, dtype=torch.uint8, device=dev)
-    check(L.gstex_view_order(n, ptr(depths), ptr(num_tiles_hit), ptr(order[0]), ptr(order[1]), ptr(info), ptr(ws), wsb,
-                             st), "view_order")
+    check(L.gstex_view_order(n, ptr(depths), ptr(num_tiles_hit), p_order, p_cum, ptr(info), ptr(ws), wsb, st),
+          "view_order")
     total, ties = info.tolist()
     if total >= 2 ** 31:
         raise OverflowError(f"{total} intersections exceed the int32 range of the reference's cumsum")
@@ -209,7 +211,7 @@ def bin_view(centers, extents, depths, num_tiles_hit, tile_bounds, block_width):
     bins = torch.empty((int(tile_bounds[0]) * int(tile_bounds[1]), 2), dtype=torch.int32, device=dev)
     wsb = L.gstex_view_bins_workspace_bytes(total)
     ws = torch.empty(wsb, dtype=torch.uint8, device=dev)
-    check(L.gstex_view_bins(n, total, ptr(centers), ptr(extents), ptr(depths), ptr(order[0]), ptr(order[1]),
+    check(L.gstex_view_bins(n, total, ptr(centers), ptr(extents), ptr(depths), p_order, p_cum,
                             int(tile_bounds[0]), int(tile_bounds[1]), int(block_width), ptr(gids), ptr(bins), ptr(ws),
                             wsb, st), "view_bins")
     return total, gids, bins
@@ -296,6 +298,16 @@ def texture_forward(tile_bounds, block, img_size, texture_info, texture_dims, ga
 
     c2w is accepted for interface compatibility; rays are built from viewmat
     (the two must be inverses of each other, as in the reference)."""
+    return forward_with_records(tile_bounds, block, img_size, texture_info, texture_dims, gaussian_ids_sorted,
+                                tile_bins, colors, opacities, means, scales, glob_scale, quats, uv0, umap, vmap,
+                                texture, viewmat, c2w, fx, fy, cx, cy, settings, background)[0]
+
+
+def forward_with_records(tile_bounds, block, img_size, texture_info, texture_dims, gaussian_ids_sorted, tile_bins,
+                         colors, opacities, means, scales, glob_scale, quats, uv0, umap, vmap, texture, viewmat, c2w,
+                         fx, fy, cx, cy, settings, background):
+    """(texture_forward's outputs, the view's splat records or None); the
+    records spare texture_backward of the same call their rebuilding."""
     W, H = int(img_size[0]), int(img_size[1])
     bw = int(block[0])
     ri, C = _raster_inputs(W, H, bw, texture_info, texture_dims, gaussian_ids_sorted, tile_bins, colors, opacities,
@@ -314,17 +326,18 @@ def texture_forward(tile_bounds, block, img_size, texture_info, texture_dims, ga
     reg_s = torch.empty((H, W, 3), **f32)
     fo = _lib.ForwardOutputs(ptr(out_img), ptr(out_depth), ptr(out_reg), ptr(out_tex), ptr(out_normal), ptr(final_T),
                              ptr(final_idx), ptr(depth_idx), ptr(reg_s))
-    recs = _attach_records(ri, dev)  # noqa: F841 (alive until the launch is queued)
+    recs = _attach_records(ri, dev)
     check(_lib.lib().gstex_texture_forward(ctypes.byref(ri), ctypes.byref(fo), _lib.stream_of(means)),
           "texture_forward")
-    return out_img, out_depth, out_reg, out_tex, out_normal, final_T, final_idx, depth_idx, reg_s
+    return (out_img, out_depth, out_reg, out_tex, out_normal, final_T, final_idx, depth_idx, reg_s), recs
 
 
 def texture_backward(img_height, img_width, block_width, texture_info, texture_dims, gaussian_ids_sorted, tile_bins,
                      colors, opacities, means, scales, glob_scale, quats, uv0, umap, vmap, texture, viewmat, c2w, fx,
                      fy, cx, cy, settings, background, final_Ts, final_idx, depth_idx, final_s, v_output,
-                     v_output_depth, v_output_reg, v_output_alpha, v_output_texture, v_output_normal):
-    """Returns (v_colors, v_opacity, v_means, v_scales, v_quats, v_uv0, v_umap, v_vmap, v_texture)."""
+                     v_output_depth, v_output_reg, v_output_alpha, v_output_texture, v_output_normal, records=None):
+    """Returns (v_colors, v_opacity, v_means, v_scales, v_quats, v_uv0, v_umap, v_vmap, v_texture).
+    records: those of forward_with_records with the same inputs (None: built here)."""
     ri, C = _raster_inputs(img_width, img_height, block_width, texture_info, texture_dims, gaussian_ids_sorted,
                            tile_bins, colors, opacities, means, scales, glob_scale, quats, uv0, umap, vmap, texture,
                            viewmat, fx, fy, cx, cy, settings, background)
@@ -353,7 +366,10 @@ def texture_backward(img_height, img_width, block_width, texture_info, texture_d
                           ptr(v_output_depth), ptr(v_output_reg), ptr(v_output_alpha), ptr(v_output_texture),
                           ptr(v_output_normal), ptr(v_colors), ptr(v_opacity), ptr(v_means), ptr(v_scales),
                           ptr(v_quats), ptr(v_uv0), ptr(v_umap), ptr(v_vmap), ptr(v_texture), ptr(ws), wsb)
-    recs = _attach_records(ri, dev)  # noqa: F841 (alive until the launch is queued)
+    if records is None:
+        records = _attach_records(ri, dev)  # (alive until the launch is queued)
+    else:
+        ri.records = ptr(records)
     check(L.gstex_texture_backward(ctypes.byref(ri), ctypes.byref(bio), _lib.stream_of(means)), "texture_backward")
     return v_colors, v_opacity, v_means, v_scales, v_quats, v_uv0, v_umap, v_vmap, v_texture
 

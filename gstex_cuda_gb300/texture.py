@@ -7,6 +7,7 @@ library; the hot path has no PyTorch or CPU fallback.
 """
 from __future__ import annotations
 
+import math
 from typing import Optional, Tuple
 
 import torch
@@ -63,9 +64,10 @@ class _TextureGaussians(Function):
         # this case, gstex_cuda/texture.py:197-205, leaves most outputs undefined)
         num_intersects, gaussian_ids_sorted, tile_bins = bin_view(centers, extents, depths, num_tiles_hit, tile_bounds,
                                                                   block_width)
-        outs = _C.texture_forward(tile_bounds, block, img_size, texture_info, texture_dims, gaussian_ids_sorted,
-                                  tile_bins, colors, opacity, means, scales, glob_scale, quats, uv0, umap, vmap,
-                                  texture, viewmat, c2w, fx, fy, cx, cy, settings, background)
+        outs, records = _C.forward_with_records(tile_bounds, block, img_size, texture_info, texture_dims,
+                                                gaussian_ids_sorted, tile_bins, colors, opacity, means, scales,
+                                                glob_scale, quats, uv0, umap, vmap, texture, viewmat, c2w, fx, fy, cx,
+                                                cy, settings, background)
         out_img, out_depth, out_reg, out_texture, out_normal, final_Ts, final_idx, depth_idx, out_reg_s = outs
         ctx.img_width, ctx.img_height = img_width, img_height
         ctx.texture_info = texture_info
@@ -74,27 +76,27 @@ class _TextureGaussians(Function):
         ctx.num_intersects = num_intersects
         ctx.block_width = block_width
         ctx.settings = settings
-        ctx.save_for_backward(texture_dims, gaussian_ids_sorted, tile_bins, colors, opacity, means, scales, quats,
-                              uv0, umap, vmap, texture, viewmat, c2w, background, final_Ts, final_idx, depth_idx,
-                              out_reg_s)
+        ctx.set_materialize_grads(False)  # (backward makes the zeros that it needs)
+        if not any(ctx.needs_input_grad):
+            records = None
+        ctx.save_for_backward(records, texture_dims, gaussian_ids_sorted, tile_bins, colors, opacity, means, scales,
+                              quats, uv0, umap, vmap, texture, viewmat, c2w, background, final_Ts, final_idx,
+                              depth_idx, out_reg_s)
         out_alpha = 1 - final_Ts
         return out_img, out_depth, out_reg, out_alpha, out_texture, out_normal
 
     @staticmethod
     def backward(ctx, v_out_img, v_out_depth, v_out_reg, v_out_alpha, v_out_texture, v_out_normal):
-        (texture_dims, gaussian_ids_sorted, tile_bins, colors, opacity, means, scales, quats, uv0, umap, vmap,
+        (records, texture_dims, gaussian_ids_sorted, tile_bins, colors, opacity, means, scales, quats, uv0, umap, vmap,
          texture, viewmat, c2w, background, final_Ts, final_idx, depth_idx, out_reg_s) = ctx.saved_tensors
-
-        def g(t, like):
-            return torch.zeros_like(like) if t is None else t.contiguous()
-
-        v_out_img = g(v_out_img, final_Ts.unsqueeze(-1).expand(*final_Ts.shape, 3))
-        v_out_depth = g(v_out_depth, final_Ts)
-        v_out_reg = g(v_out_reg, final_Ts)
-        v_out_alpha = g(v_out_alpha, final_Ts)
+        # one buffer of zeros serves all outputs that no gradient reaches
+        H, W = final_Ts.shape
         C = int(ctx.texture_info[2])
-        v_out_texture = g(v_out_texture, final_Ts.new_zeros(*final_Ts.shape, C))
-        v_out_normal = g(v_out_normal, final_Ts.new_zeros(*final_Ts.shape, 3))
+        ups = [v_out_img, v_out_depth, v_out_reg, v_out_alpha, v_out_texture, v_out_normal]
+        shapes = [(H, W, 3), (H, W), (H, W), (H, W), (H, W, C), (H, W, 3)]
+        need = [math.prod(sh) for t, sh in zip(ups, shapes) if t is None]
+        zeros = final_Ts.new_zeros(max(need)) if need else None
+        ups = [t.contiguous() if t is not None else zeros[:math.prod(sh)].view(sh) for t, sh in zip(ups, shapes)]
         if ctx.num_intersects < 1:
             grads = [torch.zeros_like(t) for t in (colors, opacity, means, scales, quats, uv0, umap, vmap, texture)]
         else:
@@ -102,7 +104,7 @@ class _TextureGaussians(Function):
                 ctx.img_height, ctx.img_width, ctx.block_width, ctx.texture_info, texture_dims, gaussian_ids_sorted,
                 tile_bins, colors, opacity, means, scales, ctx.glob_scale, quats, uv0, umap, vmap, texture, viewmat,
                 c2w, ctx.fx, ctx.fy, ctx.cx, ctx.cy, ctx.settings, background, final_Ts, final_idx, depth_idx,
-                out_reg_s, v_out_img, v_out_depth, v_out_reg, v_out_alpha, v_out_texture, v_out_normal)
+                out_reg_s, *ups, records=records)
         v_colors, v_opacity, v_means, v_scales, v_quats, v_uv0, v_umap, v_vmap, v_texture = grads
         return (None, None, None, None, None, None, v_colors, v_opacity, v_means, v_scales, None, v_quats, v_uv0,
                 v_umap, v_vmap, v_texture, None, None, None, None, None, None, None, None, None, None, None)

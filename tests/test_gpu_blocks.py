@@ -156,3 +156,36 @@ def test_skipped_splat_ends_a_pixel():
         assert float((new["final_idx"] == old["final_idx"]).float().mean()) >= 0.99
         np.testing.assert_allclose(np_(out["final_T"]), ref["final_T"], atol=5e-7)
         np.testing.assert_allclose(np_(out["img"]), ref["img"], atol=2e-5)
+
+
+@pytest.mark.parametrize("hooks", [False, True])
+def test_backward_of_some_outputs_and_again(hooks):
+    """Outputs without a gradient count as zero gradients, a second backward
+    over a retained graph gives the same, and saved tensors may come back
+    through hooks (the splat records are among them)."""
+    import contextlib
+
+    import gstex_cuda_gb300 as G
+    spec = small_scene(n=120, width=40, height=28, seed=6)
+    case = Case(spec)
+    t = case.t
+    names = ("colors", "opacity", "means", "scales", "quats", "uv0", "umap", "vmap", "texture")
+    for k in names:
+        t[k].requires_grad_()
+    b = case.binning_cuda(16)
+    ctx = torch.autograd.graph.save_on_cpu() if hooks else contextlib.nullcontext()
+    with ctx:
+        outs = G.texture_gaussians((spec.num_points, 1, 3), t["dims"], b["centers"], b["extents"], b["depths"],
+                                   b["counts"], t["colors"], t["opacity"], t["means"], t["scales"], 1.0, t["quats"],
+                                   t["uv0"], t["umap"], t["vmap"], t["texture"], t["viewmat"], t["c2w"], *case.intr,
+                                   28, 40, 16, 1 << 8, torch.zeros(3, device=DEV))
+    g = torch.Generator().manual_seed(0)
+    ups = [torch.randn(o.shape, generator=g).to(DEV) for o in outs]
+    ins = [t[k] for k in names]
+    full = [u if k in (0, 4) else torch.zeros_like(u) for k, u in enumerate(ups)]
+    ref = torch.autograd.grad(outs, ins, full, retain_graph=True)
+    for _ in range(2):
+        got = torch.autograd.grad((outs[0], outs[4]), ins, (ups[0], ups[4]), retain_graph=True)
+        for k, x, y in zip(names, got, ref):
+            # (sums in another order: 1e-5 of the largest entry)
+            assert float((x - y).abs().max()) <= 1e-5 * float(y.abs().max()) + 1e-12, k
