@@ -72,6 +72,7 @@ _SIGS = {
     "gstex_view_order": (_I, [_I, _P, _P, _P, _P, _P, _P, ctypes.c_size_t, _P]),
     "gstex_view_bins_workspace_bytes": (ctypes.c_size_t, [_I]),
     "gstex_view_bins": (_I, [_I, _I, _P, _P, _P, _P, _P, _I, _I, _I, _P, _P, _P, ctypes.c_size_t, _P]),
+    "gstex_chart_texels": (_I, [_I, _P, _P, _P]),
     "gstex_texture_forward": (_I, [ctypes.POINTER(RasterInputs), ctypes.POINTER(ForwardOutputs), _P]),
     "gstex_texture_edit": (_I, [ctypes.POINTER(RasterInputs), ctypes.POINTER(EditIO), _P]),
     "gstex_preprocess_forward": (_I, [_I, _I] + [_P] * 10 + [_P]),

@@ -2,6 +2,8 @@
 //
 // Built with -fmad=false and IEEE division so that the AABB and tile counts
 // are reproducible bit for bit by a CPU restatement of the same operations.
+#include <algorithm>
+
 #include "common.cuh"
 #include "project.cuh"
 
@@ -285,6 +287,36 @@ extern "C" int gstex_project_points(int n, const float* points, const float* vie
     project_points_kernel<<<ceil_div(n, 256), 256, 0, (cudaStream_t)stream>>>(n, (const float3*)points, viewmat, fx, fy,
                                                                             cx, cy, (float2*)pix, depths);
     return check_launch("project_points");
+}
+
+// sum of h * w over the charts of dims [n, 3]
+namespace gstex {
+__global__ void __launch_bounds__(1024) chart_texels_kernel(int n, const int32_t* __restrict__ dims,
+                                                            int64_t* __restrict__ total) {
+    __shared__ long long part[32];
+    long long s = 0;
+    for (int i = blockIdx.x * 1024 + threadIdx.x; i < n; i += gridDim.x * 1024)
+        s += (long long)dims[3 * (size_t)i] * dims[3 * (size_t)i + 1];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        s = part[threadIdx.x];
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (threadIdx.x == 0) atomicAdd((unsigned long long*)total, (unsigned long long)s);
+    }
+}
+}  // namespace gstex
+
+extern "C" int gstex_chart_texels(int n, const int32_t* dims, int64_t* total, gstex_stream_t s) {
+    GSTEX_REQUIRE(n >= 0 && total);
+    cudaStream_t stream = (cudaStream_t)s;
+    cudaError_t e = cudaMemsetAsync(total, 0, sizeof(int64_t), stream);
+    if (e != cudaSuccess) { set_cuda_error(e, "chart_texels"); return GSTEX_ERR_CUDA; }
+    if (n == 0) return GSTEX_OK;
+    GSTEX_REQUIRE(dims);
+    chart_texels_kernel<<<std::min(ceil_div(n, 1024), 152), 1024, 0, stream>>>(n, dims, total);
+    return check_launch("chart_texels");
 }
 
 extern "C" size_t gstex_scan_workspace_bytes(int n) {

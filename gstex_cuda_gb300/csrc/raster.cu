@@ -838,14 +838,6 @@ __device__ __forceinline__ void bwd_tile(const SceneArgs& a, const TileJob& J, c
 // camera depth lies in the pixel's [lower, upper] range a bilinear splat of
 // (r a, g a, b a, a, 1) of the edited pixel into the chart's [T, 5] texels.
 // ---------------------------------------------------------------------------
-struct EditIO {
-    const float3* img;
-    const float* alpha;
-    const float* lower;
-    const float* upper;
-    float* out;  // [T, 5]
-};
-
 __device__ __forceinline__ void edit_tile(const SceneArgs& a, const TileJob& J, const EditIO& E, const Recs& R) {
     const int nthr = blockDim.x * blockDim.y;
     const int tr = threadIdx.y * blockDim.x + threadIdx.x;
@@ -1604,6 +1596,12 @@ extern "C" int gstex_texture_edit(const gstex_raster_inputs* in, const gstex_edi
     va.bins = (const int2*)in->tile_bins;
     EditIO E{ (const float3*)io->updated_img, io->updated_alpha, io->depth_lower, io->depth_upper,
               io->updated_texture };
+    if ((bw & 7) == 0 && in->records) {
+        GSTEX_REQUIRE(((uintptr_t)in->records & 15) == 0);
+        va.recs = (const RecAll*)in->records;
+        a.settings = (in->settings & 1) << 9;  // the walk's blur bit
+        return launch_edit_blocks(a, block_args(va, bw, a.N), E, stream);
+    }
     const size_t smem = (size_t)kRecBytes * bw * bw;
     int rc = set_smem(edit_view_kernel<1>, smem, "texture_edit");
     if (rc) return rc;

@@ -116,6 +116,14 @@ struct BwdArgs {
     float* v_texgrad;       // [T, C] (fp32 texture) or [T, 4] (bf16 texture)
 };
 
+struct EditIO {
+    const float3* img;
+    const float* alpha;
+    const float* lower;
+    const float* upper;
+    float* out;  // [T, 5]
+};
+
 int fill_scene(const gstex_raster_inputs* in, SceneArgs& a, bool need_bins);
 int ppt_of(int bw, int requested);
 int gs_of(int bw, int ppt, int C, int requested);
@@ -154,6 +162,7 @@ constexpr int kFixedBwdSettings = 1 << 8;
 constexpr int kFixedFwdMask = (1 << 2) | (1 << 9) | (1 << 10) | (1 << 15) | (1 << 16);
 bool blocks_apply(int bw, int C, int settings, const RecAll* recs);
 int launch_fwd_blocks(const SceneArgs& a, const BlockArgs& ba, const FwdOut& o, int texmode, cudaStream_t stream);
+int launch_edit_blocks(const SceneArgs& a, const BlockArgs& ba, const EditIO& E, cudaStream_t stream);
 int launch_bwd_blocks(const SceneArgs& a, const BlockArgs& ba, const BwdArgs& g, int texmode, cudaStream_t stream);
 int launch_records(const SceneArgs& a, const BatchArgs& ba, int num_views, const int32_t* counts, RecAll* recs,
                    int* fix_count, uint32_t* fix, cudaStream_t stream);

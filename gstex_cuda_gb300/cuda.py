@@ -180,10 +180,11 @@ def get_tile_bin_edges(num_intersects, isect_ids_sorted, tile_bounds):
     return bins
 
 
-def bin_view(centers, extents, depths, num_tiles_hit, tile_bounds, block_width):
+def bin_view(centers, extents, depths, num_tiles_hit, tile_bounds, block_width, texture_dims=None):
     """Depth-first binning of one view: (number of intersections,
     gaussian_ids_sorted, tile_bins), equal to the scan, emission, sort and
-    ranges of the functions above.  Reads the number back to the host."""
+    ranges of the functions above.  Reads the number back to the host; with
+    texture_dims the charts' number of texels comes along as a fourth result."""
     _chk(("centers", centers), ("extents", extents), ("depths", depths), ("num_tiles_hit", num_tiles_hit))
     _i32("num_tiles_hit", num_tiles_hit)
     n = min(num_tiles_hit.shape[0], centers.shape[0])
@@ -192,12 +193,17 @@ def bin_view(centers, extents, depths, num_tiles_hit, tile_bounds, block_width):
     st = _lib.stream_of(num_tiles_hit)
     order = torch.empty(2 * n, dtype=torch.int32, device=dev)  # depth order, inclusive slot sums
     p_order, p_cum = ptr(order), ptr(order) + 4 * n
-    info = torch.empty(2, dtype=torch.int64, device=dev)
+    info = torch.empty(3, dtype=torch.int64, device=dev)
+    if texture_dims is not None:
+        _chk(("texture_dims", texture_dims))
+        _i32("texture_dims", texture_dims)
+        check(L.gstex_chart_texels(texture_dims.shape[0], ptr(texture_dims), ptr(info) + 16, st), "chart_texels")
     wsb = L.gstex_view_order_workspace_bytes(n)
     ws = torch.empty(wsb, dtype=torch.uint8, device=dev)
     check(L.gstex_view_order(n, ptr(depths), ptr(num_tiles_hit), p_order, p_cum, ptr(info), ptr(ws), wsb, st),
           "view_order")
-    total, ties = info.tolist()
+    total, ties, texels = info.tolist()
+    more = () if texture_dims is None else (texels,)
     if total >= 2 ** 31:
         raise OverflowError(f"{total} intersections exceed the int32 range of the reference's cumsum")
     if ties:  # depths of +0: the order of the 64-bit keys
@@ -205,7 +211,7 @@ def bin_view(centers, extents, depths, num_tiles_hit, tile_bounds, block_width):
         keys, ids = map_gaussian_to_intersects(n, total, centers, extents, depths, cum, tile_bounds, block_width)
         num_tiles = int(tile_bounds[0]) * int(tile_bounds[1])
         keys, ids = sort_pairs(keys, ids, sort_end_bit(num_tiles))
-        return total, ids, get_tile_bin_edges(total, keys, tile_bounds)
+        return (total, ids, get_tile_bin_edges(total, keys, tile_bounds)) + more
     total = max(total, 0)
     gids = torch.empty(total, dtype=torch.int32, device=dev)
     bins = torch.empty((int(tile_bounds[0]) * int(tile_bounds[1]), 2), dtype=torch.int32, device=dev)
@@ -214,7 +220,7 @@ def bin_view(centers, extents, depths, num_tiles_hit, tile_bounds, block_width):
     check(L.gstex_view_bins(n, total, ptr(centers), ptr(extents), ptr(depths), p_order, p_cum,
                             int(tile_bounds[0]), int(tile_bounds[1]), int(block_width), ptr(gids), ptr(bins), ptr(ws),
                             wsb, st), "view_bins")
-    return total, gids, bins
+    return (total, gids, bins) + more
 
 
 # ---------------------------------------------------------------------------
@@ -442,6 +448,15 @@ def texture_edit(tile_bounds, block, img_size, texture_info, texture_total_size,
     ri.viewmat = ptr(viewmat)
     ri.fx, ri.fy, ri.cx, ri.cy = float(fx), float(fy), float(cx), float(cy)
     ri.settings = int(settings)
+    recs = None
+    if PREBUILT_RECORDS and ri.num_points > 0 and ri.block_width in (8, 16):
+        # the records of the forward walk with editing's blur bit (0) in the
+        # renderer's place (9); their colours are not read
+        rr = _lib.RasterInputs.from_buffer_copy(ri)
+        rr.channels, rr.num_texels, rr.colors, rr.background = 0, 0, ptr(means), ptr(means)
+        rr.settings = (int(settings) & 1) << 9
+        recs = _attach_records(rr, means.device)  # (alive until the launch is queued)
+        ri.records = ptr(recs)
     out = torch.empty((T, 5), dtype=torch.float32, device=means.device)
     io = _lib.EditIO(ptr(updated_img), ptr(updated_alpha), ptr(depth_lower), ptr(depth_upper), T, ptr(out))
     check(_lib.lib().gstex_texture_edit(ctypes.byref(ri), ctypes.byref(io), _lib.stream_of(means)), "texture_edit")

@@ -34,14 +34,14 @@ def texture_edit(texture_info: Tuple[int, int, int], texture_dims: Tensor, updat
     tile_bounds = ((img_width + block_width - 1) // block_width, (img_height + block_width - 1) // block_width, 1)
     block = (block_width, block_width, 1)
     img_size = (img_width, img_height, 1)
-    texture_total_size = int(torch.sum(texture_dims[:, 0].long() * texture_dims[:, 1].long()).item())
-    num_intersects, gaussian_ids_sorted, tile_bins = bin_view(centers, extents, depths, num_tiles_hit, tile_bounds,
-                                                              block_width)
+    texture_dims = texture_dims.contiguous()
+    num_intersects, gaussian_ids_sorted, tile_bins, texture_total_size = bin_view(
+        centers, extents, depths, num_tiles_hit, tile_bounds, block_width, texture_dims)
     if num_intersects < 1:
         raise ValueError("texture_edit: no Gaussian intersects the image")
     if background is None:
         background = torch.zeros(3, device=means.device)
-    return _C.texture_edit(tile_bounds, block, img_size, texture_info, texture_total_size, texture_dims.contiguous(),
+    return _C.texture_edit(tile_bounds, block, img_size, texture_info, texture_total_size, texture_dims,
                            updated_img.contiguous(), updated_alpha.contiguous(), depth_lower.contiguous(),
                            depth_upper.contiguous(), gaussian_ids_sorted, tile_bins, opacity.contiguous(),
                            means.contiguous(), scales.contiguous(), glob_scale, quats.contiguous(),

@@ -6,7 +6,7 @@ radix sort over the key bits that can be non-zero for valid keys.
 """
 from __future__ import annotations
 
-from typing import Tuple
+from typing import Optional, Tuple
 
 import torch
 from torch import Tensor
@@ -57,11 +57,13 @@ def bin_and_sort_gaussians(num_points: int, num_intersects: int, centers: Tensor
 
 
 def bin_view(centers: Tensor, extents: Tensor, depths: Tensor, num_tiles_hit: Tensor,
-             tile_bounds: Tuple[int, int, int], block_size: int) -> Tuple[int, Tensor, Tensor]:
+             tile_bounds: Tuple[int, int, int], block_size: int, texture_dims: Optional[Tensor] = None):
     """(num_intersects, gaussian_ids_sorted, tile_bins) of one view: what
     compute_cumulative_intersects and bin_and_sort_gaussians give a renderer,
-    without the 64-bit intersection keys."""
+    without the 64-bit intersection keys; with texture_dims also the charts'
+    number of texels."""
     counts = num_tiles_hit.contiguous()
     if counts.dtype != torch.int32:
         counts = counts.to(torch.int32)
-    return _C.bin_view(centers.contiguous(), extents.contiguous(), depths.contiguous(), counts, tile_bounds, block_size)
+    return _C.bin_view(centers.contiguous(), extents.contiguous(), depths.contiguous(), counts, tile_bounds, block_size,
+                       texture_dims)

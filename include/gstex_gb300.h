@@ -170,6 +170,9 @@ int gstex_view_bins(int n, int num_intersects, const float* centers, const float
                     int32_t* gaussian_ids_sorted, int32_t* tile_bins, void* workspace, size_t workspace_bytes,
                     gstex_stream_t stream);
 
+/* Texels of all charts: the sum of h * w over dims [n,3]. */
+int gstex_chart_texels(int n, const int32_t* texture_dims, int64_t* total, gstex_stream_t stream);
+
 /* ---------------------------------------------------------------------
  * Textured compositor (texture_forward / texture_backward)
  * ------------------------------------------------------------------- */

@@ -189,3 +189,37 @@ def test_backward_of_some_outputs_and_again(hooks):
         for k, x, y in zip(names, got, ref):
             # (sums in another order: 1e-5 of the largest entry)
             assert float((x - y).abs().max()) <= 1e-5 * float(y.abs().max()) + 1e-12, k
+
+
+@pytest.mark.parametrize("bw", [8, 16])
+@pytest.mark.parametrize("settings", [0, 1])
+def test_edit_matches_the_tile_kernel(bw, settings):
+    """Texture editing by blocks against one CTA per tile: sums in another
+    order (1e-5 of a row's weights), one texel row in a thousand on a
+    threshold; and an infinite edited pixel spoils the same texels."""
+    import gstex_cuda_gb300 as G
+    spec = small_scene(n=400, width=61, height=43, seed=12, chart=(1, 5))
+    case = Case(spec)
+    b, t, cam = case.binning_cuda(bw), case.t, case.cam
+    T = spec.texture.shape[0]
+    g = torch.Generator().manual_seed(1)
+    img, alpha = torch.rand(43, 61, 3, generator=g), (torch.rand(43, 61, generator=g) > 0.3).float()
+    lo, hi = 3.0 - torch.rand(43, 61, generator=g), 3.0 + torch.rand(43, 61, generator=g)
+    img[20, 30, 1] = float("inf")
+    alpha[20, 30] = 1.0
+    outs = []
+    for prebuilt in (True, False):
+        G.cuda.PREBUILT_RECORDS = prebuilt
+        try:
+            outs.append(G.cuda.texture_edit(b["tile_bounds"], (bw, bw, 1), (61, 43, 1), (400, 1, 5), T, t["dims"],
+                                            *(x.to(DEV) for x in (img, alpha, lo, hi)), b["gaussian_ids_sorted"],
+                                            b["tile_bins"], t["opacity"], t["means"], t["scales"], 1.0, t["quats"],
+                                            t["uv0"], t["umap"], t["vmap"], t["viewmat"], t["c2w"], *case.intr,
+                                            settings, None))
+        finally:
+            G.cuda.PREBUILT_RECORDS = True
+    new, old = outs
+    assert torch.equal(torch.isfinite(new), torch.isfinite(old)) and not torch.isfinite(old).all()
+    fine = torch.isfinite(old)
+    bad = ((new - old).abs() > 1e-5 * (1 + old.abs())) & fine
+    assert float(bad.any(1).float().mean()) <= 1e-3
