@@ -1,4 +1,6 @@
 // Tile binning: intersection emission, stable LSD radix sort, tile ranges.
+#include <algorithm>
+
 #include "common.cuh"
 #include "project.cuh"
 
@@ -96,19 +98,29 @@ __global__ void bin_edges_kernel(int n, const int64_t* __restrict__ n_dev, const
 }
 
 // ---------------------------------------------------------------------------
-// Stable LSD radix sort of (u64 key, u32 value), 8-bit digits.
+// Stable LSD radix sort of (u64 or u32 key, u32 value), digits of at most 8
+// bits, of equal width in all passes.
 //
 // Each pass: per-block digit histograms -> one exclusive scan in
 // (digit, block) order -> stable scatter.  Blocks own contiguous chunks; a
-// block ranks each 2048-item tile with warp match + per-warp counters, so the
+// block ranks each 3072-item tile with ballots + per-warp counters, so the
 // order of equal digits is the input order.
+//
+// What bounds the scatter: instruction issue (62% of cycles) and the runs of a
+// digit in a tile, whose partial sectors cost writes: 14 bits as 7 + 7 and 20 as
+// 7 + 7 + 6 beat 8 + 6 and 8 + 8 + 4 (158M items 2.56 -> 2.14 ms, 80M 2.13 ->
+// 1.68 ms), tiles of 3072 beat 2048 by 3 to 8%.  Ranks by __match_any_sync with
+// a counter read and written in every round kept the warps waiting on shared
+// memory (14 of 25 stall cycles).  Altogether 158M items of 14 bits 2.71 -> 1.99
+// ms, 80M of 20 bits 2.15 -> 1.57 ms, 16M of 32 bits 0.67 -> 0.56 ms.
 // ---------------------------------------------------------------------------
 constexpr int kRadix = 256;
 constexpr int kSortThreads = 256;
 constexpr int kSortWarps = kSortThreads / 32;
-constexpr int kSortItems = 8;
+constexpr int kSortItems = 12;
 constexpr int kSortTile = kSortThreads * kSortItems;
 constexpr int kSortMaxBlocks = 1216;
+static_assert(kSortThreads == kRadix, "a thread per digit");
 
 struct SortPlan {
     int blocks, chunk;
@@ -137,13 +149,13 @@ __device__ __forceinline__ void resolve_count(const int64_t* n_dev, int& n, int&
 }
 
 // Per-block digit counts: each warp loads its kSortItems keys per thread of a
-// 2048-item tile up front (so the loads overlap) and counts them in its own
+// tile of items up front (so the loads overlap) and counts them in its own
 // shared-memory histogram with plain atomics; the warps' histograms are summed
 // at the end.
 template <typename K>
 __global__ void __launch_bounds__(kSortThreads) radix_hist_kernel(const K* __restrict__ keys, int n, int chunk,
                                                                   const int64_t* __restrict__ n_dev, int shift,
-                                                                  uint32_t* __restrict__ hist) {
+                                                                  uint32_t dmask, uint32_t* __restrict__ hist) {
     __shared__ uint32_t h[kSortWarps][kRadix];
     for (int i = threadIdx.x; i < kSortWarps * kRadix; i += blockDim.x) (&h[0][0])[i] = 0;
     resolve_count(n_dev, n, chunk);
@@ -153,7 +165,7 @@ __global__ void __launch_bounds__(kSortThreads) radix_hist_kernel(const K* __res
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     uint32_t* hw = h[warp];
-    for (int tbase = start; tbase < end; tbase += kSortTile) {
+    for (int tbase = start; tbase < end; tbase += kSortThreads * kSortItems) {
         K key[kSortItems];
 #pragma unroll
         for (int k = 0; k < kSortItems; k++) {
@@ -163,7 +175,7 @@ __global__ void __launch_bounds__(kSortThreads) radix_hist_kernel(const K* __res
 #pragma unroll
         for (int k = 0; k < kSortItems; k++) {
             const int i = tbase + warp * (32 * kSortItems) + k * 32 + lane;
-            if (i < end) atomicAdd(&hw[(unsigned)(key[k] >> shift) & (kRadix - 1)], 1u);
+            if (i < end) atomicAdd(&hw[(uint32_t)(key[k] >> shift) & dmask], 1u);
         }
     }
     __syncthreads();
@@ -221,28 +233,62 @@ __global__ void __launch_bounds__(kSortThreads) radix_scan_rows_kernel(uint32_t*
     if (threadIdx.x == 0) totals[blockIdx.x] = carry;
 }
 
-// Stable scatter of one block's chunk, 2048 items at a time: items are ranked
-// by digit (warp match + per-warp counters, so equal digits keep their input
+// Of the lanes in `valid` (a ballot of the whole warp), those whose digit
+// equals this lane's d.
+template <int DB>
+__device__ __forceinline__ uint32_t same_digit(uint32_t valid, uint32_t d) {
+    uint32_t peers = valid;
+#pragma unroll
+    for (int b = 0; b < DB; b++) {
+        const bool bit = (d >> b) & 1u;
+        const uint32_t m = __ballot_sync(0xffffffffu, bit);
+        peers &= bit ? m : ~m;
+    }
+    return peers;
+}
+
+// Exclusive scan of one value per thread of a scatter block.  Ends with a
+// barrier.
+__device__ __forceinline__ uint32_t scatter_scan(uint32_t v, uint32_t* wsum) {
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= (unsigned)o) x += y;
+    }
+    if (lane == 31) wsum[warp] = x;
+    __syncthreads();
+    uint32_t before = x - v;
+    for (unsigned w = 0; w < warp; w++) before += wsum[w];
+    __syncthreads();
+    return before;
+}
+
+// Stable scatter of one block's chunk, 3072 items at a time: items are ranked
+// by digit (ballots + per-warp counters, so equal digits keep their input
 // order), regrouped by digit in shared memory, and written out as runs of
 // consecutive positions.  K: 64- or 32-bit keys.
-template <typename K>
-__global__ void __launch_bounds__(kSortThreads) radix_scatter_kernel(
+template <typename K, int DB>
+__global__ void __launch_bounds__(kSortThreads, 4) radix_scatter_kernel(
     const K* __restrict__ kin, const uint32_t* __restrict__ vin, K* __restrict__ kout,
-    uint32_t* __restrict__ vout, int n, int chunk, const int64_t* __restrict__ n_dev, int shift,
+    uint32_t* __restrict__ vout, int n, int chunk, const int64_t* __restrict__ n_dev, int shift, int dbits,
     const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ totals) {
     __shared__ uint32_t run_off[kRadix];
     __shared__ uint32_t tile_base[kRadix];
     __shared__ uint32_t wsum[kSortWarps];
     __shared__ uint32_t wcnt[kSortWarps][kRadix];
-    __shared__ K skey[kSortTile];
-    __shared__ uint32_t sval[kSortTile];
+    extern __shared__ __align__(16) unsigned char sort_smem[];
+    K* skey = reinterpret_cast<K*>(sort_smem);
+    uint32_t* sval = reinterpret_cast<uint32_t*>(skey + kSortTile);
     resolve_count(n_dev, n, chunk);
+    const uint32_t dmask = (1u << dbits) - 1u;
     const int tid = threadIdx.x, warp = tid >> 5;
     const unsigned lane = tid & 31;
     const unsigned lt_mask = (1u << lane) - 1u;
     // digit d starts at (sum of the totals of smaller digits) + (this block's row prefix)
     {
-        const uint32_t base = block_exclusive_scan(totals[tid], wsum, nullptr);
+        const uint32_t base = scatter_scan(totals[tid], wsum);
         run_off[tid] = base + offsets[(size_t)tid * gridDim.x + blockIdx.x];
     }
     const int start = blockIdx.x * chunk;
@@ -260,22 +306,24 @@ __global__ void __launch_bounds__(kSortThreads) radix_scatter_kernel(
             key[k] = i < end ? kin[i] : K(0);
             val[k] = i < end ? vin[i] : 0u;
         }
+        // Each round's lowest lane of a digit adds its count to the warp's
+        // counter; the additions of a warp are in order, so no round waits for
+        // the one before.
+        uint32_t old[kSortItems];
 #pragma unroll
         for (int k = 0; k < kSortItems; k++) {
             const int i = tbase + warp * (32 * kSortItems) + k * 32 + (int)lane;
-            const bool valid = i < end;
-            const unsigned mask = __ballot_sync(0xffffffffu, valid);
-            uint32_t d = 0, before = 0, peers = 0;
-            if (valid) {
-                d = (uint32_t)(key[k] >> shift) & (kRadix - 1);
-                peers = __match_any_sync(mask, d);
-                before = wcnt[warp][d];
-                rank[k] = before + __popc(peers & lt_mask);
-            }
-            __syncwarp();
-            if (valid && lane == (unsigned)(31 - __clz(peers))) wcnt[warp][d] = before + __popc(peers);
+            const uint32_t d = (uint32_t)(key[k] >> shift) & dmask;
+            const uint32_t peers = same_digit<DB>(__ballot_sync(0xffffffffu, i < end), d);
+            const uint32_t first = __ffs(peers) - 1;
+            old[k] = 0;
+            if (i < end && first == lane) old[k] = atomicAdd(&wcnt[warp][d], (uint32_t)__popc(peers));
+            rank[k] = (first << 8) | (uint32_t)__popc(peers & lt_mask);
             __syncwarp();
         }
+#pragma unroll
+        for (int k = 0; k < kSortItems; k++)
+            rank[k] = __shfl_sync(0xffffffffu, old[k], rank[k] >> 8) + (rank[k] & 255u);
         __syncthreads();
         // per-warp offsets within each digit, then the digit's start in the tile
         uint32_t tot = 0;
@@ -285,14 +333,14 @@ __global__ void __launch_bounds__(kSortThreads) radix_scatter_kernel(
             wcnt[w][tid] = tot;
             tot += c;
         }
-        const uint32_t tb = block_exclusive_scan(tot, wsum, nullptr);
+        const uint32_t tb = scatter_scan(tot, wsum);
         tile_base[tid] = tb;
         __syncthreads();
 #pragma unroll
         for (int k = 0; k < kSortItems; k++) {
             const int i = tbase + warp * (32 * kSortItems) + k * 32 + (int)lane;
             if (i < end) {
-                const uint32_t d = (uint32_t)(key[k] >> shift) & (kRadix - 1);
+                const uint32_t d = (uint32_t)(key[k] >> shift) & dmask;
                 const uint32_t local = tile_base[d] + wcnt[warp][d] + rank[k];
                 skey[local] = key[k];
                 sval[local] = val[k];
@@ -302,7 +350,7 @@ __global__ void __launch_bounds__(kSortThreads) radix_scatter_kernel(
         const int tile_n = min(kSortTile, end - tbase);
         for (int l = tid; l < tile_n; l += kSortThreads) {
             const K kk = skey[l];
-            const uint32_t d = (uint32_t)(kk >> shift) & (kRadix - 1);
+            const uint32_t d = (uint32_t)(kk >> shift) & dmask;
             const uint32_t pos = run_off[d] + (uint32_t)l - tile_base[d];
             kout[pos] = kk;
             vout[pos] = sval[l];
@@ -719,6 +767,7 @@ static int sort_impl(int n, const int64_t* n_dev, int end_bit, const K* keys_in,
     w += align_up((size_t)n * 4, 256);
     uint32_t* hist = (uint32_t*)w;
     uint32_t* totals = hist + (size_t)kRadix * p.blocks;
+    const int digit = ceil_div(end_bit, passes);
     // Ping-pong so that the last pass lands in the output buffers.
     const K* ksrc = keys_in;
     const uint32_t* vsrc = (const uint32_t*)vals_in;
@@ -726,11 +775,17 @@ static int sort_impl(int n, const int64_t* n_dev, int end_bit, const K* keys_in,
         const bool to_out = ((passes - 1 - pass) % 2) == 0;
         K* kdst = to_out ? keys_out : kalt;
         uint32_t* vdst = to_out ? (uint32_t*)vals_out : valt;
-        const int shift = pass * 8;
-        radix_hist_kernel<K><<<p.blocks, kSortThreads, 0, stream>>>(ksrc, n, p.chunk, n_dev, shift, hist);
+        const int shift = pass * digit, dbits = std::min(digit, end_bit - shift);
+        radix_hist_kernel<K><<<p.blocks, kSortThreads, 0, stream>>>(ksrc, n, p.chunk, n_dev, shift, (1u << dbits) - 1u,
+                                                                    hist);
         radix_scan_rows_kernel<<<kRadix, kSortThreads, 0, stream>>>(hist, p.blocks, totals);
-        radix_scatter_kernel<K><<<p.blocks, kSortThreads, 0, stream>>>(ksrc, vsrc, kdst, vdst, n, p.chunk, n_dev,
-                                                                       shift, hist, totals);
+        auto scatter = dbits <= 5 ? radix_scatter_kernel<K, 5> : dbits == 6 ? radix_scatter_kernel<K, 6>
+                     : dbits == 7 ? radix_scatter_kernel<K, 7> : radix_scatter_kernel<K, 8>;
+        const size_t smem = (size_t)kSortTile * (sizeof(K) + 4);
+        cudaError_t e = cudaFuncSetAttribute(scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) { set_cuda_error(e, "sort_pairs"); return GSTEX_ERR_CUDA; }
+        scatter<<<p.blocks, kSortThreads, smem, stream>>>(ksrc, vsrc, kdst, vdst, n, p.chunk, n_dev, shift, dbits,
+                                                             hist, totals);
         ksrc = kdst;
         vsrc = vdst;
     }
