@@ -70,6 +70,7 @@ _BATCH_SIGS = {
     "gstex_get_tile_bin_edges32_dyn": (_I, [_I, _P, _P, _I, _I, _P, _P]),
     "gstex_batch_tile_order_workspace_bytes": (ctypes.c_size_t, [_I]),
     "gstex_batch_tile_order": (_I, [_I, _P, _P, _P, _I, _P, _P, ctypes.c_size_t, _P]),
+    "gstex_batch_tile_groups": (_I, [_I, ctypes.POINTER(ViewDesc), _I, _I, _I, _P, ctypes.POINTER(_I)]),
     "gstex_batch_tile_order_small": (_I, [_I, _P, _P, _P, _P]),
     "gstex_batch_emit": (_I, [_I, _I, _P, _P, _P, _F, _P, _I, _P, _P, _LL, _P, _P, _P, _P, _P]),
     "gstex_sort_pairs_dyn": (_I, [_I, _P, _I, _P, _P, _P, _P, _P, ctypes.c_size_t, _P]),
@@ -304,17 +305,12 @@ class BatchRenderer:
         ([n, 4]: first tile, tiles per row, width, height), with the
         order_group they were made for; None in their place if there are too
         many for the one-launch order."""
-        G, rows, off, n = self.order_group, [], 0, 0
-        for h, w in self.sizes:
-            tx, ty = (w + self.bw - 1) // self.bw, (h + self.bw - 1) // self.bw
-            n += ((tx + G - 1) // G) * ((ty + G - 1) // G) if G >= 1 else self.MAX_SMALL_GROUPS + 1
-            if n > self.MAX_SMALL_GROUPS:
-                return G, None
-            y, x = torch.meshgrid(torch.arange(0, ty, G), torch.arange(0, tx, G), indexing="ij")
-            rows.append(torch.stack([off + y * tx + x, torch.full_like(x, tx), (tx - x).clamp(max=G),
-                                     (ty - y).clamp(max=G)], -1).reshape(-1, 4))
-            off += tx * ty
-        return G, torch.cat(rows).to(torch.int32).to(self.dev)
+        G, n = self.order_group, _I(0)
+        rows = torch.empty((self.MAX_SMALL_GROUPS, 4), dtype=torch.int32)
+        if G < 1 or _L().gstex_batch_tile_groups(self.V, self.descs, self.bw, G, self.MAX_SMALL_GROUPS, ptr(rows),
+                                                 ctypes.byref(n)):
+            return G, None
+        return G, rows[:n.value].to(self.dev)
 
     def _alloc_isect(self):
         L = _L()

@@ -7,6 +7,7 @@
 // are numbered view by view (tile_offset); sort keys are
 // (global tile << 32 | float bits of the camera depth), so one sort orders
 // every view's tiles front to back.
+#include <algorithm>
 #include <vector>
 
 #include "common.cuh"
@@ -424,6 +425,32 @@ extern "C" int gstex_batch_prepare(int num_views, const gstex_view_desc* views, 
                             stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);  // host vectors go out of scope
     if (e != cudaSuccess) { set_cuda_error(e, "batch_prepare"); return GSTEX_ERR_CUDA; }
+    return GSTEX_OK;
+}
+
+extern "C" int gstex_batch_tile_groups(int num_views, const gstex_view_desc* views, int block_width, int group,
+                                       int max_groups, int32_t* groups, int* num_groups) {
+    int total_tiles = 0;
+    long long total_pix = 0;
+    int rc = gstex_batch_layout(num_views, views, block_width, &total_tiles, &total_pix);
+    if (rc) return rc;
+    GSTEX_REQUIRE(group >= 1 && max_groups >= 0 && num_groups && (groups || max_groups == 0));
+    long long n = 0;
+    int off = 0;
+    for (int v = 0; v < num_views; v++) {
+        const int tx = ceil_div(views[v].width, block_width), ty = ceil_div(views[v].height, block_width);
+        for (int y = 0; y < ty; y += group)
+            for (int x = 0; x < tx; x += group, n++) {
+                if (n >= max_groups) return GSTEX_ERR_UNSUPPORTED;
+                int32_t* g = groups + 4 * n;
+                g[0] = off + y * tx + x;
+                g[1] = tx;
+                g[2] = std::min(group, tx - x);
+                g[3] = std::min(group, ty - y);
+            }
+        off += tx * ty;
+    }
+    *num_groups = (int)n;
     return GSTEX_OK;
 }
 

@@ -551,10 +551,10 @@ __global__ void __launch_bounds__(32 * kBlockWarps, kFwdCtas)
 //
 // What bounds it: the L1 data path (71% of its cycles; a 16-byte reduction
 // takes about a cycle per lane there) and the latency of its chains at 16 warps
-// per SM.  Of 22.8 ms on 32 views (36.6 ms with the list walk, its moment
+// per SM.  Of 22.5 ms on 32 views (36.6 ms with the list walk, its moment
 // reduction by shuffles and 8-lane groups) the scan, staging and ray-plane
 // solves take 6 ms, the adjoint 4, texel reads 3.5, texel atomics 4 and the
-// sums 5.  8 clustered full-HD views: 22.3 -> 13.7 ms; one 800x800 view of 1x1
+// sums 5.  8 clustered full-HD views: 22.3 -> 13.5 ms; one 800x800 view of 1x1
 // charts 254 -> 111 us; one full-HD view of large splats 36.0 -> 8.4 ms (where
 // the list walk also staged every splat behind the last contributor).
 // ---------------------------------------------------------------------------
@@ -752,13 +752,15 @@ __device__ __forceinline__ void add_coarse_texel_grads(const BwdMem& M, const Sc
     if (cell.i00 >= 0) flush();
 }
 
+// (The sums as asynchronous bulk additions from shared memory, 80 and 16 bytes a
+// splat, took 23.5 instead of 22.5 ms on 32 views.)
 // Adds the sums of one splat over the pixels of a block to its gradients (the
-// moment layout of finalize_kernel).  m: 0-2 colour, 3 opacity, 4-6 l1^2, l2^2,
+// moment rows of finalize_kernel).  m: 0-2 colour, 3 opacity, 4-6 l1^2, l2^2,
 // l1 l2 times v_sigma, 7-8 l v_sigma, 9-11 (1, l1, l2) v_t / (n . r), 12-14
 // normal, 15-16 v_uv, 17-20 l v_uv, 21-22 blur; l in units of the scales.
 template <int FIX>
-__device__ __forceinline__ void flush_moments(const float* m, const SceneArgs& a, const BlockArgs& ba, const BwdArgs& g,
-                                              const Block& J, int gid, float is1, float is2, bool use_blur) {
+__device__ __forceinline__ void flush_moments(const float* m, const BlockArgs& ba, const BwdArgs& g, const Block& J,
+                                              int gid, bool use_blur) {
     if (ba.vc_stride == 4) {
         atomicAdd(reinterpret_cast<float4*>(J.vcolors) + gid, make_float4(m[0], m[1], m[2], 0.f));
     } else {
@@ -767,25 +769,18 @@ __device__ __forceinline__ void flush_moments(const float* m, const SceneArgs& a
         atomicAdd(vc + 1, m[1]);
         atomicAdd(vc + 2, m[2]);
     }
-    float3 vmb = make_float3(0.f, 0.f, 0.f);
-    if (!FIX && use_blur) {
-        // blur moments -> world-space mean gradient (helpers.cuh:155-164, 114-121)
-        const float4 p = __ldg(J.recs[gid].c + kChunkMu);
-        const float rw = 1.f / (p.z + 1e-6f);
-        const float vx = J.fx * m[21], vy = J.fy * m[22];
-        vmb = block_view(ba, J.view).rot_t(make_float3(vx * rw, vy * rw, -(vx * p.x + vy * p.y) * rw * rw));
-    }
-    const float r1 = 1.f / is1, r2 = 1.f / is2;
     float4* dst = reinterpret_cast<float4*>(g.moments + (size_t)gid * kMomStride);
-    atomicAdd(dst + 0, make_float4(m[3], -is1 * a.glob * m[4], -is2 * a.glob * m[5], is1 * m[7]));
-    atomicAdd(dst + 1, make_float4(is2 * m[8], m[9], m[4], is1 * r2 * m[6]));
-    atomicAdd(dst + 2, make_float4(is2 * r1 * m[6], m[5], r1 * m[10], r2 * m[11]));
-    atomicAdd(dst + 3, make_float4(m[12], m[13], m[14], m[15]));
-    atomicAdd(dst + 4, make_float4(m[16], r1 * m[17], r2 * m[18], r1 * m[19]));
-    if (FIX || !use_blur)
-        atomicAdd(reinterpret_cast<float*>(dst + 5), r2 * m[20]);
-    else
-        atomicAdd(dst + 5, make_float4(r2 * m[20], vmb.x, vmb.y, vmb.z));
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+        atomicAdd(dst + q, make_float4(m[3 + 4 * q], m[4 + 4 * q], m[5 + 4 * q], m[6 + 4 * q]));
+    atomicAdd(reinterpret_cast<float2*>(dst + 4), make_float2(m[19], m[20]));
+    if (!FIX && use_blur) {
+        const float3 vmb = blur_mean_grad(block_view(ba, J.view), f3(__ldg(J.recs[gid].c + kChunkMu)), m[21], m[22]);
+        float* vb = reinterpret_cast<float*>(dst + 5);
+        atomicAdd(vb + 0, vmb.x);
+        atomicAdd(vb + 1, vmb.y);
+        atomicAdd(vb + 2, vmb.z);
+    }
 }
 
 template <int TM, int CT, int FIX>
@@ -949,8 +944,7 @@ __global__ void __launch_bounds__(32 * kBlockWarps, kBwdCtas)
 #pragma unroll
                     for (int q = 4; q < 9; q++) m[q] *= -nop.z;
                 }
-                flush_moments<FIX>(m, a, ba, g, J, M.q.gid[k], M.rec.c[kChunkCol - kChunkOrg][k].w,
-                                   M.rec.c[kChunkNrm - kChunkOrg][k].w, use_blur);
+                flush_moments<FIX>(m, ba, g, J, M.q.gid[k], use_blur);
             }
             if (CT == 3) {
                 const unsigned coarse = is_coarse(nop) ? own : 0u;

@@ -51,4 +51,12 @@ __device__ __forceinline__ T ld_or(const T* p, size_t i, T z) {
     return p ? p[i] : z;
 }
 
+// Blur moments -> world-space mean gradient (helpers.cuh:155-164, 114-121);
+// p: the camera-space mean.
+__device__ __forceinline__ float3 blur_mean_grad(const View& V, float3 p, float mx, float my) {
+    const float rw = 1.f / (p.z + 1e-6f);
+    const float vx = V.fx * mx, vy = V.fy * my;
+    return V.rot_t(make_float3(vx * rw, vy * rw, -(vx * p.x + vy * p.y) * rw * rw));
+}
+
 }  // namespace gstex

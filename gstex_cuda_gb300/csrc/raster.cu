@@ -559,7 +559,7 @@ __device__ __forceinline__ void bwd_pair(const SceneArgs& a, const BwdArgs& g, c
     S.vT_run = vT_cur;
     const float v_sigma = -nbf * Hr.nop.z * e * v_alpha;
     // sigma = (l1s^2 + l2s^2) / 2 with l_ks = l_k * is_k, so v_lk = is_k l_ks v_sigma;
-    // the per-Gaussian factors is_k, 1 / is_k and glob are applied at the flush
+    // the per-Gaussian factors is_k, 1 / is_k and glob are applied by finalize_kernel
     const float p1 = H.l1s * v_sigma, p2 = H.l2s * v_sigma;
     const float l1 = __fdividef(H.l1s, is1), l2 = __fdividef(H.l2s, is2);
     // ray . axis from the hit: l = a . (t r - mu) gives a . r = (l + a . mu) / t
@@ -796,37 +796,12 @@ __device__ __forceinline__ void bwd_tile(const SceneArgs& a, const TileJob& J, c
                     atomicAdd(vc + 2, sm[2]);
                 }
                 float4* dst = reinterpret_cast<float4*>(g.moments + (size_t)gid * kMomStride);
-                // blur moments -> world-space mean gradient (helpers.cuh:155-164, 114-121)
-                const float3 p = f3(R.cold[tr].mu);
-                const float rw = 1.f / (p.z + 1e-6f);
-                const float vx = V.fx * sm[21], vy = V.fy * sm[22];
-                const float3 vmb = V.rot_t(make_float3(vx * rw, vy * rw, -(vx * p.x + vy * p.y) * rw * rw));
-                // the per-Gaussian factors left out of the pixel sums
-                const float is1 = R.warm[tr].col.w, is2 = R.warm[tr].nrm.w;
-                const float r1 = 1.f / is1, r2 = 1.f / is2;
-                float v[kMomStride];
-                v[0] = sm[3];
-                v[1] = -is1 * a.glob * sm[4];
-                v[2] = -is2 * a.glob * sm[5];
-                v[3] = is1 * sm[7];
-                v[4] = is2 * sm[8];
-                v[5] = sm[9];
-                v[6] = sm[4];
-                v[7] = is1 * r2 * sm[6];
-                v[8] = is2 * r1 * sm[6];
-                v[9] = sm[5];
-                v[10] = r1 * sm[10];
-                v[11] = r2 * sm[11];
-                v[12] = sm[12]; v[13] = sm[13]; v[14] = sm[14];
-                v[15] = sm[15]; v[16] = sm[16];
-                v[17] = r1 * sm[17];
-                v[18] = r2 * sm[18];
-                v[19] = r1 * sm[19];
-                v[20] = r2 * sm[20];
-                v[21] = vmb.x; v[22] = vmb.y; v[23] = vmb.z;
+                const float3 vmb = blur_mean_grad(V, f3(R.cold[tr].mu), sm[21], sm[22]);
 #pragma unroll
-                for (int q = 0; q < kMomStride / 4; q++)
-                    atomicAdd(dst + q, make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]));
+                for (int q = 0; q < 4; q++)
+                    atomicAdd(dst + q, make_float4(sm[3 + 4 * q], sm[4 + 4 * q], sm[5 + 4 * q], sm[6 + 4 * q]));
+                atomicAdd(dst + 4, make_float4(sm[19], sm[20], 0.f, 0.f));
+                atomicAdd(dst + 5, make_float4(vmb.x, vmb.y, vmb.z, 0.f));
             }
         }
     }
@@ -1183,19 +1158,29 @@ int launch_records(const SceneArgs& a, const BatchArgs& ba, int num_views, const
 // d/d theta = vu.v - vv.u and, with us cs = u.a1 and us sn = u.a2, the
 // gradients into the axes a1, a2 that join the quaternion's; the
 // normalisation adds (I - q q^T) / |raw q|.
-__global__ void finalize_kernel(int N, const float* __restrict__ mom, const float4* __restrict__ quats,
-                                const float3* __restrict__ umap, const float3* __restrict__ vmap, float* v_opac,
+__global__ void finalize_kernel(int N, const float* __restrict__ mom, const float* __restrict__ scales, float glob,
+                                const float4* __restrict__ quats, const float3* __restrict__ umap, const float3* __restrict__ vmap, float* v_opac,
                                 float3* v_means, float3* v_scales, float4* v_quats, float2* v_uv0, float3* v_umap,
                                 float3* v_vmap, RawGradArgs rg) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N) return;
-    float M[kMomStride];
+    float R[kMomStride];
     const float4* src = reinterpret_cast<const float4*>(mom + (size_t)i * kMomStride);
 #pragma unroll
     for (int q = 0; q < kMomStride / 4; q++) {
         const float4 v = src[q];
-        M[4 * q] = v.x; M[4 * q + 1] = v.y; M[4 * q + 2] = v.z; M[4 * q + 3] = v.w;
+        R[4 * q] = v.x; R[4 * q + 1] = v.y; R[4 * q + 2] = v.z; R[4 * q + 3] = v.w;
     }
+    // R, l in units of the scales s_k = scale_k glob: 0 v_opac, 1-3 (l1^2, l2^2, l1 l2) v_sigma, 4-5 l_k v_sigma,
+    // 6-8 (1, l1, l2) v_t/(n.r), 9-11 vis v_normal, 12-13 v_uv, 14-17 (l1, l2) v_u, (l1, l2) v_v, 20-22 blur
+    // mean gradient; a view changes none of the factors, so they are applied to the sums
+    const float s1 = scales[3 * i] * glob, s2 = scales[3 * i + 1] * glob, is1 = 1.f / s1, is2 = 1.f / s2;
+    // (a sum that no pixel added to stays 0 whatever the scale)
+    auto by = [](float f, float r) { return r == 0.f ? 0.f : f * r; };
+    const float M[kMomStride] = { R[0], by(-is1 * glob, R[1]), by(-is2 * glob, R[2]), by(is1, R[4]), by(is2, R[5]),
+                                  R[6], R[1], by(is1 * s2, R[3]), by(is2 * s1, R[3]), R[2], by(s1, R[7]),
+                                  by(s2, R[8]), R[9], R[10], R[11], R[12], R[13], by(s1, R[14]), by(s2, R[15]),
+                                  by(s1, R[16]), by(s2, R[17]), R[20], R[21], R[22] };
     // M: 0 v_opac, 1-2 v_scale, 3-4 sum v_l, 5 sum v_t/(n.r), 6-9 S_lk v_lj, 10-11 S_l v_t/(n.r),
     //    12-14 sum vis*v_normal, 15-16 sum v_uv, 17-20 S_l v_uv, 21-23 blur mean gradient
     const float4 q = quats[i];
@@ -1363,7 +1348,7 @@ int launch_finalize(const SceneArgs& a, const float* moments, float* v_opac, flo
                     float* v_quats, float* v_uv0, float* v_umap, float* v_vmap, cudaStream_t stream,
                     const RawGradArgs& rg) {
     if (a.N == 0) return GSTEX_OK;
-    finalize_kernel<<<ceil_div(a.N, 256), 256, 0, stream>>>(a.N, moments, a.quats, a.umap, a.vmap, v_opac,
+    finalize_kernel<<<ceil_div(a.N, 256), 256, 0, stream>>>(a.N, moments, a.scales, a.glob, a.quats, a.umap, a.vmap, v_opac,
                                                            (float3*)v_means, (float3*)v_scales, (float4*)v_quats,
                                                            (float2*)v_uv0, (float3*)v_umap, (float3*)v_vmap, rg);
     return check_launch("finalize");
