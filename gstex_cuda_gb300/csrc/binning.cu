@@ -155,7 +155,8 @@ __device__ __forceinline__ void resolve_count(const int64_t* n_dev, int& n, int&
 template <typename K>
 __global__ void __launch_bounds__(kSortThreads) radix_hist_kernel(const K* __restrict__ keys, int n, int chunk,
                                                                   const int64_t* __restrict__ n_dev, int shift,
-                                                                  uint32_t dmask, uint32_t* __restrict__ hist) {
+                                                                  uint32_t dmask, uint32_t* __restrict__ hist,
+                                                                  bool by_block = false) {
     __shared__ uint32_t h[kSortWarps][kRadix];
     for (int i = threadIdx.x; i < kSortWarps * kRadix; i += blockDim.x) (&h[0][0])[i] = 0;
     resolve_count(n_dev, n, chunk);
@@ -183,7 +184,7 @@ __global__ void __launch_bounds__(kSortThreads) radix_hist_kernel(const K* __res
         uint32_t c = 0;
 #pragma unroll
         for (int w = 0; w < kSortWarps; w++) c += h[w][d];
-        hist[(size_t)d * gridDim.x + blockIdx.x] = c;
+        hist[by_block ? (size_t)blockIdx.x * kRadix + d : (size_t)d * gridDim.x + blockIdx.x] = c;
     }
 }
 
@@ -269,11 +270,18 @@ __device__ __forceinline__ uint32_t scatter_scan(uint32_t v, uint32_t* wsum) {
 // by digit (ballots + per-warp counters, so equal digits keep their input
 // order), regrouped by digit in shared memory, and written out as runs of
 // consecutive positions.  K: 64- or 32-bit keys.
-template <typename K, int DB>
+//
+// DIRECT: one tile per block and few blocks.  A pass is then bound by its
+// launches, so there is only this one: `offsets` holds the counts [block][digit]
+// themselves, every block sums them up for its own digits, and counts the next
+// pass's digits (shift + dbits on, next_mask) of the places it writes to into
+// `next`, which is zero before (null in the last pass).
+template <typename K, int DB, bool DIRECT = false>
 __global__ void __launch_bounds__(kSortThreads, 4) radix_scatter_kernel(
     const K* __restrict__ kin, const uint32_t* __restrict__ vin, K* __restrict__ kout,
     uint32_t* __restrict__ vout, int n, int chunk, const int64_t* __restrict__ n_dev, int shift, int dbits,
-    const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ totals) {
+    const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ totals, uint32_t* __restrict__ next = nullptr,
+    uint32_t next_mask = 0u) {
     __shared__ uint32_t run_off[kRadix];
     __shared__ uint32_t tile_base[kRadix];
     __shared__ uint32_t wsum[kSortWarps];
@@ -287,7 +295,22 @@ __global__ void __launch_bounds__(kSortThreads, 4) radix_scatter_kernel(
     const unsigned lane = tid & 31;
     const unsigned lt_mask = (1u << lane) - 1u;
     // digit d starts at (sum of the totals of smaller digits) + (this block's row prefix)
-    {
+    if (DIRECT) {
+        const int blocks = ceil_div(n, kSortTile);
+        if ((int)blockIdx.x >= blocks) return;
+        uint32_t before = 0, total = 0;
+        for (int b0 = 0; b0 < blocks; b0 += 32) {
+            uint32_t c[32];  // (all loads of a round first)
+#pragma unroll
+            for (int j = 0; j < 32; j++) c[j] = b0 + j < blocks ? offsets[(size_t)(b0 + j) * kRadix + tid] : 0u;
+#pragma unroll
+            for (int j = 0; j < 32; j++) {
+                before += b0 + j < (int)blockIdx.x ? c[j] : 0u;
+                total += c[j];
+            }
+        }
+        run_off[tid] = scatter_scan(total, wsum) + before;
+    } else {
         const uint32_t base = scatter_scan(totals[tid], wsum);
         run_off[tid] = base + offsets[(size_t)tid * gridDim.x + blockIdx.x];
     }
@@ -354,6 +377,8 @@ __global__ void __launch_bounds__(kSortThreads, 4) radix_scatter_kernel(
             const uint32_t pos = run_off[d] + (uint32_t)l - tile_base[d];
             kout[pos] = kk;
             vout[pos] = sval[l];
+            if (DIRECT && next)
+                atomicAdd(&next[(size_t)(pos / kSortTile) * kRadix + ((uint32_t)(kk >> (shift + dbits)) & next_mask)], 1u);
         }
         __syncthreads();
         // advance each digit's cursor by the tile's count of that digit
@@ -734,10 +759,23 @@ extern "C" int gstex_map_gaussian_to_intersects(int n, int num_isect, const floa
     return check_launch("map_gaussian_to_intersects");
 }
 
+// 32-bit sorts of at most this many tiles take one launch a pass (DIRECT)
+// instead of three.  Every block reads the counts of all blocks, so the gain
+// shrinks with their number: 32 bits of 100k items 66 -> 46 us, 240k 66 -> 52,
+// 390k 66 -> 55, 500k (163 tiles) 74 -> 72, 780k (254) 74 -> 80.  A count on the
+// device is often a third of the capacity that the host knows, so the line lies
+// higher there.
+constexpr int kDirectBlocks = 192, kDirectBlocksDyn = 384;
+
+static bool sort_direct(const SortPlan& p, size_t key_bytes, bool dyn) {
+    return key_bytes == 4 && p.chunk == kSortTile && p.blocks <= (dyn ? kDirectBlocksDyn : kDirectBlocks);
+}
+
 static size_t sort_workspace_bytes(int n, size_t key_bytes) {
     if (n < 1) n = 1;
     const SortPlan p = sort_plan(n);
-    return align_up((size_t)n * key_bytes, 256) + align_up((size_t)n * 4, 256) + (size_t)kRadix * p.blocks * 4 +
+    const size_t counts = sort_direct(p, key_bytes, true) ? 4 : 1;  // of each pass, or of one
+    return align_up((size_t)n * key_bytes, 256) + align_up((size_t)n * 4, 256) + counts * kRadix * p.blocks * 4 +
            (size_t)kRadix * 4;
 }
 
@@ -771,25 +809,51 @@ static int sort_impl(int n, const int64_t* n_dev, int end_bit, const K* keys_in,
     // Ping-pong so that the last pass lands in the output buffers.
     const K* ksrc = keys_in;
     const uint32_t* vsrc = (const uint32_t*)vals_in;
+    const bool direct = sort_direct(p, sizeof(K), n_dev != nullptr);
+    const size_t row = (size_t)kRadix * p.blocks;  // counts of one pass
+    if (direct) {
+        if (passes > 1) {
+            cudaError_t e = cudaMemsetAsync(hist + row, 0, (passes - 1) * row * 4, stream);
+            if (e != cudaSuccess) { set_cuda_error(e, "sort_pairs memset"); return GSTEX_ERR_CUDA; }
+        }
+        radix_hist_kernel<K><<<p.blocks, kSortThreads, 0, stream>>>(ksrc, n, p.chunk, n_dev, 0,
+                                                                    (1u << std::min(digit, end_bit)) - 1u, hist, true);
+    }
     for (int pass = 0; pass < passes; pass++) {
         const bool to_out = ((passes - 1 - pass) % 2) == 0;
         K* kdst = to_out ? keys_out : kalt;
         uint32_t* vdst = to_out ? (uint32_t*)vals_out : valt;
         const int shift = pass * digit, dbits = std::min(digit, end_bit - shift);
+        const size_t smem = (size_t)kSortTile * (sizeof(K) + 4);
+        if (direct) {
+            if constexpr (sizeof(K) == 4) {
+                const int left = end_bit - shift - dbits;
+                const uint32_t next_mask = left > 0 ? (1u << std::min(digit, left)) - 1u : 0u;
+                auto scatter = dbits <= 5 ? radix_scatter_kernel<K, 5, true> : dbits == 6 ? radix_scatter_kernel<K, 6, true>
+                             : dbits == 7 ? radix_scatter_kernel<K, 7, true> : radix_scatter_kernel<K, 8, true>;
+                cudaError_t e = cudaFuncSetAttribute(scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                if (e != cudaSuccess) { set_cuda_error(e, "sort_pairs"); return GSTEX_ERR_CUDA; }
+                scatter<<<p.blocks, kSortThreads, smem, stream>>>(ksrc, vsrc, kdst, vdst, n, p.chunk, n_dev, shift, dbits,
+                                                                  hist + pass * row, nullptr,
+                                                                  left > 0 ? hist + (pass + 1) * row : nullptr, next_mask);
+            }
+            ksrc = kdst;
+            vsrc = vdst;
+            continue;
+        }
         radix_hist_kernel<K><<<p.blocks, kSortThreads, 0, stream>>>(ksrc, n, p.chunk, n_dev, shift, (1u << dbits) - 1u,
                                                                     hist);
         radix_scan_rows_kernel<<<kRadix, kSortThreads, 0, stream>>>(hist, p.blocks, totals);
         auto scatter = dbits <= 5 ? radix_scatter_kernel<K, 5> : dbits == 6 ? radix_scatter_kernel<K, 6>
                      : dbits == 7 ? radix_scatter_kernel<K, 7> : radix_scatter_kernel<K, 8>;
-        const size_t smem = (size_t)kSortTile * (sizeof(K) + 4);
         cudaError_t e = cudaFuncSetAttribute(scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) { set_cuda_error(e, "sort_pairs"); return GSTEX_ERR_CUDA; }
         scatter<<<p.blocks, kSortThreads, smem, stream>>>(ksrc, vsrc, kdst, vdst, n, p.chunk, n_dev, shift, dbits,
-                                                             hist, totals);
+                                                          hist, totals, nullptr, 0u);
         ksrc = kdst;
         vsrc = vdst;
     }
-    return check_launch("sort_pairs", 3 * passes);
+    return check_launch("sort_pairs", direct ? 1 + passes : 3 * passes);
 }
 
 extern "C" int gstex_sort_pairs(int n, int end_bit, const int64_t* keys_in, const int32_t* vals_in,
