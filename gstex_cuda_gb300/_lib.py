@@ -62,6 +62,7 @@ _SIGS = {
     "gstex_view_records": (_I, [_P, _P, ctypes.c_size_t, _P]),
     "gstex_scan_workspace_bytes": (ctypes.c_size_t, [_I]),
     "gstex_inclusive_scan_i32": (_I, [_I, _P, _P, _P, _P, ctypes.c_size_t, _P]),
+    "gstex_inclusive_scan_picked_i32": (_I, [_I, _P, _P, _P, _P, _P, _P, ctypes.c_size_t, _P]),
     "gstex_compute_sh_forward": (_I, [_I, _I, _I, _P, _P, _P, _P]),
     "gstex_compute_sh_backward": (_I, [_I, _I, _I, _P, _P, _P, _P]),
     "gstex_map_gaussian_to_intersects": (_I, [_I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _P, _P, _P]),

@@ -408,10 +408,9 @@ class BatchRenderer:
         # sort by (global tile << 1 | real)
         check(L.gstex_sort_pairs32(VN, None, 32, ptr(self.dkeys), ptr(self.pair_ids), ptr(self.dkeys_sorted),
                                    ptr(self.order), ptr(self.dsort_ws), self.dsort_ws.numel(), st), "sort_pairs32")
-        check(L.gstex_batch_gather_counts(VN, ptr(self.order), ptr(self.counts), ptr(self.scounts), st),
-              "batch_gather_counts")
-        check(L.gstex_inclusive_scan_i32(VN, ptr(self.scounts), ptr(self.cum), ptr(self.total), ptr(self.scan_ws),
-                                         self.scan_ws.numel(), st), "scan")
+        check(L.gstex_inclusive_scan_picked_i32(VN, ptr(self.counts), ptr(self.order), ptr(self.scounts),
+                                                ptr(self.cum), ptr(self.total), ptr(self.scan_ws),
+                                                self.scan_ws.numel(), st), "scan_picked")
         check(L.gstex_batch_emit_sorted(self.N, self.V, ptr(self.views_dev), ptr(self.order), ptr(self.cum),
                                         ptr(self.rects), ptr(self.total), self.capacity, ptr(self.keys),
                                         ptr(self.vals), ptr(self.count), ptr(self.overflow), st), "batch_emit_sorted")

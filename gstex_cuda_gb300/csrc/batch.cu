@@ -161,11 +161,20 @@ __global__ void gather_counts_kernel(int n, const int32_t* __restrict__ order, c
     if (p < n) out[p] = counts[order[p]];
 }
 
+// The number of slots written, and whether there were more than that.
+__device__ __forceinline__ void clamp_count(const int64_t* total, long long capacity, int64_t* n, int* overflow) {
+    const long long t = *total;
+    *n = t < capacity ? t : capacity;
+    if (t > capacity) atomicOr(overflow, 1);
+}
+
 // Pair p of the depth order writes [cum[p-1], cum[p]) (clipped to the capacity).
 __global__ void batch_emit_sorted_kernel(int VN, int N, const BatchView* __restrict__ views,
                                          const int32_t* __restrict__ order, const int32_t* __restrict__ cum,
-                                         const uint2* __restrict__ rects, long long capacity,
-                                         uint32_t* __restrict__ keys, int32_t* __restrict__ vals) {
+                                         const uint2* __restrict__ rects, const int64_t* __restrict__ total,
+                                         long long capacity, uint32_t* __restrict__ keys, int32_t* __restrict__ vals,
+                                         int64_t* __restrict__ count, int* __restrict__ overflow) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) clamp_count(total, capacity, count, overflow);
     // A warp emits the slots of its 32 pairs, which are contiguous: each lane
     // takes every 32nd slot of the range, finds its pair by a binary search
     // over the pairs' first slots and writes one key, so the stores are
@@ -353,9 +362,7 @@ __global__ void __launch_bounds__(RowStage<1>::kRows) batch_sh_backward_kernel(i
 
 __global__ void clamp_count_kernel(const int64_t* __restrict__ total, long long capacity, int64_t* __restrict__ n,
                                    int* __restrict__ overflow) {
-    const long long t = *total;
-    *n = t < capacity ? t : capacity;
-    if (t > capacity) atomicOr(overflow, 1);
+    clamp_count(total, capacity, n, overflow);
 }
 
 }  // namespace gstex
@@ -588,13 +595,16 @@ extern "C" int gstex_batch_emit_sorted(int N, int V, const void* views_dev, cons
     GSTEX_REQUIRE(N >= 0 && V > 0 && views_dev && capacity >= 0 && total && count && overflow);
     if ((unsigned long long)N * (unsigned long long)V > 0x7fffffffull) return GSTEX_ERR_UNSUPPORTED;
     cudaStream_t stream = (cudaStream_t)s;
-    clamp_count_kernel<<<1, 1, 0, stream>>>(total, capacity, count, overflow);
-    if (N == 0 || capacity == 0) return check_launch("batch_emit_sorted");
+    if (N == 0 || capacity == 0) {
+        clamp_count_kernel<<<1, 1, 0, stream>>>(total, capacity, count, overflow);
+        return check_launch("batch_emit_sorted");
+    }
     GSTEX_REQUIRE(order && cum && rects && keys && vals && ((uintptr_t)rects & 7) == 0);
     const int VN = N * V;
     batch_emit_sorted_kernel<<<ceil_div(VN, 256), 256, 0, stream>>>(VN, N, (const BatchView*)views_dev, order, cum,
-                                                                     (const uint2*)rects, capacity, keys, vals);
-    return check_launch("batch_emit_sorted", 2);
+                                                                     (const uint2*)rects, total, capacity, keys, vals, count,
+                                                                     overflow);
+    return check_launch("batch_emit_sorted");
 }
 
 extern "C" int gstex_batch_emit(int N, int V, const void* views_dev, const float* means, const float* scales,
@@ -677,7 +687,9 @@ extern "C" int gstex_batch_records(const gstex_batch_inputs* in, const int32_t* 
                           (cudaStream_t)s);
 }
 
-static int grid_of(const gstex_batch_inputs* in, bool backward) {
+// (of the tile kernels)
+static int grid_of(const gstex_batch_inputs* in, const BatchArgs& ba, bool backward) {
+    if (blocks_apply(in->block_width, in->channels, in->settings, ba.recs)) return 0;
     if (in->grid > 0) return in->grid;
     int g = resident_ctas(in->block_width, backward, in->texture_dtype, in->channels, in->pixels_per_thread,
                           in->group_lanes, backward ? in->resident_ctas : 0, in->batch_size, in->settings);
@@ -693,11 +705,9 @@ extern "C" int gstex_batch_forward(const gstex_batch_inputs* in, const gstex_for
                   out->depth_idx && out->reg_s);
     if (a.C > 0) GSTEX_REQUIRE(out->texture);
     cudaStream_t stream = (cudaStream_t)s;
-    cudaError_t e = cudaMemsetAsync(in->queue, 0, sizeof(int), stream);
-    if (e != cudaSuccess) { set_cuda_error(e, "batch_forward"); return GSTEX_ERR_CUDA; }
     FwdOut o{ (float3*)out->img, out->depth, out->reg, out->texture, (float3*)out->normal, out->final_T,
               out->final_idx, out->depth_idx, (float3*)out->reg_s };
-    return launch_fwd_batch(a, ba, o, in->block_width, in->texture_dtype, in->pixels_per_thread, grid_of(in, false),
+    return launch_fwd_batch(a, ba, o, in->block_width, in->texture_dtype, in->pixels_per_thread, grid_of(in, ba, false),
                             stream);
 }
 
@@ -730,8 +740,7 @@ static int batch_backward_impl(const gstex_batch_inputs* in, const gstex_backwar
     if (io->workspace_bytes < gstex_batch_backward_workspace_bytes(a.N)) return GSTEX_ERR_CAPACITY;
     if (a.N == 0) return GSTEX_OK;
     cudaStream_t stream = (cudaStream_t)s;
-    cudaError_t e = cudaMemsetAsync(in->queue, 0, sizeof(int), stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(io->workspace, 0, gstex_batch_backward_workspace_bytes(a.N), stream);
+    cudaError_t e = cudaMemsetAsync(io->workspace, 0, gstex_batch_backward_workspace_bytes(a.N), stream);
     if (e == cudaSuccess)
         e = cudaMemsetAsync(io->v_colors, 0, (size_t)in->num_views * a.N * 4 * sizeof(float), stream);
     if (e != cudaSuccess) { set_cuda_error(e, "batch_backward"); return GSTEX_ERR_CUDA; }
@@ -740,7 +749,7 @@ static int batch_backward_impl(const gstex_batch_inputs* in, const gstex_backwar
                io->v_depth, io->v_reg, io->v_alpha, io->v_texture, (const float3*)io->v_normal,
                (float*)io->workspace, io->v_tex_grad };
     if ((rc = launch_bwd_batch(a, ba, g, in->block_width, in->texture_dtype, in->pixels_per_thread,
-                               in->group_lanes, in->resident_ctas, grid_of(in, true), stream)))
+                               in->group_lanes, in->resident_ctas, grid_of(in, ba, true), stream)))
         return rc;
     return launch_finalize(a, (const float*)io->workspace, io->v_opacity, io->v_means, io->v_scales, io->v_quats,
                            io->v_uv0, io->v_umap, io->v_vmap, stream, rg);

@@ -151,12 +151,13 @@ __device__ __forceinline__ void resolve_count(const int64_t* n_dev, int& n, int&
 // Per-block digit counts: each warp loads its kSortItems keys per thread of a
 // tile of items up front (so the loads overlap) and counts them in its own
 // shared-memory histogram with plain atomics; the warps' histograms are summed
-// at the end.
+// at the end.  by_block: as [block][digit], followed by zeros for that many
+// passes less one.
 template <typename K>
 __global__ void __launch_bounds__(kSortThreads) radix_hist_kernel(const K* __restrict__ keys, int n, int chunk,
                                                                   const int64_t* __restrict__ n_dev, int shift,
                                                                   uint32_t dmask, uint32_t* __restrict__ hist,
-                                                                  bool by_block = false) {
+                                                                  int by_block = 0) {
     __shared__ uint32_t h[kSortWarps][kRadix];
     for (int i = threadIdx.x; i < kSortWarps * kRadix; i += blockDim.x) (&h[0][0])[i] = 0;
     resolve_count(n_dev, n, chunk);
@@ -184,7 +185,11 @@ __global__ void __launch_bounds__(kSortThreads) radix_hist_kernel(const K* __res
         uint32_t c = 0;
 #pragma unroll
         for (int w = 0; w < kSortWarps; w++) c += h[w][d];
-        hist[by_block ? (size_t)blockIdx.x * kRadix + d : (size_t)d * gridDim.x + blockIdx.x] = c;
+        if (by_block) {
+            for (int p = 0; p < by_block; p++) hist[((size_t)p * gridDim.x + blockIdx.x) * kRadix + d] = p ? 0u : c;
+        } else {
+            hist[(size_t)d * gridDim.x + blockIdx.x] = c;
+        }
     }
 }
 
@@ -812,12 +817,8 @@ static int sort_impl(int n, const int64_t* n_dev, int end_bit, const K* keys_in,
     const bool direct = sort_direct(p, sizeof(K), n_dev != nullptr);
     const size_t row = (size_t)kRadix * p.blocks;  // counts of one pass
     if (direct) {
-        if (passes > 1) {
-            cudaError_t e = cudaMemsetAsync(hist + row, 0, (passes - 1) * row * 4, stream);
-            if (e != cudaSuccess) { set_cuda_error(e, "sort_pairs memset"); return GSTEX_ERR_CUDA; }
-        }
         radix_hist_kernel<K><<<p.blocks, kSortThreads, 0, stream>>>(ksrc, n, p.chunk, n_dev, 0,
-                                                                    (1u << std::min(digit, end_bit)) - 1u, hist, true);
+                                                                    (1u << std::min(digit, end_bit)) - 1u, hist, passes);
     }
     for (int pass = 0; pass < passes; pass++) {
         const bool to_out = ((passes - 1 - pass) % 2) == 0;
@@ -952,8 +953,8 @@ extern "C" int gstex_view_order(int n, const float* depths, const int32_t* count
     if (rc) return rc;
     rc = gstex_sort_pairs32(n, nullptr, 32, keys, ids, sorted, order, w + 4 * a, sb, s);
     if (rc) return rc;
-    if ((rc = gstex_batch_gather_counts(n, order, counts, scounts, s))) return rc;
-    return gstex_inclusive_scan_i32(n, scounts, cum, info, w + 4 * a + sb, gstex_scan_workspace_bytes(n), s);
+    return gstex_inclusive_scan_picked_i32(n, counts, order, scounts, cum, info, w + 4 * a + sb,
+                                           gstex_scan_workspace_bytes(n), s);
 }
 
 extern "C" size_t gstex_view_bins_workspace_bytes(int num_isect) {

@@ -1393,6 +1393,12 @@ static BlockArgs block_args(const ViewArgs& va, int bw, int n) {
     return b;
 }
 
+static int zero_queue(const BatchArgs& ba, cudaStream_t stream, const char* what) {
+    cudaError_t e = cudaMemsetAsync(ba.queue, 0, sizeof(int), stream);
+    if (e != cudaSuccess) { set_cuda_error(e, what); return GSTEX_ERR_CUDA; }
+    return GSTEX_OK;
+}
+
 int launch_fwd_batch(const SceneArgs& a, const BatchArgs& ba, const FwdOut& o, int bw, int texmode, int ppt, int grid,
                      cudaStream_t stream) {
     if (blocks_apply(bw, a.C, a.settings, ba.recs)) return launch_fwd_blocks(a, block_args(ba, bw), o, texmode, stream);
@@ -1401,6 +1407,7 @@ int launch_fwd_batch(const SceneArgs& a, const BatchArgs& ba, const FwdOut& o, i
     const size_t smem = fwd_smem(bw, ppt, a.batch);
     int rc = set_smem(k, smem, "batch forward");
     if (rc) return rc;
+    if ((rc = zero_queue(ba, stream, "batch forward"))) return rc;
     k<<<grid, block_of(bw, ppt), smem, stream>>>(a, ba, o);
     return check_launch("batch forward");
 }
@@ -1443,6 +1450,7 @@ int launch_bwd_batch(const SceneArgs& a, const BatchArgs& ba, const BwdArgs& g, 
     const size_t smem = bwd_smem(bw, ppt, gs, a.batch);
     int rc = set_bwd_smem(k, smem, "batch backward");
     if (rc) return rc;
+    if ((rc = zero_queue(ba, stream, "batch backward"))) return rc;
     k<<<grid, block_of(bw, ppt), smem, stream>>>(a, ba, g);
     return check_launch("batch backward");
 }

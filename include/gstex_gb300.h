@@ -69,6 +69,9 @@ int gstex_num_tiles_hit(int n, const float* centers, const float* extents, int i
 size_t gstex_scan_workspace_bytes(int n);
 int gstex_inclusive_scan_i32(int n, const int32_t* counts, int32_t* cum, int64_t* total, void* workspace,
                              size_t workspace_bytes, gstex_stream_t stream);
+/* The same of counts[order[i]], which picked [n] receives. */
+int gstex_inclusive_scan_picked_i32(int n, const int32_t* counts, const int32_t* order, int32_t* picked, int32_t* cum,
+                                    int64_t* total, void* workspace, size_t workspace_bytes, gstex_stream_t stream);
 
 /* Spherical harmonics colours from coefficients [n, bases(degree), 3] using
  * the first bases(degrees_to_use) bases.  Replaces _C.compute_sh_forward
@@ -358,7 +361,7 @@ int gstex_batch_emit(int num_points, int num_views, const void* views_dev, const
  *      pair_ids[j] = j and the tile rectangle rects [V*N, 2] (uint32 x0 | x1 << 16,
  *      y0 | y1 << 16; 8-byte aligned);
  *   2. gstex_sort_pairs32 of (depth_keys, pair_ids), end_bit 32 -> order;
- *   3. gstex_batch_gather_counts(order) and gstex_inclusive_scan_i32 -> cum;
+ *   3. gstex_inclusive_scan_picked_i32 of the counts in that order -> cum;
  *   4. gstex_batch_emit_sorted: pair order[p] writes [cum[p-1], cum[p]) with
  *      keys (global tile << 1 | 1) and its Gaussian id; slots it does not write
  *      get (view's first tile << 1 | 0) and Gaussian 0, which sort first in that
