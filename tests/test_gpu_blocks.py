@@ -223,3 +223,31 @@ def test_edit_matches_the_tile_kernel(bw, settings):
     fine = torch.isfinite(old)
     bad = ((new - old).abs() > 1e-5 * (1 + old.abs())) & fine
     assert float(bad.any(1).float().mean()) <= 1e-3
+
+
+@pytest.mark.parametrize("chart", [(1, 1), (1, 5), (2, 16)])
+@pytest.mark.parametrize("offset", [0, 1, 2, 3])
+def test_texel_gradient_words(chart, offset):
+    """Gradients of float32 texels leave as 16-byte words: charts that start at
+    every place within one, a buffer that does too, and its ends, beyond which
+    nothing is touched (-0 + 0 would turn the guards into +0)."""
+    from gstex_cuda_gb300 import batch as B
+    spec = small_scene(n=80, width=40, height=28, seed=offset, chart=chart)
+    _check(Case(spec), 8)
+    cam = spec.cameras[0]
+    scene = B.Scene(**{k: getattr(spec, k).to(DEV) for k in ("means", "scales", "quats", "opacity", "sh_coeffs", "uv0",
+                                                             "umap", "vmap", "texture_dims", "texture")}, sh_degree=0)
+    r = B.BatchRenderer([B.Camera(cam.viewmat, cam.fx, cam.fy, cam.cx, cam.cy, cam.width, cam.height)],
+                        spec.num_points, capacity=1 << 14, block_width=8)
+    gen = torch.Generator().manual_seed(1)
+    tgt = [torch.rand(r.total_pixels, 3, generator=gen).to(DEV) for _ in range(2)]
+    r.step(scene, *tgt)
+    want = r.grads["texture"].clone()
+    n = want.numel()
+    buf = torch.full((n + 16,), -0.0, device=DEV)
+    r.grads["texture"] = buf[4 + offset:4 + offset + n].view(-1, 3)
+    r.step(scene, *tgt)
+    # the sums' order differs between two runs: 80 splats' pairs over a few pixels each
+    assert (r.grads["texture"] - want).abs().max() <= 1e-5 * want.abs().max()
+    guard = torch.cat([buf[:4 + offset], buf[4 + offset + n:]])
+    assert bool(torch.signbit(guard).all()) and bool((guard == 0).all())
