@@ -32,6 +32,7 @@ __global__ void __launch_bounds__(RowStage<1>::kRows) batch_project_kernel(int N
                                      const SHT* __restrict__ sh, int bw, float3* __restrict__ colors,
                                      int32_t* __restrict__ counts, uint32_t* __restrict__ depth_keys,
                                      int32_t* __restrict__ pair_ids, uint2* __restrict__ rects, RawParams raw) {
+    chain_wait();
     constexpr int B = (DEG + 1) * (DEG + 1);
     __shared__ RowStage<3 * B> rows;
     const int i0 = blockIdx.x * rows.kRows, i = i0 + threadIdx.x;
@@ -174,6 +175,7 @@ __global__ void batch_emit_sorted_kernel(int VN, int N, const BatchView* __restr
                                          const uint2* __restrict__ rects, const int64_t* __restrict__ total,
                                          long long capacity, uint32_t* __restrict__ keys, int32_t* __restrict__ vals,
                                          int64_t* __restrict__ count, int* __restrict__ overflow) {
+    chain_wait();
     if (blockIdx.x == 0 && threadIdx.x == 0) clamp_count(total, capacity, count, overflow);
     // A warp emits the slots of its 32 pairs, which are contiguous: each lane
     // takes every 32nd slot of the range, finds its pair by a binary search
@@ -240,6 +242,7 @@ __global__ void batch_emit_sorted_kernel(int VN, int N, const BatchView* __restr
 __global__ void tile_group_keys_kernel(int T, const int2* __restrict__ bins, const int32_t* __restrict__ tile_view,
                                        const BatchView* __restrict__ views, int G, uint32_t* __restrict__ group_key,
                                        int32_t* __restrict__ ids, uint32_t* __restrict__ cost_key) {
+    chain_wait();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= T) return;
     ids[t] = t;
@@ -264,6 +267,7 @@ __global__ void tile_group_keys_kernel(int T, const int2* __restrict__ bins, con
 
 __global__ void gather_keys_kernel(int T, const int32_t* __restrict__ ids, const uint32_t* __restrict__ key,
                                    uint32_t* __restrict__ out) {
+    chain_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < T) out[i] = key[ids[i]];
 }
@@ -281,6 +285,7 @@ __global__ void batch_loss_kernel(long long total, int V, const long long* __res
                                   float w_tex, float w_reg, float w_normal, float3* __restrict__ v_img,
                                   float* __restrict__ v_tex, float3* __restrict__ v_normal, float* __restrict__ v_reg,
                                   float* __restrict__ loss) {
+    chain_wait();
     __shared__ float part[32];
     float acc = 0.f;
     for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < total;
@@ -328,6 +333,7 @@ template <int DEG>
 __global__ void __launch_bounds__(RowStage<1>::kRows) batch_sh_backward_kernel(int N, int V, const BatchView* __restrict__ views,
                                          const float3* __restrict__ means, const float4* __restrict__ vcol,
                                          float* __restrict__ v_coeffs) {
+    chain_wait();
     constexpr int B = (DEG + 1) * (DEG + 1);
     __shared__ RowStage<3 * B> rows;
     const int i0 = blockIdx.x * rows.kRows, i = i0 + threadIdx.x;
@@ -470,11 +476,16 @@ static void project_launch(int deg, int N, int V, const BatchView* bv, const flo
     const float4* q = (const float4*)quats;
     float3* c = (float3*)colors;
     switch (deg) {
-        case 0: batch_project_kernel<SHT, 0><<<grid, block, 0, stream>>>(N, V, bv, m, scales, glob, q, sh, bw, c, counts, dk, ids, rects, raw); break;
-        case 1: batch_project_kernel<SHT, 1><<<grid, block, 0, stream>>>(N, V, bv, m, scales, glob, q, sh, bw, c, counts, dk, ids, rects, raw); break;
-        case 2: batch_project_kernel<SHT, 2><<<grid, block, 0, stream>>>(N, V, bv, m, scales, glob, q, sh, bw, c, counts, dk, ids, rects, raw); break;
-        case 3: batch_project_kernel<SHT, 3><<<grid, block, 0, stream>>>(N, V, bv, m, scales, glob, q, sh, bw, c, counts, dk, ids, rects, raw); break;
-        default: batch_project_kernel<SHT, 4><<<grid, block, 0, stream>>>(N, V, bv, m, scales, glob, q, sh, bw, c, counts, dk, ids, rects, raw); break;
+        case 0: launch_chained(batch_project_kernel<SHT, 0>, grid, block, 0, stream,
+                               N, V, bv, m, scales, glob, q, sh, bw, c, counts, dk, ids, rects, raw); break;
+        case 1: launch_chained(batch_project_kernel<SHT, 1>, grid, block, 0, stream,
+                               N, V, bv, m, scales, glob, q, sh, bw, c, counts, dk, ids, rects, raw); break;
+        case 2: launch_chained(batch_project_kernel<SHT, 2>, grid, block, 0, stream,
+                               N, V, bv, m, scales, glob, q, sh, bw, c, counts, dk, ids, rects, raw); break;
+        case 3: launch_chained(batch_project_kernel<SHT, 3>, grid, block, 0, stream,
+                               N, V, bv, m, scales, glob, q, sh, bw, c, counts, dk, ids, rects, raw); break;
+        default: launch_chained(batch_project_kernel<SHT, 4>, grid, block, 0, stream,
+                                N, V, bv, m, scales, glob, q, sh, bw, c, counts, dk, ids, rects, raw); break;
     }
 }
 
@@ -563,7 +574,7 @@ extern "C" int gstex_batch_tile_order(int total_tiles, const int32_t* tile_bins,
     const size_t sort_bytes = workspace_bytes - 6 * a;
     cudaStream_t st = (cudaStream_t)s;
     const int blocks = ceil_div(total_tiles, 256);
-    tile_group_keys_kernel<<<blocks, 256, 0, st>>>(total_tiles, (const int2*)tile_bins, tile_view,
+    launch_chained(tile_group_keys_kernel, blocks, 256, 0, st, total_tiles, (const int2*)tile_bins, tile_view,
                                                    (const BatchView*)views_dev, group, group_key, ids, cost_key);
     int rc = check_launch("batch_tile_order");
     if (rc) return rc;
@@ -573,7 +584,7 @@ extern "C" int gstex_batch_tile_order(int total_tiles, const int32_t* tile_bins,
     while (bits < 31 && (1u << bits) < (uint32_t)total_tiles) bits++;
     rc = gstex_sort_pairs32(total_tiles, nullptr, bits, group_key, ids, keys_sorted, by_group, sort_ws, sort_bytes, s);
     if (rc) return rc;
-    gather_keys_kernel<<<blocks, 256, 0, st>>>(total_tiles, by_group, cost_key, cost_in);
+    launch_chained(gather_keys_kernel, blocks, 256, 0, st, total_tiles, by_group, cost_key, cost_in);
     rc = check_launch("batch_tile_order");
     if (rc) return rc;
     return gstex_sort_pairs32(total_tiles, nullptr, 32, cost_in, by_group, keys_sorted, order, sort_ws, sort_bytes, s);
@@ -601,7 +612,8 @@ extern "C" int gstex_batch_emit_sorted(int N, int V, const void* views_dev, cons
     }
     GSTEX_REQUIRE(order && cum && rects && keys && vals && ((uintptr_t)rects & 7) == 0);
     const int VN = N * V;
-    batch_emit_sorted_kernel<<<ceil_div(VN, 256), 256, 0, stream>>>(VN, N, (const BatchView*)views_dev, order, cum,
+    launch_chained(batch_emit_sorted_kernel, ceil_div(VN, 256), 256, 0, stream,
+                   VN, N, (const BatchView*)views_dev, order, cum,
                                                                      (const uint2*)rects, total, capacity, keys, vals, count,
                                                                      overflow);
     return check_launch("batch_emit_sorted");
@@ -776,11 +788,11 @@ extern "C" int gstex_batch_sh_backward(int N, int V, const void* views_dev, cons
     const float4* vc = (const float4*)v_colors;
     cudaStream_t stream = (cudaStream_t)s;
     switch (sh_degree) {
-        case 0: batch_sh_backward_kernel<0><<<grid, block, 0, stream>>>(N, V, bv, m, vc, v_coeffs); break;
-        case 1: batch_sh_backward_kernel<1><<<grid, block, 0, stream>>>(N, V, bv, m, vc, v_coeffs); break;
-        case 2: batch_sh_backward_kernel<2><<<grid, block, 0, stream>>>(N, V, bv, m, vc, v_coeffs); break;
-        case 3: batch_sh_backward_kernel<3><<<grid, block, 0, stream>>>(N, V, bv, m, vc, v_coeffs); break;
-        default: batch_sh_backward_kernel<4><<<grid, block, 0, stream>>>(N, V, bv, m, vc, v_coeffs); break;
+        case 0: launch_chained(batch_sh_backward_kernel<0>, grid, block, 0, stream, N, V, bv, m, vc, v_coeffs); break;
+        case 1: launch_chained(batch_sh_backward_kernel<1>, grid, block, 0, stream, N, V, bv, m, vc, v_coeffs); break;
+        case 2: launch_chained(batch_sh_backward_kernel<2>, grid, block, 0, stream, N, V, bv, m, vc, v_coeffs); break;
+        case 3: launch_chained(batch_sh_backward_kernel<3>, grid, block, 0, stream, N, V, bv, m, vc, v_coeffs); break;
+        default: launch_chained(batch_sh_backward_kernel<4>, grid, block, 0, stream, N, V, bv, m, vc, v_coeffs); break;
     }
     return check_launch("batch_sh_backward");
 }
@@ -798,7 +810,8 @@ extern "C" int gstex_batch_image_loss(long long total_pixels, int V, const long 
     if (e != cudaSuccess) { set_cuda_error(e, "batch_image_loss"); return GSTEX_ERR_CUDA; }
     if (total_pixels == 0) return GSTEX_OK;
     const int blocks = (int)std::min<long long>(ceil_div((int)std::min<long long>(total_pixels, 1ll << 30), 256), 152 * 16);
-    batch_loss_kernel<<<blocks, 256, 0, stream>>>(total_pixels, V, pix_offsets, channels, (const float3*)img, tex,
+    launch_chained(batch_loss_kernel, blocks, 256, 0, stream,
+                   total_pixels, V, pix_offsets, channels, (const float3*)img, tex,
                                                   (const float3*)normal, reg, (const float3*)tgt_img, tgt_tex, w_img,
                                                   w_tex, w_reg, w_normal, (float3*)v_img, v_tex, (float3*)v_normal,
                                                   v_reg, loss);

@@ -71,6 +71,7 @@ constexpr int kEdgeItems = 4;
 template <typename K>
 __global__ void bin_edges_kernel(int n, const int64_t* __restrict__ n_dev, const K* __restrict__ sorted, int shift,
                                  int num_tiles, int2* __restrict__ bins) {
+    chain_wait();
     if (n_dev) {
         const int64_t m = *n_dev;
         n = (int)(m < (int64_t)n ? (m > 0 ? m : 0) : n);
@@ -160,6 +161,7 @@ __global__ void __launch_bounds__(kSortThreads) radix_hist_kernel(const K* __res
                                                                   int by_block = 0) {
     __shared__ uint32_t h[kSortWarps][kRadix];
     for (int i = threadIdx.x; i < kSortWarps * kRadix; i += blockDim.x) (&h[0][0])[i] = 0;
+    chain_wait();
     resolve_count(n_dev, n, chunk);
     __syncthreads();
     const int start = blockIdx.x * chunk;
@@ -225,6 +227,7 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* w
 // digit; the row total goes to totals[digit].
 __global__ void __launch_bounds__(kSortThreads) radix_scan_rows_kernel(uint32_t* __restrict__ hist, int blocks,
                                                                        uint32_t* __restrict__ totals) {
+    chain_wait();
     __shared__ uint32_t wsum[kSortWarps];
     uint32_t* row = hist + (size_t)blockIdx.x * blocks;
     uint32_t carry = 0;
@@ -287,6 +290,7 @@ __global__ void __launch_bounds__(kSortThreads, 4) radix_scatter_kernel(
     uint32_t* __restrict__ vout, int n, int chunk, const int64_t* __restrict__ n_dev, int shift, int dbits,
     const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ totals, uint32_t* __restrict__ next = nullptr,
     uint32_t next_mask = 0u) {
+    chain_wait();
     __shared__ uint32_t run_off[kRadix];
     __shared__ uint32_t tile_base[kRadix];
     __shared__ uint32_t wsum[kSortWarps];
@@ -411,6 +415,7 @@ __global__ void __launch_bounds__(kSortThreads, 4) radix_scatter_kernel(
 // ---------------------------------------------------------------------------
 __global__ void depth_keys_kernel(int n, const float* __restrict__ depths, const int32_t* __restrict__ counts,
                                   uint32_t* __restrict__ keys, int32_t* __restrict__ ids, int64_t* __restrict__ info) {
+    chain_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint32_t k = __float_as_uint(depths[i]);
@@ -464,6 +469,7 @@ __global__ void __launch_bounds__(256) view_emit_kernel(int n, int num_isect, in
                                                         const int32_t* __restrict__ cum, int tiles_x, int tiles_y,
                                                         int bw, uint32_t* __restrict__ keys,
                                                         int32_t* __restrict__ vals) {
+    chain_wait();
     const unsigned lane = threadIdx.x & 31;
     const long long first = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * slots;
     if (first >= num_isect) return;
@@ -714,6 +720,7 @@ __global__ void __launch_bounds__(kSmallThreads) view_bins_small_kernel(
 __global__ void __launch_bounds__(kSmallThreads) tile_order_small_kernel(int n, const int4* __restrict__ groups,
                                                                          const int2* __restrict__ bins,
                                                                          int32_t* __restrict__ order) {
+    chain_wait();
     extern __shared__ __align__(16) unsigned char smem[];
     SmallSort& S = *reinterpret_cast<SmallSort*>(smem);
     for (int i = threadIdx.x; i < n; i += kSmallThreads) {
@@ -764,22 +771,20 @@ extern "C" int gstex_map_gaussian_to_intersects(int n, int num_isect, const floa
     return check_launch("map_gaussian_to_intersects");
 }
 
-// 32-bit sorts of at most this many tiles take one launch a pass (DIRECT)
-// instead of three.  Every block reads the counts of all blocks, so the gain
-// shrinks with their number: 32 bits of 100k items 66 -> 46 us, 240k 66 -> 52,
-// 390k 66 -> 55, 500k (163 tiles) 74 -> 72, 780k (254) 74 -> 80.  A count on the
-// device is often a third of the capacity that the host knows, so the line lies
-// higher there.
-constexpr int kDirectBlocks = 192, kDirectBlocksDyn = 384;
+// 32-bit sorts of at most one tile per multiprocessor take one launch a pass
+// (DIRECT) instead of three.  Every block reads the counts of all blocks, so the
+// gain shrinks with their number: 32 bits of 100k items 64 -> 32 us, 240k 65 ->
+// 37, 390k (127 tiles) 66 -> 42, but 500k (163) 49 -> 57.
+constexpr int kDirectBlocks = 152;
 
-static bool sort_direct(const SortPlan& p, size_t key_bytes, bool dyn) {
-    return key_bytes == 4 && p.chunk == kSortTile && p.blocks <= (dyn ? kDirectBlocksDyn : kDirectBlocks);
+static bool sort_direct(const SortPlan& p, size_t key_bytes) {
+    return key_bytes == 4 && p.chunk == kSortTile && p.blocks <= kDirectBlocks;
 }
 
 static size_t sort_workspace_bytes(int n, size_t key_bytes) {
     if (n < 1) n = 1;
     const SortPlan p = sort_plan(n);
-    const size_t counts = sort_direct(p, key_bytes, true) ? 4 : 1;  // of each pass, or of one
+    const size_t counts = sort_direct(p, key_bytes) ? 4 : 1;  // of each pass, or of one
     return align_up((size_t)n * key_bytes, 256) + align_up((size_t)n * 4, 256) + counts * kRadix * p.blocks * 4 +
            (size_t)kRadix * 4;
 }
@@ -814,10 +819,10 @@ static int sort_impl(int n, const int64_t* n_dev, int end_bit, const K* keys_in,
     // Ping-pong so that the last pass lands in the output buffers.
     const K* ksrc = keys_in;
     const uint32_t* vsrc = (const uint32_t*)vals_in;
-    const bool direct = sort_direct(p, sizeof(K), n_dev != nullptr);
+    const bool direct = sort_direct(p, sizeof(K));
     const size_t row = (size_t)kRadix * p.blocks;  // counts of one pass
     if (direct) {
-        radix_hist_kernel<K><<<p.blocks, kSortThreads, 0, stream>>>(ksrc, n, p.chunk, n_dev, 0,
+        launch_chained(radix_hist_kernel<K>, p.blocks, kSortThreads, 0, stream, ksrc, n, p.chunk, n_dev, 0,
                                                                     (1u << std::min(digit, end_bit)) - 1u, hist, passes);
     }
     for (int pass = 0; pass < passes; pass++) {
@@ -834,7 +839,8 @@ static int sort_impl(int n, const int64_t* n_dev, int end_bit, const K* keys_in,
                              : dbits == 7 ? radix_scatter_kernel<K, 7, true> : radix_scatter_kernel<K, 8, true>;
                 cudaError_t e = cudaFuncSetAttribute(scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
                 if (e != cudaSuccess) { set_cuda_error(e, "sort_pairs"); return GSTEX_ERR_CUDA; }
-                scatter<<<p.blocks, kSortThreads, smem, stream>>>(ksrc, vsrc, kdst, vdst, n, p.chunk, n_dev, shift, dbits,
+                launch_chained(scatter, p.blocks, kSortThreads, smem, stream,
+                               ksrc, vsrc, kdst, vdst, n, p.chunk, n_dev, shift, dbits,
                                                                   hist + pass * row, nullptr,
                                                                   left > 0 ? hist + (pass + 1) * row : nullptr, next_mask);
             }
@@ -842,14 +848,16 @@ static int sort_impl(int n, const int64_t* n_dev, int end_bit, const K* keys_in,
             vsrc = vdst;
             continue;
         }
-        radix_hist_kernel<K><<<p.blocks, kSortThreads, 0, stream>>>(ksrc, n, p.chunk, n_dev, shift, (1u << dbits) - 1u,
-                                                                    hist);
-        radix_scan_rows_kernel<<<kRadix, kSortThreads, 0, stream>>>(hist, p.blocks, totals);
+        launch_chained(radix_hist_kernel<K>, p.blocks, kSortThreads, 0, stream,
+                       ksrc, n, p.chunk, n_dev, shift, (1u << dbits) - 1u,
+                                                                    hist, 0);
+        launch_chained(radix_scan_rows_kernel, kRadix, kSortThreads, 0, stream, hist, p.blocks, totals);
         auto scatter = dbits <= 5 ? radix_scatter_kernel<K, 5> : dbits == 6 ? radix_scatter_kernel<K, 6>
                      : dbits == 7 ? radix_scatter_kernel<K, 7> : radix_scatter_kernel<K, 8>;
         cudaError_t e = cudaFuncSetAttribute(scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) { set_cuda_error(e, "sort_pairs"); return GSTEX_ERR_CUDA; }
-        scatter<<<p.blocks, kSortThreads, smem, stream>>>(ksrc, vsrc, kdst, vdst, n, p.chunk, n_dev, shift, dbits,
+        launch_chained(scatter, p.blocks, kSortThreads, smem, stream,
+                       ksrc, vsrc, kdst, vdst, n, p.chunk, n_dev, shift, dbits,
                                                           hist, totals, nullptr, 0u);
         ksrc = kdst;
         vsrc = vdst;
@@ -886,7 +894,8 @@ extern "C" int gstex_get_tile_bin_edges(int num_isect, const int64_t* sorted, in
     if (e != cudaSuccess) { set_cuda_error(e, "tile_bin_edges memset"); return GSTEX_ERR_CUDA; }
     if (num_isect == 0) return GSTEX_OK;
     GSTEX_REQUIRE(sorted);
-    bin_edges_kernel<int64_t><<<ceil_div(num_isect, 256 * kEdgeItems), 256, 0, stream>>>(num_isect, nullptr, sorted, 32,
+    launch_chained(bin_edges_kernel<int64_t>, ceil_div(num_isect, 256 * kEdgeItems), 256, 0, stream,
+                   num_isect, nullptr, sorted, 32,
                                                                              num_tiles, (int2*)bins);
     return check_launch("get_tile_bin_edges");
 }
@@ -899,7 +908,8 @@ extern "C" int gstex_get_tile_bin_edges_dyn(int capacity, const int64_t* count, 
     if (e != cudaSuccess) { set_cuda_error(e, "tile_bin_edges memset"); return GSTEX_ERR_CUDA; }
     if (capacity == 0) return GSTEX_OK;
     GSTEX_REQUIRE(sorted);
-    bin_edges_kernel<int64_t><<<ceil_div(capacity, 256 * kEdgeItems), 256, 0, stream>>>(capacity, count, sorted, 32, num_tiles,
+    launch_chained(bin_edges_kernel<int64_t>, ceil_div(capacity, 256 * kEdgeItems), 256, 0, stream,
+                   capacity, count, sorted, 32, num_tiles,
                                                                             (int2*)bins);
     return check_launch("get_tile_bin_edges_dyn");
 }
@@ -912,7 +922,8 @@ extern "C" int gstex_get_tile_bin_edges32_dyn(int capacity, const int64_t* count
     if (e != cudaSuccess) { set_cuda_error(e, "tile_bin_edges32 memset"); return GSTEX_ERR_CUDA; }
     if (capacity == 0) return GSTEX_OK;
     GSTEX_REQUIRE(sorted);
-    bin_edges_kernel<uint32_t><<<ceil_div(capacity, 256 * kEdgeItems), 256, 0, stream>>>(capacity, count, sorted, shift, num_tiles,
+    launch_chained(bin_edges_kernel<uint32_t>, ceil_div(capacity, 256 * kEdgeItems), 256, 0, stream,
+                   capacity, count, sorted, shift, num_tiles,
                                                                              (int2*)bins);
     return check_launch("get_tile_bin_edges32_dyn");
 }
@@ -948,7 +959,7 @@ extern "C" int gstex_view_order(int n, const float* depths, const int32_t* count
     int32_t* ids = (int32_t*)(w + a);
     uint32_t* sorted = (uint32_t*)(w + 2 * a);
     int32_t* scounts = (int32_t*)(w + 3 * a);
-    depth_keys_kernel<<<ceil_div(n, 256), 256, 0, stream>>>(n, depths, counts, keys, ids, info);
+    launch_chained(depth_keys_kernel, ceil_div(n, 256), 256, 0, stream, n, depths, counts, keys, ids, info);
     int rc = check_launch("view_order");
     if (rc) return rc;
     rc = gstex_sort_pairs32(n, nullptr, 32, keys, ids, sorted, order, w + 4 * a, sb, s);
@@ -996,7 +1007,7 @@ extern "C" int gstex_view_bins(int n, int num_isect, const float* centers, const
     uint32_t* sorted = (uint32_t*)(w + 2 * a);
     const int slots = num_isect >= kEmitSlots * kEmitWarps ? kEmitSlots : (num_isect / kEmitWarps / 32 + 1) * 32;
     const int warps = (int)(((long long)num_isect + slots - 1) / slots);
-    view_emit_kernel<<<ceil_div(warps, 8), 256, 0, stream>>>(n, num_isect, slots, (const float2*)centers,
+    launch_chained(view_emit_kernel, ceil_div(warps, 8), 256, 0, stream, n, num_isect, slots, (const float2*)centers,
                                                              (const float2*)extents, depths, order, cum, tiles_x,
                                                              tiles_y, bw, keys, vals);
     int rc = check_launch("view_bins");
@@ -1004,7 +1015,8 @@ extern "C" int gstex_view_bins(int n, int num_isect, const float* centers, const
     rc = sort_impl<uint32_t>(num_isect, nullptr, end_bit, keys, vals, sorted, gids, w + 3 * a,
                              sort_workspace_bytes(num_isect, 4), stream);
     if (rc) return rc;
-    bin_edges_kernel<uint32_t><<<ceil_div(num_isect, 256 * kEdgeItems), 256, 0, stream>>>(num_isect, nullptr, sorted, 1,
+    launch_chained(bin_edges_kernel<uint32_t>, ceil_div(num_isect, 256 * kEdgeItems), 256, 0, stream,
+                   num_isect, nullptr, sorted, 1,
                                                                                           num_tiles, (int2*)bins);
     return check_launch("view_bins");
 }
@@ -1018,7 +1030,7 @@ extern "C" int gstex_batch_tile_order_small(int num_groups, const int32_t* group
     cudaError_t e = cudaFuncSetAttribute(tile_order_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)sizeof(SmallSort));
     if (e != cudaSuccess) { set_cuda_error(e, "batch_tile_order"); return GSTEX_ERR_CUDA; }
-    tile_order_small_kernel<<<1, kSmallThreads, sizeof(SmallSort), (cudaStream_t)s>>>(
+    launch_chained(tile_order_small_kernel, 1, kSmallThreads, sizeof(SmallSort), (cudaStream_t)s, 
         num_groups, (const int4*)groups, (const int2*)tile_bins, order);
     return check_launch("batch_tile_order");
 }

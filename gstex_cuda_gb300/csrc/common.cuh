@@ -2,6 +2,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <utility>
 #include <cuda_bf16.h>
 #include <stdint.h>
 
@@ -608,6 +609,32 @@ __device__ __forceinline__ Bilerp bilerp(int h, int w, int start, float u, float
         else B.w11 = 1.f;
     }
     return B;
+}
+
+// A chain of short kernels: launch_chained lets a kernel be set up while the one
+// before it in the stream still runs; chain_wait, before it reads or writes
+// anything that kernel may touch, waits for its end (and that of all before it).
+// Then the next one of the chain may be set up in turn.  Binning of four small
+// views (17 launches) 157 -> 138 us, of eight large ones 422 -> 382; a 32-bit
+// sort of 100k items 46 -> 32, of 780k 74 -> 50.  Not for the compositor: blocks
+// set up around those of the kernel before are spread unevenly over the
+// multiprocessors (forward of a 720p view 354 -> 388 us).
+__device__ __forceinline__ void chain_wait() {
+    asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");
+}
+template <typename... P, typename... A>
+inline void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);  // (errors: check_launch)
 }
 
 }  // namespace gstex

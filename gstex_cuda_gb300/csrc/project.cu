@@ -94,6 +94,7 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int* warp_sums, int& 
 // order: sums in[order[i]] and keeps these in `picked`.
 __global__ void scan_block_sums(int n, const int32_t* __restrict__ in, const int32_t* __restrict__ order,
                                 int32_t* __restrict__ picked, int64_t* __restrict__ sums) {
+    chain_wait();
     __shared__ int ws[32];
     const int base = blockIdx.x * kScanTile;
     int s = 0;
@@ -113,6 +114,7 @@ __global__ void scan_block_sums(int n, const int32_t* __restrict__ in, const int
 
 // single block: exclusive scan of the block sums (64-bit to detect overflow)
 __global__ void scan_sums(int nb, int64_t* __restrict__ sums, int64_t* __restrict__ total) {
+    chain_wait();
     __shared__ long long carry;
     if (threadIdx.x == 0) carry = 0;
     __syncthreads();
@@ -141,6 +143,7 @@ __global__ void scan_sums(int nb, int64_t* __restrict__ sums, int64_t* __restric
 // and each block adds up those before it.
 __global__ void scan_apply(int n, const int32_t* __restrict__ in, const int64_t* __restrict__ offsets,
                            int64_t* __restrict__ total_out, int32_t* __restrict__ out) {
+    chain_wait();
     __shared__ int ws[32];
     __shared__ long long before[kScanThreads / 32];
     long long offset = 0;
@@ -345,9 +348,9 @@ extern "C" size_t gstex_scan_workspace_bytes(int n) {
     return (size_t)(ceil_div(n > 0 ? n : 1, kScanTile) + 1) * sizeof(int64_t);
 }
 
-// Up to one block per thread of a block (2M counts) two launches do: for 100k to
-// 800k counts 16 to 22 us with the third and a launch that gathers, 8 to 12 us
-// without.
+// Up to one block per thread of a block (2M counts) two launches do: with the
+// third and one that gathers, 21 instead of 11 us for 32k to 100k counts and 33
+// instead of 22 us for 800k.
 static int inclusive_scan(int n, const int32_t* counts, const int32_t* order, int32_t* picked, int32_t* cum,
                           int64_t* total, void* ws, size_t ws_bytes, cudaStream_t stream) {
     if (n == 0) {
@@ -360,9 +363,10 @@ static int inclusive_scan(int n, const int32_t* counts, const int32_t* order, in
     const int nb = ceil_div(n, kScanTile);
     const bool two = nb <= kScanThreads;
     int64_t* sums = (int64_t*)ws;
-    scan_block_sums<<<nb, kScanThreads, 0, stream>>>(n, counts, order, picked, sums);
-    if (!two) scan_sums<<<1, 1024, 0, stream>>>(nb, sums, total);
-    scan_apply<<<nb, kScanThreads, 0, stream>>>(n, order ? picked : counts, sums, two ? total : nullptr, cum);
+    launch_chained(scan_block_sums, nb, kScanThreads, 0, stream, n, counts, order, picked, sums);
+    if (!two) launch_chained(scan_sums, 1, 1024, 0, stream, nb, sums, total);
+    launch_chained(scan_apply, nb, kScanThreads, 0, stream,
+                   n, order ? picked : counts, sums, two ? total : nullptr, cum);
     return check_launch("inclusive_scan", two ? 2 : 3);
 }
 

@@ -1047,6 +1047,7 @@ __device__ __forceinline__ void copy_out_records(const RecAll* __restrict__ src,
 __global__ void __launch_bounds__(128) records_kernel(SceneArgs a, BatchArgs ba, int num_views,
                                                       const int32_t* __restrict__ counts, RecAll* __restrict__ recs,
                                                       int* __restrict__ fix_count, uint32_t* __restrict__ fix) {
+    chain_wait();
     __shared__ RecAll srec[128];
     const int v = blockIdx.x % num_views;
     const int i0 = (blockIdx.x / num_views) * 128;
@@ -1091,6 +1092,7 @@ __device__ __forceinline__ void fix_record(const SceneArgs& a, const View& V, in
 // The double solve of the deferred near-edge-on records, densely.
 __global__ void records_fixup_kernel(SceneArgs a, BatchArgs ba, const int* __restrict__ fix_count,
                                      const uint32_t* __restrict__ fix, RecAll* __restrict__ recs) {
+    chain_wait();
     const int n = *fix_count;
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
         const uint32_t j = fix[t];
@@ -1104,6 +1106,7 @@ __global__ void records_fixup_kernel(SceneArgs a, BatchArgs ba, const int* __res
 // Gaussian of one view, so that any Gaussian a tile names has one.
 __global__ void __launch_bounds__(128) view_records_kernel(SceneArgs a, ViewArgs va, RecAll* __restrict__ recs,
                                                            int* __restrict__ fix_count, uint32_t* __restrict__ fix) {
+    chain_wait();
     __shared__ RecAll srec[128];
     const int i0 = blockIdx.x * 128;
     const int i = i0 + threadIdx.x;
@@ -1128,6 +1131,7 @@ __global__ void __launch_bounds__(128) view_records_kernel(SceneArgs a, ViewArgs
 
 __global__ void view_records_fixup_kernel(SceneArgs a, ViewArgs va, const int* __restrict__ fix_count,
                                           const uint32_t* __restrict__ fix, RecAll* __restrict__ recs) {
+    chain_wait();
     const int n = *fix_count;
     if (blockIdx.x * blockDim.x >= n) return;
     const View V = load_view(va.viewmat, va.fx, va.fy, va.cx, va.cy);
@@ -1144,8 +1148,8 @@ int launch_records(const SceneArgs& a, const BatchArgs& ba, int num_views, const
     if (e != cudaSuccess) { set_cuda_error(e, "batch_records"); return GSTEX_ERR_CUDA; }
     const long long blocks = (long long)ceil_div(a.N, 128) * num_views;
     if (blocks > 0x7fffffffLL) return GSTEX_ERR_UNSUPPORTED;
-    records_kernel<<<(unsigned)blocks, 128, 0, stream>>>(a, ba, num_views, counts, recs, fix_count, fix);
-    records_fixup_kernel<<<152 * 4, 128, 0, stream>>>(a, ba, fix_count, fix, recs);
+    launch_chained(records_kernel, (unsigned)blocks, 128, 0, stream, a, ba, num_views, counts, recs, fix_count, fix);
+    launch_chained(records_fixup_kernel, 152 * 4, 128, 0, stream, a, ba, fix_count, fix, recs);
     return check_launch("batch_records", 2);
 }
 
@@ -1162,6 +1166,7 @@ __global__ void finalize_kernel(int N, const float* __restrict__ mom, const floa
                                 const float4* __restrict__ quats, const float3* __restrict__ umap, const float3* __restrict__ vmap, float* v_opac,
                                 float3* v_means, float3* v_scales, float4* v_quats, float2* v_uv0, float3* v_umap,
                                 float3* v_vmap, RawGradArgs rg) {
+    chain_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N) return;
     float R[kMomStride];
@@ -1348,7 +1353,8 @@ int launch_finalize(const SceneArgs& a, const float* moments, float* v_opac, flo
                     float* v_quats, float* v_uv0, float* v_umap, float* v_vmap, cudaStream_t stream,
                     const RawGradArgs& rg) {
     if (a.N == 0) return GSTEX_OK;
-    finalize_kernel<<<ceil_div(a.N, 256), 256, 0, stream>>>(a.N, moments, a.scales, a.glob, a.quats, a.umap, a.vmap, v_opac,
+    launch_chained(finalize_kernel, ceil_div(a.N, 256), 256, 0, stream,
+                   a.N, moments, a.scales, a.glob, a.quats, a.umap, a.vmap, v_opac,
                                                            (float3*)v_means, (float3*)v_scales, (float4*)v_quats,
                                                            (float2*)v_uv0, (float3*)v_umap, (float3*)v_vmap, rg);
     return check_launch("finalize");
@@ -1518,8 +1524,8 @@ extern "C" int gstex_view_records(const gstex_raster_inputs* in, void* records, 
     cudaStream_t stream = (cudaStream_t)s;
     cudaError_t e = cudaMemsetAsync(fix_count, 0, sizeof(int), stream);
     if (e != cudaSuccess) { set_cuda_error(e, "view_records"); return GSTEX_ERR_CUDA; }
-    view_records_kernel<<<ceil_div(a.N, 128), 128, 0, stream>>>(a, va, recs, fix_count, fix);
-    view_records_fixup_kernel<<<152 * 2, 128, 0, stream>>>(a, va, fix_count, fix, recs);
+    launch_chained(view_records_kernel, ceil_div(a.N, 128), 128, 0, stream, a, va, recs, fix_count, fix);
+    launch_chained(view_records_fixup_kernel, 152 * 2, 128, 0, stream, a, va, fix_count, fix, recs);
     return check_launch("view_records", 2);
 }
 

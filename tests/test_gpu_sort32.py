@@ -1,6 +1,5 @@
 """gstex_sort_pairs32: stable order at the edges of a sort tile (3072 items), of
-the sorts with one launch a pass (192 tiles, or 384 where the count is on the
-device) and of the digit widths."""
+the sorts with one launch a pass (152 tiles) and of the digit widths."""
 import pytest
 import torch
 
@@ -39,18 +38,18 @@ def _check(n, bits, count=None, few=False):
         assert bool((vo[m:] == -1).all()) and bool((ko[m:] == -1).all())
 
 
-@pytest.mark.parametrize("n", [2, 33, TILE - 1, TILE, TILE + 1, 191 * TILE + 1, 192 * TILE, 192 * TILE + 1])
+@pytest.mark.parametrize("n", [2, 33, TILE - 1, TILE, TILE + 1, 151 * TILE + 1, 152 * TILE, 152 * TILE + 1])
 @pytest.mark.parametrize("bits", [1, 8, 9, 13, 32])
 def test_known_count(n, bits):
     _check(n, bits)
 
 
-@pytest.mark.parametrize("n", [TILE, 100000, 192 * TILE])
+@pytest.mark.parametrize("n", [TILE, 100000, 152 * TILE])
 def test_few_values(n):
     _check(n, 32, few=True)
 
 
-@pytest.mark.parametrize("cap", [2 * TILE, 384 * TILE, 384 * TILE + 1])
+@pytest.mark.parametrize("cap", [2 * TILE, 152 * TILE, 152 * TILE + 1])
 @pytest.mark.parametrize("count", [0, 1, TILE, TILE + 1, None])
 def test_count_on_device(cap, count):
     _check(cap, 13, cap if count is None else count)
