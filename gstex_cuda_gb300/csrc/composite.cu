@@ -16,11 +16,12 @@
 //   3. walk: every lane goes through its own set in order.  The lanes of one
 //      step are usually at different splats.
 //
-// What bounds it: the L1 data path (77% of its cycles at 24 warps per SM; half
-// of it staged records, half texel gathers), then the ALUs (47%).  Measured
+// What bounds it: the L1 data path (73% of its cycles at 24 warps per SM, 78% with
+// float32 texels; half of it staged records, a third to a half texel gathers),
+// then the ALUs (49%).  Measured
 // against the list walk with one CTA per tile (forward kernel alone): 32 views
-// with 81M intersections, bf16 texels, 8x8 tiles 17.4 -> 8.9 ms; 8 clustered
-// full-HD views 9.2 -> 5.3 ms; one 800x800 view, 16x16 tiles 232 -> 62 us; one
+// with 81M intersections, bf16 texels, 8x8 tiles 17.4 -> 8.7 ms; 8 clustered
+// full-HD views 9.2 -> 5.2 ms; one 800x800 view, 16x16 tiles 232 -> 59 us; one
 // full-HD view of large splats 5.1 -> 2.2 ms.  About 16 of 32 lanes blend in a
 // step, against 3 to 7 before.
 //
@@ -545,34 +546,37 @@ __global__ void __launch_bounds__(32 * kBlockWarps, kFwdCtas)
 // Backward.  The walk is the forward's, back to front; a splat's gradients are
 // sums over pixels (finalize_kernel turns 21 of them into the parameters'
 // gradients), and the pixels of a step are at different splats.  So every lane
-// first steps back over up to kRounds of its pixel's pairs and leaves eight
-// numbers per pair in shared memory; then the roles turn (one more transpose):
+// first steps back over its pixel's pairs with as many staged splats as there
+// is room for (kPairs) and leaves eight numbers per pair in shared memory; then the roles turn (one more transpose):
 // every lane takes a splat and sums the pairs of its pixels in registers,
 // without the shuffles and shared-memory atomics of a reduction over the warp,
 // and adds the sums to the splat's row with 16-byte atomics.
 //
-// What bounds it: the L1 data path (71% of its cycles; a 16-byte reduction
+// What bounds it: the L1 data path (75% of its cycles; a 16-byte reduction
 // takes about a cycle per lane there) and the latency of its chains at 16 warps
-// per SM.  Of 22.5 ms on 32 views (36.6 ms with the list walk, its moment
+// per SM.  Of 22.1 ms on 32 views (36.6 ms with the list walk, its moment
 // reduction by shuffles and 8-lane groups) the scan, staging and ray-plane
 // solves take 6 ms, the adjoint 4, texel reads 3.5, texel atomics 4 and the
-// sums 5.  8 clustered full-HD views: 22.3 -> 13.5 ms; one 800x800 view of 1x1
-// charts 254 -> 111 us; one full-HD view of large splats 36.0 -> 8.4 ms (where
-// the list walk also staged every splat behind the last contributor).
+// sums 5.  8 clustered full-HD views: 22.3 -> 13.2 ms; one 800x800 view of 1x1
+// charts 254 -> 108 us; one full-HD view of large splats 36.0 -> 6.9 ms (where
+// the list walk also staged every splat behind the last contributor).  The
+// pixels' upstream gradients by shuffles instead of from shared memory in the
+// sums: 23.7 ms.
 // ---------------------------------------------------------------------------
 constexpr int kBwdChunks = 8;
 // Pairs between two summations, and CTAs per SM (at most 128 registers): what
 // fits 8 CTAs' shared memory (32 staged splats have 230 pairs on average; with
-// 192, 1% slower).  Pairs are placed splat by splat, so the room is used up and
-// a splat is summed once: 7 rounds of one pair per pixel in the same room took
-// 23.6 instead of 22.8 ms on 32 views, 14.4 instead of 13.7 ms on 8 clustered
-// ones.
-constexpr int kPairs = 212;
+// 192, 1% slower; with 224, which fit 7 CTAs, 23.5 instead of 22.1 ms).  Pairs
+// are placed splat by splat, so the room is used up and a splat is summed once:
+// 7 rounds of one pair per pixel in the same room took 23.6 instead of 22.8 ms
+// on 32 views, 14.4 instead of 13.7 ms on 8 clustered ones.
+constexpr int kPairs = 220;
 constexpr int kBwdCtas = 8;
 struct BwdMem {
     Staged<kBwdChunks> rec;
     float4 pair[2][kPairs];       // (vis, e v_alpha, v_sigma, v_t / (n . r)), (v_u, v_v, l1s, l2s), splat by splat
-    float4 pix[3][32];            // upstream colour, normal and texture gradients of the pixels (w: centre x, y)
+    float4 pix[2][32];            // the pixels' upstream colour and normal x; texture gradients
+    float2 pix_n[32];             // normal y, z
     uint2 place[32];              // first pair of a staged splat; its pixels that may have one
     uint8_t slot[32];             // splats with pairs
     Queue q;
@@ -735,7 +739,8 @@ __device__ __forceinline__ void pair_adjoint(BwdState<CT>& S, const SceneArgs& a
 // lane's staged splat, whose pairs start at `first` in the order of `may`.
 template <int TM, int FIX>
 __device__ __forceinline__ void add_coarse_texel_grads(const BwdMem& M, const SceneArgs& a, float* __restrict__ v_texgrad,
-                                                       int k, unsigned own, unsigned may, int first) {
+                                                       int k, unsigned own, unsigned may, int first, float fx0,
+                                                       float fy0) {
     const StagedRec<kBwdChunks> rec(M.rec, k);
     const float4 nop = rec(kChunkNop), uvs = rec(kChunkUvs), uvm = rec(kChunkUvm);
     RecHot Hr;
@@ -761,10 +766,10 @@ __device__ __forceinline__ void add_coarse_texel_grads(const BwdMem& M, const Sc
     for (; own; own &= own - 1) {
         const int p = __ffs(own) - 1;
         const float vis = M.pair[0][first + __popc(may & ((1u << p) - 1u))].x;
-        const float4 vt = M.pix[2][p];
+        const float4 vt = M.pix[1][p];
         PixelRay P;
-        P.px = M.pix[0][p].w;
-        P.py = M.pix[1][p].w;
+        P.px = fx0 + (float)lane_col(p);
+        P.py = fy0 + (float)lane_row(p);
         P.dn = 0.f;
         const Hit H = intersect(Hr, P);
         const float2 t = fma2(make_float2(uvm.y, uvm.w), dup2(H.dv), mul2(make_float2(uvm.x, uvm.z), dup2(H.du)));
@@ -849,9 +854,9 @@ __global__ void __launch_bounds__(32 * kBlockWarps, kBwdCtas)
 #pragma unroll
     for (int c = 0; c < (CT > 0 ? CT : 1); c++) S.vtex[c] = (CT > 0 && inside && g.v_tex) ? g.v_tex[pix * CT + c] : 0.f;
     S.vT_run = a.bg[0] * S.vout.x + a.bg[1] * S.vout.y + a.bg[2] * S.vout.z - valph;
-    M.pix[0][lane] = f4(S.vout, P.px);
-    M.pix[1][lane] = f4(S.vnorm, P.py);
-    if (CT == 3) M.pix[2][lane] = make_float4(S.vtex[0], S.vtex[CT > 1 ? 1 : 0], S.vtex[CT > 2 ? 2 : 0], 0.f);
+    M.pix[0][lane] = f4(S.vout, S.vnorm.x);
+    M.pix_n[lane] = make_float2(S.vnorm.y, S.vnorm.z);
+    if (CT == 3) M.pix[1][lane] = make_float4(S.vtex[0], S.vtex[CT > 1 ? 1 : 0], S.vtex[CT > 2 ? 2 : 0], 0.f);
     const float fx0 = (float)J.x0 + 0.5f, fy0 = (float)J.y0 + 0.5f;
     const unsigned live = __ballot_sync(kFull, S.bfin >= J.range.x), below = (1u << lane) - 1u;
     int n = 0;
@@ -931,7 +936,8 @@ __global__ void __launch_bounds__(32 * kBlockWarps, kBwdCtas)
                 const int p = __ffs(todo_p) - 1;
                 const int at = (int)pl.x - base + __popc(pl.y & ((1u << p) - 1u));
                 const float4 q0 = M.pair[0][at], q1 = M.pair[1][at];
-                const float4 vo = M.pix[0][p], vn = M.pix[1][p];
+                const float4 vo = M.pix[0][p];
+                const float2 vn = M.pix_n[p];
                 const float vis = q0.x, vtd = q0.w;
                 const float vsig = FIX ? q0.y : q0.z;  // (FIX: v_sigma = -opacity times this, applied below)
                 const float2 ls = make_float2(q1.z, q1.w);
@@ -948,9 +954,9 @@ __global__ void __launch_bounds__(32 * kBlockWarps, kBwdCtas)
                 m[9] += vtd;
                 t2 = fma2(ls, dup2(vtd), make_float2(m[10], m[11]));
                 m[10] = t2.x; m[11] = t2.y;
-                t2 = fma2(dup2(vis), make_float2(vn.x, vn.y), make_float2(m[12], m[13]));
-                m[12] = t2.x; m[13] = t2.y;
-                m[14] += vis * vn.z;
+                m[12] += vis * vo.w;
+                t2 = fma2(dup2(vis), vn, make_float2(m[13], m[14]));
+                m[13] = t2.x; m[14] = t2.y;
                 if (CT > 0) {
                     t2 = add2(make_float2(m[15], m[16]), make_float2(q1.x, q1.y));
                     m[15] = t2.x; m[16] = t2.y;
@@ -964,8 +970,8 @@ __global__ void __launch_bounds__(32 * kBlockWarps, kBwdCtas)
                     if (use_blur) {
                         const float4 c = __ldg(J.recs[M.q.gid[k]].c + kChunkMisc);
                         const float vsb = -nop.z * q0.y - q0.z;
-                        m[21] += kBlurFsq * vsb * (c.x - vo.w);
-                        m[22] += kBlurFsq * vsb * (c.y - vn.w);
+                        m[21] += kBlurFsq * vsb * (c.x - (fx0 + (float)lane_col(p)));
+                        m[22] += kBlurFsq * vsb * (c.y - (fy0 + (float)lane_row(p)));
                     }
                 }
             }
@@ -983,7 +989,7 @@ __global__ void __launch_bounds__(32 * kBlockWarps, kBwdCtas)
             }
             if (CT == 3) {
                 const unsigned coarse = is_coarse(nop) ? own : 0u;
-                if (coarse) add_coarse_texel_grads<TM, FIX>(M, a, g.v_texgrad, k, coarse, pl.y, (int)pl.x - base);
+                if (coarse) add_coarse_texel_grads<TM, FIX>(M, a, g.v_texgrad, k, coarse, pl.y, (int)pl.x - base, fx0, fy0);
             }
             __syncwarp();
             base = stop;
