@@ -411,7 +411,7 @@ __global__ void __launch_bounds__(kSortThreads, 4) radix_scatter_kernel(
 // the reference turns into tile -1, go to the tile behind the last.
 //
 // 158M intersections of 200k Gaussians (full HD): emission 3.1 -> 0.46 ms, sorts
-// and scans 6.6 -> 2.5 ms; a few thousand: one launch each instead of 18 to 25.
+// and scans 6.6 -> 2.0 ms; a few thousand: one launch each instead of 18 to 25.
 // ---------------------------------------------------------------------------
 __global__ void depth_keys_kernel(int n, const float* __restrict__ depths, const int32_t* __restrict__ counts,
                                   uint32_t* __restrict__ keys, int32_t* __restrict__ ids, int64_t* __restrict__ info) {
