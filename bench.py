@@ -220,21 +220,16 @@ def reference_kernels_leg(spec, dev, steps, warmup=1):
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one compositor
 # launch on the full workloads, from single-pass ncu captures of the launches
 # of one step (profiles/compositor_dram_traffic_full_workloads.txt gives the
-# commands and the raw figures).  Keyed by (workload, kernel, tile width), for
-# the kernels the autotuner picks at that width: 8x8 tiles, forward compiled
-# for the default settings with its queue in 4x4-tile groups and the 10-CTA
-# backward (8-lane groups on the 32-view scene; 32-lane walk and 48 Gaussians
-# per batch on the stress scene); 16x16 tiles, the general backward (8-lane
-# groups on the 32-view scene, 32-lane walk on the stress scene).
+# commands and the raw figures).  Keyed by (workload, kernel, tile width).
 DRAM_BYTES_PER_LAUNCH = {
-    ("batched", "forward", 8): 12_075_774_720 + 1_747_140_608,
-    ("batched", "backward", 8): 21_443_585_792 + 7_728_033_280,
-    ("batched", "forward", 16): 9_822_225_152 + 1_737_394_176,
-    ("batched", "backward", 16): 20_452_395_264 + 7_372_365_824,
-    ("stress", "forward", 8): 5_279_288_320 + 1_163_496_192,
-    ("stress", "backward", 8): 8_169_039_360 + 2_389_876_992,
-    ("stress", "forward", 16): 4_011_032_064 + 1_154_998_272,
-    ("stress", "backward", 16): 7_881_462_272 + 2_271_416_064,
+    ("batched", "forward", 8): 9_666_715_648 + 1_839_194_880,
+    ("batched", "backward", 8): 18_363_544_576 + 7_332_036_608,
+    ("batched", "forward", 16): 8_731_305_984 + 1_816_420_352,
+    ("batched", "backward", 16): 18_503_348_736 + 7_362_116_352,
+    ("stress", "forward", 8): 4_471_555_072 + 1_234_865_152,
+    ("stress", "backward", 8): 5_997_352_192 + 2_231_673_856,
+    ("stress", "forward", 16): 3_528_233_728 + 1_212_915_968,
+    ("stress", "backward", 16): 5_955_748_352 + 2_236_045_568,
 }
 DEFAULT_VIEWS = {"batched": 32, "stress": 8}
 TRAFFIC_SOURCE = "ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch of this workload"

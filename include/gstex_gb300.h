@@ -207,8 +207,10 @@ typedef struct gstex_raster_inputs {
     int pixels_per_thread;              /* 0 = default (1); 2 needs an even block width */
     /* Optional splat records of this view built by gstex_view_records from
      * the same inputs (16-byte aligned); NULL: every tile derives the records
-     * of its Gaussians itself.  Read by texture_forward / texture_backward,
-     * not by texture_edit. */
+     * of its Gaussians itself.  With records, a block width that is a multiple
+     * of 8, 0 or 3 channels and without alpha visualisation the compositor
+     * runs one warp per 8x4 pixels, to which pixels_per_thread and
+     * group_lanes do not apply. */
     const void* records;
     /* texture_backward: lanes that walk one list of staged splats, 32 (a
      * warp's 8x4 pixel block), 16 (4x4), 8 (4x2) or 4 (2x2); 0 = 32.  Values
@@ -433,7 +435,9 @@ typedef struct gstex_batch_inputs {
                                            null = each tile derives the records it stages */
     int group_lanes;                    /* backward: lanes per splat walk (see gstex_raster_inputs) */
     int batch_size;                     /* Gaussians a tile stages per round; 0, or at least the
-                                           threads of a CTA: one per thread (the reference's bw^2) */
+                                           threads of a CTA: one per thread (the reference's bw^2).
+                                           This, group_lanes, resident_ctas, pixels_per_thread and
+                                           grid are for the tile kernels (see gstex_raster_inputs) */
     int resident_ctas;                  /* backward, 8x8 tiles with bf16 RGB texels and 8-lane groups (or
                                            32 at the default settings): 10 selects a kernel compiled for
                                            10 CTAs per SM (96 registers per thread instead of 124); other
