@@ -87,3 +87,12 @@ def test_odd_depths_and_counts(n, what):
         assert got[0] == 0 and got[1].numel() == 0 and int(got[2].abs().sum()) == 0 and tuple(got[2].shape) == (104, 2)
         return
     _both(c, e, d, counts, 200, 120, 16)
+
+
+@pytest.mark.parametrize("n", [2 ** 18, 2 ** 18 + 1])
+@pytest.mark.parametrize("w,h", [(1024, 1024), (1024, 1008)])
+def test_key_and_id_in_one_word(n, w, h):
+    """18 or 19 bits of id beside 14 or 13 of tile: sorted as one word up to 32."""
+    import gstex_cuda_gb300 as G
+    c, e, d = _inputs(n, w, h, 12.0, n + h)
+    _both(c, e, d, G.get_aabb_2d.get_num_tiles_hit_2d(c, e, h, w, 16), w, h, 16)
