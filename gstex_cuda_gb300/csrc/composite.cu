@@ -631,8 +631,11 @@ __device__ __forceinline__ void add_texel_grads(float* __restrict__ v_texgrad, i
 #pragma unroll
     for (int q = 0; q < 4; q += 2) {
         const float w0 = wts[q], w1 = wts[q + 1];
-        const float2 a01 = mul2(dup2(w0), gv01), b01 = mul2(dup2(w1), gv01);
-        const float a2 = w0 * gv2, b2 = w1 * gv2;
+        // (a corner without weight adds 0 whatever the gradient: the word it shares
+        // may be another chart's texel, and 0 times infinity is not 0)
+        const float2 z = make_float2(0.f, 0.f);
+        const float2 a01 = w0 != 0.f ? mul2(dup2(w0), gv01) : z, b01 = w1 != 0.f ? mul2(dup2(w1), gv01) : z;
+        const float a2 = w0 != 0.f ? w0 * gv2 : 0.f, b2 = w1 != 0.f ? w1 * gv2 : 0.f;
         if (TM == 1) {
             if (w0 != 0.f) atomicAdd(reinterpret_cast<float4*>(v_texgrad) + rows[q], make_float4(a01.x, a01.y, a2, 0.f));
             if (w1 != 0.f)
