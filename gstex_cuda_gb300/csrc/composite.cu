@@ -703,8 +703,8 @@ __device__ __forceinline__ void pair_adjoint(BwdState<CT>& S, const SceneArgs& a
         }
         const float2 vs = mul2(val, vt);
         v_vis += vs.x + vs.y + val2 * S.vtex[2];
-        // (a coarse chart's are summed over the pixels first)
-        if (!is_coarse(nop)) add_texel_grads<TM>(g.v_texgrad, a.T, B, gv01, gv2);
+        // (a coarse chart's are summed over the pixels first, but for pairs in the direct form)
+        if (!is_coarse(nop) || H.direct) add_texel_grads<TM>(g.v_texgrad, a.T, B, gv01, gv2);
     }
     float v_alpha = T * v_vis - T * S.vT_run;
     float vT_cur = alpha * v_vis + (1.f - alpha) * S.vT_run;
@@ -739,7 +739,9 @@ __device__ __forceinline__ void pair_adjoint(BwdState<CT>& S, const SceneArgs& a
 // Texel gradients of a coarse chart (kCoarseChart): atomics of 32 lanes on the
 // same texel are served one after the other, so the lane sums a staged splat's pairs over
 // its pixels (own) as long as they fall between the same four texels.  k: the
-// lane's staged splat, whose pairs start at `first` in the order of `may`.
+// lane's staged splat, whose pairs start at `first` in the order of `may`.  Pairs
+// in the direct form are not among them: the fast form, which this takes again,
+// has no uv where the ray lies in the splat's plane (pair_adjoint adds theirs).
 template <int TM, int FIX>
 __device__ __forceinline__ void add_coarse_texel_grads(const BwdMem& M, const SceneArgs& a, float* __restrict__ v_texgrad,
                                                        int k, unsigned own, unsigned may, int first, float fx0,
@@ -896,7 +898,7 @@ __global__ void __launch_bounds__(32 * kBlockWarps, kBwdCtas)
             const int stop = __shfl_sync(kFull, last, 31 - __clz(fits));
             __syncwarp();
             // every lane steps back over its pixel's pairs
-            unsigned valid = 0;
+            unsigned valid = 0, direct = 0;
             for (unsigned bits = todo & fits; bits; bits &= bits - 1) {
                 const int k = __ffs(bits) - 1;
                 const StagedRec<kBwdChunks> rec(M.rec, k);
@@ -912,6 +914,7 @@ __global__ void __launch_bounds__(32 * kBlockWarps, kBwdCtas)
                 M.pair[0][at] = q0;
                 M.pair[1][at] = q1;
                 valid |= 1u << k;
+                if (CT == 3 && H.direct) direct |= 1u << k;
             }
             __syncwarp();
             // sum every splat's pairs over the pixels: one lane per splat, or
@@ -991,7 +994,8 @@ __global__ void __launch_bounds__(32 * kBlockWarps, kBwdCtas)
                 flush_moments<FIX>(m, ba, g, J, M.q.gid[k], use_blur);
             }
             if (CT == 3) {
-                const unsigned coarse = is_coarse(nop) ? own : 0u;
+                unsigned coarse = is_coarse(nop) ? own : 0u;
+                if (__any_sync(kFull, direct != 0u)) coarse &= ~__shfl_sync(kFull, transpose32(direct, lane), k);
                 if (coarse) add_coarse_texel_grads<TM, FIX>(M, a, g.v_texgrad, k, coarse, pl.y, (int)pl.x - base, fx0, fy0);
             }
             __syncwarp();
