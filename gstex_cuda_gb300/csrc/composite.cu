@@ -972,10 +972,12 @@ __global__ void __launch_bounds__(32 * kBlockWarps, kBwdCtas)
                     m[19] = t2.x; m[20] = t2.y;
                 }
                 if constexpr (!FIX) {
-                    // one of the two alphas is the pair's: v_sigma_blur = -opacity e v_alpha - v_sigma
+                    // one of the two alphas is the pair's.  The filter's has no v_sigma, and the
+                    // splat's no v_sigma_blur: as -opacity e v_alpha - v_sigma it would be the two
+                    // products' rounding, which a large splat's small gradients do not bear
                     if (use_blur) {
                         const float4 c = __ldg(J.recs[M.q.gid[k]].c + kChunkMisc);
-                        const float vsb = -nop.z * q0.y - q0.z;
+                        const float vsb = q0.z == 0.f ? -nop.z * q0.y : 0.f;
                         m[21] += kBlurFsq * vsb * (c.x - (fx0 + (float)lane_col(p)));
                         m[22] += kBlurFsq * vsb * (c.y - (fy0 + (float)lane_row(p)));
                     }
