@@ -36,12 +36,13 @@ __device__ __forceinline__ void fetch3(const void* tex, const Bilerp& B, float c
             c[q][2] = __low2float(hi);
         }
     } else {
-        const float* t = (const float*)tex;
+        // (3 times a row passes 31 bits from 716M texels on)
 #pragma unroll
         for (int q = 0; q < 4; q++) {
-            c[q][0] = __ldg(t + 3 * rows[q] + 0);
-            c[q][1] = __ldg(t + 3 * rows[q] + 1);
-            c[q][2] = __ldg(t + 3 * rows[q] + 2);
+            const float* t = (const float*)tex + 3 * (size_t)rows[q];
+            c[q][0] = __ldg(t + 0);
+            c[q][1] = __ldg(t + 1);
+            c[q][2] = __ldg(t + 2);
         }
     }
 }
