@@ -45,8 +45,8 @@ __global__ void __launch_bounds__(RowStage<1>::kRows) batch_project_kernel(int N
         activate(raw, i, sx, sy, q);
     } else {
         q = quats[i];
-        sx = scales[3 * i];
-        sy = scales[3 * i + 1];
+        sx = scales[3 * (size_t)i];
+        sy = scales[3 * (size_t)i + 1];
     }
     float k[B][3];
 #pragma unroll
@@ -106,7 +106,7 @@ __global__ void batch_emit_kernel(int N, int V, const BatchView* __restrict__ vi
     if (i >= N) return;
     const float3 p = means[i];
     const float4 q = quats[i];
-    const float sx = scales[3 * i], sy = scales[3 * i + 1];
+    const float sx = scales[3 * (size_t)i], sy = scales[3 * (size_t)i + 1];
     for (int v = 0; v < V; v++) {
         const BatchView& bv = views[v];
         const size_t j = (size_t)v * N + i;

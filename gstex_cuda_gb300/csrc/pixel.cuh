@@ -14,7 +14,7 @@ __device__ __forceinline__ void direct_hit(Hit& H, const float4* __restrict__ qu
                                            const View& V, int gid, const PixelRay& P, float tvn) {
     const Axes A = quat_axes(quats[gid]);
     const float3 mc = V.xform(means[gid]);
-    const float is1 = 1.f / (scales[3 * gid] * glob), is2 = 1.f / (scales[3 * gid + 1] * glob);
+    const float is1 = 1.f / (scales[3 * (size_t)gid] * glob), is2 = 1.f / (scales[3 * (size_t)gid + 1] * glob);
     const float2 uv0 = uv0s[gid];
     intersect_direct(H, P, tvn, mc, V.rot(A.a1), V.rot(A.a2), V.rot(A.a3), V.rot(umaps[gid]), V.rot(vmaps[gid]), is1,
                      is2, uv0.x, uv0.y);

@@ -26,9 +26,9 @@ __global__ void preprocess_bwd_kernel(int N, int P, const float* __restrict__ ra
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N) return;
     // exp: d scale / d raw = scale; the third scale is detached in the trainer
-    v_raw_scales[3 * i] = v_scales ? v_scales[3 * i] * expf(raw_scales[3 * i]) : 0.f;
-    v_raw_scales[3 * i + 1] = v_scales ? v_scales[3 * i + 1] * expf(raw_scales[3 * i + 1]) : 0.f;
-    v_raw_scales[3 * i + 2] = 0.f;
+    v_raw_scales[3 * (size_t)i] = v_scales ? v_scales[3 * (size_t)i] * expf(raw_scales[3 * (size_t)i]) : 0.f;
+    v_raw_scales[3 * (size_t)i + 1] = v_scales ? v_scales[3 * (size_t)i + 1] * expf(raw_scales[3 * (size_t)i + 1]) : 0.f;
+    v_raw_scales[3 * (size_t)i + 2] = 0.f;
     const float4 r = raw_quats[i];
     const float in = 1.f / sqrtf(r.x * r.x + r.y * r.y + r.z * r.z + r.w * r.w);
     const float4 q = make_float4(r.x * in, r.y * in, r.z * in, r.w * in);

@@ -36,11 +36,11 @@ __device__ __forceinline__ float sigmoidf(float x) { return 1.f / (1.f + expf(-x
 // Activates Gaussian i, writes its activated parameters and returns the two
 // scales and the unit quaternion.
 __device__ __forceinline__ void activate(const RawParams& r, int i, float& s0, float& s1, float4& q) {
-    s0 = expf(r.raw_scales[3 * i]);
-    s1 = expf(r.raw_scales[3 * i + 1]);
-    r.scales[3 * i] = s0;
-    r.scales[3 * i + 1] = s1;
-    r.scales[3 * i + 2] = 1e-5f * (0.5f * (s0 + s1));
+    s0 = expf(r.raw_scales[3 * (size_t)i]);
+    s1 = expf(r.raw_scales[3 * (size_t)i + 1]);
+    r.scales[3 * (size_t)i] = s0;
+    r.scales[3 * (size_t)i + 1] = s1;
+    r.scales[3 * (size_t)i + 2] = 1e-5f * (0.5f * (s0 + s1));
     const float4 w = r.raw_quats[i];
     const float in = 1.f / sqrtf(w.x * w.x + w.y * w.y + w.z * w.z + w.w * w.w);
     q = make_float4(w.x * in, w.y * in, w.z * in, w.w * in);

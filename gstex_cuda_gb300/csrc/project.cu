@@ -21,7 +21,7 @@ __global__ void aabb_kernel(int n, const float3* __restrict__ means, const float
     for (int k = 0; k < 12; k++) m[k] = viewmat[k];
     float2 c, e;
     float z;
-    aabb_2d(m, fx, fy, cx, cy, means[i], quats[i], scales[3 * i], scales[3 * i + 1], glob_scale, c, e, z);
+    aabb_2d(m, fx, fy, cx, cy, means[i], quats[i], scales[3 * (size_t)i], scales[3 * (size_t)i + 1], glob_scale, c, e, z);
     centers[i] = c;
     extents[i] = e;
 }
@@ -199,9 +199,9 @@ __global__ void sh_forward_kernel(int n, int degree, const float3* __restrict__ 
         c1 += Y[b] * k[3 * b + 1];
         c2 += Y[b] * k[3 * b + 2];
     }
-    colors[3 * i + 0] = c0;
-    colors[3 * i + 1] = c1;
-    colors[3 * i + 2] = c2;
+    colors[3 * (size_t)i] = c0;
+    colors[3 * (size_t)i + 1] = c1;
+    colors[3 * (size_t)i + 2] = c2;
 }
 
 template <int DTU>
@@ -213,7 +213,7 @@ __global__ void sh_backward_kernel(int n, int degree, const float3* __restrict__
     float Y[25];
     sh_basis(DTU, dirs[i], Y);
     const int B = sh_bases(degree);
-    const float v0 = v_colors[3 * i], v1 = v_colors[3 * i + 1], v2 = v_colors[3 * i + 2];
+    const float v0 = v_colors[3 * (size_t)i], v1 = v_colors[3 * (size_t)i + 1], v2 = v_colors[3 * (size_t)i + 2];
     float* o = v_coeffs + (size_t)i * B * 3;
 #pragma unroll
     for (int b = 0; b < NB; b++) {
@@ -250,9 +250,9 @@ __global__ void __launch_bounds__(RowStage<1>::kRows) sh_forward_rows_kernel(int
         c1 += Y[b] * k[3 * b + 1];
         c2 += Y[b] * k[3 * b + 2];
     }
-    colors[3 * i + 0] = c0;
-    colors[3 * i + 1] = c1;
-    colors[3 * i + 2] = c2;
+    colors[3 * (size_t)i] = c0;
+    colors[3 * (size_t)i + 1] = c1;
+    colors[3 * (size_t)i + 2] = c2;
 }
 
 template <int DTU>
@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(RowStage<1>::kRows) sh_backward_rows_kernel(in
     if (i < n) {
         float Y[25];
         sh_basis(DTU, dirs[i], Y);
-        const float v0 = v_colors[3 * i], v1 = v_colors[3 * i + 1], v2 = v_colors[3 * i + 2];
+        const float v0 = v_colors[3 * (size_t)i], v1 = v_colors[3 * (size_t)i + 1], v2 = v_colors[3 * (size_t)i + 2];
         float* o = rows.row();
 #pragma unroll
         for (int b = 0; b < NB; b++) {

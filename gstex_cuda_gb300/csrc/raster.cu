@@ -27,7 +27,7 @@ namespace gstex {
 __device__ __forceinline__ void stage(const Recs& R, int slot, const SceneArgs& a, const View& V, const float3* colors,
                                       int gid, bool use_blur) {
     make_record(R.hot[slot], R.warm[slot], R.cold[slot], gid, V, a.means[gid], a.quats[gid],
-                make_float2(a.scales[3 * gid], a.scales[3 * gid + 1]), a.glob, a.opac[gid],
+                make_float2(a.scales[3 * (size_t)gid], a.scales[3 * (size_t)gid + 1]), a.glob, a.opac[gid],
                 colors ? colors[gid] : make_float3(0.f, 0.f, 0.f), a.uv0[gid],
                 a.umap[gid], a.vmap[gid], a.dims[gid], use_blur, true, R.cull ? R.cull + slot : nullptr,
                 !(a.settings & (1 << 16)));
@@ -1061,7 +1061,7 @@ __global__ void __launch_bounds__(128) records_kernel(SceneArgs a, BatchArgs ba,
         RecCold c;
         RecCull e;
         const bool defer = make_record(h, w, c, i, V, a.means[i], a.quats[i],
-                                       make_float2(a.scales[3 * i], a.scales[3 * i + 1]), a.glob, a.opac[i],
+                                       make_float2(a.scales[3 * (size_t)i], a.scales[3 * (size_t)i + 1]), a.glob, a.opac[i],
                                        ba.colors[j], a.uv0[i], a.umap[i], a.vmap[i], a.dims[i],
                                        a.settings & (1 << 9), false, &e, !(a.settings & (1 << 16)));
         pack_record(srec[threadIdx.x], h, w, c, e);
@@ -1078,7 +1078,7 @@ __device__ __forceinline__ void fix_record(const SceneArgs& a, const View& V, in
     const float3 mc = V.xform(a.means[i]);
     const float3 a1c = V.rot(A.a1), a2c = V.rot(A.a2), nc = V.rot(A.a3);
     const float3 umc = V.rot(a.umap[i]), vmc = V.rot(a.vmap[i]);
-    const float is1 = 1.f / (a.scales[3 * i] * a.glob), is2 = 1.f / (a.scales[3 * i + 1] * a.glob);
+    const float is1 = 1.f / (a.scales[3 * (size_t)i] * a.glob), is2 = 1.f / (a.scales[3 * (size_t)i + 1] * a.glob);
     RecHot h;
     RecWarm w;
     edge_on_solve(h, w, V, mc, a1c, a2c, nc, umc, vmc, is1, is2, dot3(nc, mc));
@@ -1118,7 +1118,7 @@ __global__ void __launch_bounds__(128) view_records_kernel(SceneArgs a, ViewArgs
         RecCold c;
         RecCull e;
         const bool defer = make_record(h, w, c, i, V, a.means[i], a.quats[i],
-                                       make_float2(a.scales[3 * i], a.scales[3 * i + 1]), a.glob, a.opac[i],
+                                       make_float2(a.scales[3 * (size_t)i], a.scales[3 * (size_t)i + 1]), a.glob, a.opac[i],
                                        va.colors[i], a.uv0[i], a.umap[i], a.vmap[i], a.dims[i], a.settings & (1 << 9),
                                        false, &e, !(a.settings & (1 << 16)));
         pack_record(srec[threadIdx.x], h, w, c, e);
@@ -1179,7 +1179,7 @@ __global__ void finalize_kernel(int N, const float* __restrict__ mom, const floa
     // R, l in units of the scales s_k = scale_k glob: 0 v_opac, 1-3 (l1^2, l2^2, l1 l2) v_sigma, 4-5 l_k v_sigma,
     // 6-8 (1, l1, l2) v_t/(n.r), 9-11 vis v_normal, 12-13 v_uv, 14-17 (l1, l2) v_u, (l1, l2) v_v, 20-22 blur
     // mean gradient; a view changes none of the factors, so they are applied to the sums
-    const float s1 = scales[3 * i] * glob, s2 = scales[3 * i + 1] * glob, is1 = 1.f / s1, is2 = 1.f / s2;
+    const float s1 = scales[3 * (size_t)i] * glob, s2 = scales[3 * (size_t)i + 1] * glob, is1 = 1.f / s1, is2 = 1.f / s2;
     // (a sum that no pixel added to stays 0 whatever the scale)
     auto by = [](float f, float r) { return r == 0.f ? 0.f : f * r; };
     const float M[kMomStride] = { R[0], by(-is1 * glob, R[1]), by(-is2 * glob, R[2]), by(is1, R[4]), by(is2, R[5]),
@@ -1212,9 +1212,9 @@ __global__ void finalize_kernel(int N, const float* __restrict__ mom, const floa
         const float o = rg.opacity[i];
         rg.v_raw_opacity[i] = M[0] * o * (1.f - o);
     }
-    rg.v_raw_scales[3 * i] = M[1] * rg.scales[3 * i];
-    rg.v_raw_scales[3 * i + 1] = M[2] * rg.scales[3 * i + 1];
-    rg.v_raw_scales[3 * i + 2] = 0.f;
+    rg.v_raw_scales[3 * (size_t)i] = M[1] * rg.scales[3 * (size_t)i];
+    rg.v_raw_scales[3 * (size_t)i + 1] = M[2] * rg.scales[3 * (size_t)i + 1];
+    rg.v_raw_scales[3 * (size_t)i + 2] = 0.f;
     const float usc = dot3(um, A.a1), uss = dot3(um, A.a2);
     rg.v_mapping[i] = make_float4(M[15], M[16], dot3(vu, um) + dot3(vv, vm), dot3(vu, vm) - dot3(vv, um));
     c0 = c0 + (usc * vu - uss * vv);

@@ -49,3 +49,24 @@ def test_charts_at_the_end_of_a_large_texture(prebuilt):
     assert torch.equal(res[0][0], res[1][0])
     for x, y in zip(res[0][1:], res[1][1:]):
         assert float(x.abs().max()) > 0 and float((x - y).abs().max()) <= 1e-5 * float(x.abs().max())
+
+
+@pytest.mark.parametrize("used", [0, 1])
+def test_sh_of_many_gaussians(used):
+    """Colours and their gradients of Gaussians beyond the 715,827,882th equal
+    those of a small call on the same rows."""
+    import gstex_cuda_gb300 as G
+    n, m = 2 ** 31 // 3 + 301, 300
+    g = torch.Generator().manual_seed(0)
+    dirs, co, up = (torch.randn(*s, generator=g).to(DEV) for s in ((m, 3), (m, 4, 3), (m, 3)))
+
+    def at_the_end(x):
+        big = torch.zeros(n, *x.shape[1:], device=DEV)
+        big[n - m:] = x
+        return big
+
+    far = at_the_end(dirs)
+    got = G.cuda.compute_sh_forward(n, 1, used, far, at_the_end(co))[-m:].clone()
+    assert torch.equal(got, G.cuda.compute_sh_forward(m, 1, used, dirs, co))
+    got = G.cuda.compute_sh_backward(n, 1, used, far, at_the_end(up))[-m:].clone()
+    assert torch.equal(got, G.cuda.compute_sh_backward(m, 1, used, dirs, up))
