@@ -91,8 +91,8 @@ __global__ void bin_edges_kernel(int n, const int64_t* __restrict__ n_dev, const
     }
 #pragma unroll
     for (int q = 0; q < kEdgeItems; q++) {
+        if (i0 + q >= n) break;
         const int i = (int)i0 + q;
-        if (i >= n) break;
         const int prev = tile[q], cur = tile[q + 1];
         const bool ok = cur >= 0 && cur < num_tiles;
         if (i == 0 && ok) bins[cur].x = 0;
@@ -170,22 +170,22 @@ __global__ void __launch_bounds__(kSortThreads) radix_hist_kernel(const K* __res
     chain_wait();
     resolve_count(n_dev, n, chunk);
     __syncthreads();
-    const int start = blockIdx.x * chunk;
-    const int end = min(start + chunk, n);
+    // (positions are unsigned and items counted from the tile's first: those behind
+    // the last item may pass 31 bits)
+    const uint32_t start = blockIdx.x * (uint32_t)chunk;
+    const uint32_t end = min(start + (uint32_t)chunk, (uint32_t)n);
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     uint32_t* hw = h[warp];
-    for (int tbase = start; tbase < end; tbase += kSortThreads * kSortItems) {
+    for (uint32_t tbase = start; tbase < end; tbase += kSortThreads * kSortItems) {
         K key[kSortItems];
+        const int l0 = warp * (32 * kSortItems) + lane, left = (int)(end - tbase);
+        const K* __restrict__ src = keys + tbase;
+#pragma unroll
+        for (int k = 0; k < kSortItems; k++) key[k] = l0 + k * 32 < left ? src[l0 + k * 32] : K(0);
 #pragma unroll
         for (int k = 0; k < kSortItems; k++) {
-            const int i = tbase + warp * (32 * kSortItems) + k * 32 + lane;
-            key[k] = i < end ? keys[i] : K(0);
-        }
-#pragma unroll
-        for (int k = 0; k < kSortItems; k++) {
-            const int i = tbase + warp * (32 * kSortItems) + k * 32 + lane;
-            if (i < end) atomicAdd(&hw[(uint32_t)(key[k] >> shift) & dmask], 1u);
+            if (l0 + k * 32 < left) atomicAdd(&hw[(uint32_t)(key[k] >> shift) & dmask], 1u);
         }
     }
     __syncthreads();
@@ -331,20 +331,23 @@ __global__ void __launch_bounds__(kSortThreads, 4) radix_scatter_kernel(
         const uint32_t base = scatter_scan(totals[tid], wsum);
         run_off[tid] = base + offsets[(size_t)tid * gridDim.x + blockIdx.x];
     }
-    const int start = blockIdx.x * chunk;
-    const int end = min(start + chunk, n);
-    for (int tbase = start; tbase < end; tbase += kSortTile) {
+    const uint32_t start = blockIdx.x * (uint32_t)chunk;
+    const uint32_t end = min(start + (uint32_t)chunk, (uint32_t)n);
+    for (uint32_t tbase = start; tbase < end; tbase += kSortTile) {
         for (int k = tid; k < kSortWarps * kRadix; k += blockDim.x) (&wcnt[0][0])[k] = 0;
         __syncthreads();
         K key[kSortItems];
         uint32_t val[kSortItems];
         uint32_t rank[kSortItems];
+        const int l0 = warp * (32 * kSortItems) + (int)lane, left = (int)(end - tbase);
+        const K* __restrict__ ksrc = kin + tbase;
+        const uint32_t* __restrict__ vsrc = VALS ? vin + tbase : nullptr;
         // all loads first, so that they overlap
 #pragma unroll
         for (int k = 0; k < kSortItems; k++) {
-            const int i = tbase + warp * (32 * kSortItems) + k * 32 + (int)lane;
-            key[k] = i < end ? kin[i] : K(0);
-            if (VALS) val[k] = i < end ? vin[i] : 0u;
+            const int l = l0 + k * 32;
+            key[k] = l < left ? ksrc[l] : K(0);
+            if (VALS) val[k] = l < left ? vsrc[l] : 0u;
         }
         // Each round's lowest lane of a digit adds its count to the warp's
         // counter; the additions of a warp are in order, so no round waits for
@@ -352,12 +355,12 @@ __global__ void __launch_bounds__(kSortThreads, 4) radix_scatter_kernel(
         uint32_t old[kSortItems];
 #pragma unroll
         for (int k = 0; k < kSortItems; k++) {
-            const int i = tbase + warp * (32 * kSortItems) + k * 32 + (int)lane;
+            const bool in = l0 + k * 32 < left;
             const uint32_t d = (uint32_t)(key[k] >> shift) & dmask;
-            const uint32_t peers = same_digit<DB>(__ballot_sync(0xffffffffu, i < end), d);
+            const uint32_t peers = same_digit<DB>(__ballot_sync(0xffffffffu, in), d);
             const uint32_t first = __ffs(peers) - 1;
             old[k] = 0;
-            if (i < end && first == lane) old[k] = atomicAdd(&wcnt[warp][d], (uint32_t)__popc(peers));
+            if (in && first == lane) old[k] = atomicAdd(&wcnt[warp][d], (uint32_t)__popc(peers));
             rank[k] = (first << 8) | (uint32_t)__popc(peers & lt_mask);
             __syncwarp();
         }
@@ -378,8 +381,7 @@ __global__ void __launch_bounds__(kSortThreads, 4) radix_scatter_kernel(
         __syncthreads();
 #pragma unroll
         for (int k = 0; k < kSortItems; k++) {
-            const int i = tbase + warp * (32 * kSortItems) + k * 32 + (int)lane;
-            if (i < end) {
+            if (l0 + k * 32 < left) {
                 const uint32_t d = (uint32_t)(key[k] >> shift) & dmask;
                 const uint32_t local = tile_base[d] + wcnt[warp][d] + rank[k];
                 skey[local] = key[k];
@@ -387,7 +389,7 @@ __global__ void __launch_bounds__(kSortThreads, 4) radix_scatter_kernel(
             }
         }
         __syncthreads();
-        const int tile_n = min(kSortTile, end - tbase);
+        const int tile_n = min(kSortTile, left);
         for (int l = tid; l < tile_n; l += kSortThreads) {
             const K kk = skey[l];
             const uint32_t d = (uint32_t)(kk >> shift) & dmask;
@@ -510,22 +512,23 @@ __global__ void __launch_bounds__(256) view_emit_kernel(int n, int num_isect, in
             behind = (__float_as_uint(depths[gi]) >> 31) != 0u;
         }
         const int stop = min(end, __shfl_sync(0xffffffffu, phi, 31));
-        for (int base = cur; base < stop; base += 32) {  // warp-uniform trip count
-            const int t = base + (int)lane;
+        // (warp-uniform trip count; unsigned, as the last step may pass 31 bits)
+        for (unsigned base = cur; base < (unsigned)stop; base += 32) {
+            const unsigned t = base + lane;
             int q = 0;  // the last lane whose first slot is <= t
 #pragma unroll
             for (int s = 16; s > 0; s >>= 1) {
                 const int l = __shfl_sync(0xffffffffu, plo, q + s);
-                if (l <= t) q += s;
+                if ((unsigned)l <= t) q += s;
             }
             const int ql = __shfl_sync(0xffffffffu, plo, q), qx = __shfl_sync(0xffffffffu, x0, q);
             const int qy = __shfl_sync(0xffffffffu, y0, q), qw = __shfl_sync(0xffffffffu, w, q);
             const int qh = __shfl_sync(0xffffffffu, h, q), qg = __shfl_sync(0xffffffffu, gi, q);
             const bool qb = __shfl_sync(0xffffffffu, (int)behind, q) != 0;
-            if (t < stop) {
+            if (t < (unsigned)stop) {
                 uint32_t key;
                 int32_t val;
-                view_slot(t - ql, qx, qy, qw, qh, qb, qg, tiles_x, tiles_x * tiles_y, key, val);
+                view_slot((int)t - ql, qx, qy, qw, qh, qb, qg, tiles_x, tiles_x * tiles_y, key, val);
                 keys[t] = vals ? key : key << id_bits | (uint32_t)val;
                 if (vals) vals[t] = val;
             }

@@ -31,7 +31,8 @@ void set_cuda_error(cudaError_t e, const char* what);
         if (!(cond)) return GSTEX_ERR_INVALID_ARGUMENT; \
     } while (0)
 
-__host__ __device__ inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
+// (a >= 0; a + b - 1 could pass 31 bits)
+__host__ __device__ inline int ceil_div(int a, int b) { return a / b + (a % b > 0); }
 
 // ---------------------------------------------------------------------------
 // quaternion (w, x, y, z) -> columns ax1, ax2, ax3 of the rotation

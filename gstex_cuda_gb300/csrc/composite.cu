@@ -115,15 +115,17 @@ struct Queue {
 // Scans the list from `pos` (towards higher positions for DIR 1, lower for
 // DIR -1, up to but not including `end`) until 32 splats that reach a pixel
 // of `live` are queued or the list ends.  Returns the number queued.
+// (Upwards, positions are compared as unsigned numbers: 32 beyond the end may
+// pass 31 bits.  Downwards, `end` may be -1.)
 template <int DIR>
 __device__ __forceinline__ int fill_queue(Queue& q, int n, int& pos, int end, const int32_t* __restrict__ gids,
                                           const RecAll* __restrict__ recs, float fx0, float fy0, unsigned live,
                                           unsigned lane) {
-    while (n < 32 && (DIR > 0 ? pos < end : pos > end)) {
-        const int i = pos + DIR * (int)lane;
+    while (n < 32 && (DIR > 0 ? (unsigned)pos < (unsigned)end : pos > end)) {
+        const int i = DIR > 0 ? (int)((unsigned)pos + lane) : pos - (int)lane;
         int gid = 0;
         unsigned m = 0;
-        if (DIR > 0 ? i < end : i > end) {
+        if (DIR > 0 ? (unsigned)i < (unsigned)end : i > end) {
             gid = __ldg(gids + i);
             const RecCull c = unpack_cull(__ldg(recs[gid].c + kChunkCull));
 #pragma unroll
@@ -142,7 +144,7 @@ __device__ __forceinline__ int fill_queue(Queue& q, int n, int& pos, int end, co
             q.mask[s] = m;
         }
         n += __popc(b);
-        pos += DIR * 32;
+        pos = DIR > 0 ? (int)((unsigned)pos + 32u) : pos - 32;
     }
     __syncwarp();
     return n;
@@ -363,9 +365,9 @@ __device__ __forceinline__ void finish_close(Pix& S, const SceneArgs& a, const B
     const PixelRay P = block_pixel(J, J.y0 + lane_row(src), J.x0 + lane_col(src));
     const bool use_blur = !FIX && (a.settings & (1 << 9)) != 0;
     float T = __shfl_sync(kFull, S.T, src);
-    for (int base = from; base < J.range.y; base += 32) {
-        const int i = base + (int)lane;
-        const bool in = i < J.range.y;
+    for (unsigned base = from; base < (unsigned)J.range.y; base += 32) {
+        const unsigned i = base + lane;
+        const bool in = i < (unsigned)J.range.y;
         float alpha = 0.f;
         bool skip = true;
         Hit H;
@@ -391,7 +393,7 @@ __device__ __forceinline__ void finish_close(Pix& S, const SceneArgs& a, const B
                 float opac, nbf, bf, e, eb;
                 const Hit Hs = block_hit(a, ba, J.view, rec, g, P, opac);
                 const float as = block_alpha<FIX>(Hs, opac, use_blur, J.recs + g, P, nbf, bf, e, eb);
-                S.take(a, rec, Hs, as, S.T * (1.f - as), base + f);
+                S.take(a, rec, Hs, as, S.T * (1.f - as), (int)base + f);
             }
             T = __shfl_sync(kFull, S.T, src);
             todo &= f == 31 ? 0u : ~0u << (f + 1);

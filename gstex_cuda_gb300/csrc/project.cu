@@ -100,8 +100,8 @@ __global__ void scan_block_sums(int n, const int32_t* __restrict__ in, const int
     int s = 0;
 #pragma unroll
     for (int k = 0; k < kScanItems; k++) {
-        const int idx = base + k * kScanThreads + threadIdx.x;
-        if (idx < n) {
+        const unsigned idx = base + k * kScanThreads + threadIdx.x;  // (may pass 31 bits)
+        if (idx < (unsigned)n) {
             const int v = in[order ? order[idx] : idx];
             if (order) picked[idx] = v;
             s += v;

@@ -263,7 +263,7 @@ __device__ __forceinline__ void fwd_tile(const SceneArgs& a, const TileJob& J, c
         if (__syncthreads_count(all_done) >= nthr) break;
         const int bstart = range.x + bsz * b;
         const int idx = bstart + tr;
-        if (tr < bsz && idx < range.y) stage_job(R, tr, a, J, a.gids[idx], use_blur);
+        if (tr < bsz && tr < range.y - bstart) stage_job(R, tr, a, J, a.gids[idx], use_blur);
         __syncthreads();
         const int bsize = min(bsz, range.y - bstart);
         if (__all_sync(wmask, all_done)) continue;
@@ -841,7 +841,7 @@ __device__ __forceinline__ void edit_tile(const SceneArgs& a, const TileJob& J, 
         if (__syncthreads_count(done) >= nthr) break;
         const int bstart = range.x + nthr * b;
         const int idx = bstart + tr;
-        if (idx < range.y) stage_job(R, tr, a, J, a.gids[idx], use_blur);
+        if (tr < range.y - bstart) stage_job(R, tr, a, J, a.gids[idx], use_blur);
         __syncthreads();
         const int bsize = min(nthr, range.y - bstart);
         for (int k = 0; k < bsize && !done; ++k) {

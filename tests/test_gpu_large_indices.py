@@ -70,3 +70,49 @@ def test_sh_of_many_gaussians(used):
     assert torch.equal(got, G.cuda.compute_sh_forward(m, 1, used, dirs, co))
     got = G.cuda.compute_sh_backward(n, 1, used, far, at_the_end(up))[-m:].clone()
     assert torch.equal(got, G.cuda.compute_sh_backward(m, 1, used, dirs, up))
+
+
+@pytest.mark.parametrize("partial", [False, True])
+def test_binning_up_to_the_last_count(partial):
+    """524,176 tiles that 4096 Gaussians cover (sorted as one word each), and
+    with two more over some of them 2^31 - 1 intersections (sorted as pairs):
+    every tile lists the covering Gaussians in depth order, and the compositor
+    walks the lists to their ends (the splats are transparent)."""
+    import gstex_cuda_gb300 as G
+    bw, side, n = 8, 724, 4096
+    W = bw * side
+    g = torch.Generator().manual_seed(0)
+    centers, extents = torch.full((n, 2), W / 2.0), torch.full((n, 2), W / 2.0 - 6)
+    depths = 1 + torch.randperm(n, generator=g).float() / n
+    rows, strip = 633, 459
+    if partial:
+        centers = torch.cat([centers, torch.tensor([[W / 2.0, 2528.0], [1836.0, 4.0]])])
+        extents = torch.cat([extents, torch.tensor([[W / 2.0 - 6, 2530.0], [1834.0, 2.0]])])
+        depths = torch.cat([depths, torch.tensor([3.0, 4.0])])
+    N = depths.numel()
+    order = torch.argsort(depths[:n]).int().to(DEV)
+    centers, extents, depths = centers.to(DEV), extents.to(DEV), depths.to(DEV)
+    counts = G.cuda.num_tiles_hit(centers, extents, W, W, bw)
+    tb = (side, side, 1)
+    total, gids, bins = G.utils.bin_view(centers, extents, depths, counts, tb, bw)
+    assert total == side * side * n + (side * rows + strip if partial else 0)
+    if partial:
+        assert total == 2 ** 31 - 1
+    tile = torch.arange(side * side, device=DEV)
+    more = torch.stack([tile < side * rows, tile < strip]).long() if partial else torch.zeros(2, 1, device=DEV).long()
+    end = (n + more.sum(0)).expand(tile.numel()).cumsum(0)
+    start = torch.cat([end.new_zeros(1), end[:-1]])
+    assert torch.equal(bins.long(), torch.stack([start, end], 1))
+    for at in start.split(8192):
+        assert bool((gids[at[:, None] + torch.arange(n, device=DEV)] == order).all())
+    if partial:
+        assert bool((gids[start[:side * rows] + n] == n).all()) and bool((gids[start[:strip] + n + 1] == n + 1).all())
+    z = lambda *s: torch.zeros(*s, device=DEV)  # noqa: E731
+    means = torch.cat([z(N, 2), depths[:, None]], 1)
+    quats = torch.tensor([1.0, 0.0, 0.0, 0.0], device=DEV).repeat(N, 1)
+    dims = torch.tensor([1, 1, 0], dtype=torch.int32, device=DEV).repeat(N, 1)
+    eye = torch.eye(4, device=DEV)
+    outs = G.cuda.texture_forward(tb, (bw, bw, 1), (W, W, 1), (N, 1, 3), dims, gids, bins, z(N, 3), z(N, 1), means,
+                                  z(N, 3) + 1, 1.0, quats, z(N, 1, 2), z(N, 1, 3), z(N, 1, 3), z(1, 3), eye, eye,
+                                  float(W), float(W), W / 2.0, W / 2.0, 1 << 8, z(3))
+    assert bool((outs[5] == 1).all())
