@@ -792,12 +792,14 @@ static bool sort_direct(const SortPlan& p, size_t key_bytes) {
     return key_bytes == 4 && p.chunk == kSortTile && p.blocks <= kDirectBlocks;
 }
 
+// Never less than for a smaller n, so that one workspace serves all counts up to
+// its own: of the rows of block counts it has what the largest launch up to n
+// takes (four of each block with one launch a pass, else one).
 static size_t sort_workspace_bytes(int n, size_t key_bytes) {
     if (n < 1) n = 1;
-    const SortPlan p = sort_plan(n);
-    const size_t counts = sort_direct(p, key_bytes) ? 4 : 1;  // of each pass, or of one
-    return align_up((size_t)n * key_bytes, 256) + align_up((size_t)n * 4, 256) + counts * kRadix * p.blocks * 4 +
-           (size_t)kRadix * 4;
+    const int tiles = ceil_div(n, kSortTile);
+    const size_t rows = std::max(std::min(tiles, kSortMaxBlocks), key_bytes == 4 ? 4 * std::min(tiles, kDirectBlocks) : 0);
+    return align_up((size_t)n * key_bytes, 256) + align_up((size_t)n * 4, 256) + rows * kRadix * 4 + (size_t)kRadix * 4;
 }
 
 extern "C" size_t gstex_sort_workspace_bytes(int n) { return sort_workspace_bytes(n, 8); }
