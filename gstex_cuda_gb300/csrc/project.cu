@@ -95,9 +95,9 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int* warp_sums, int& 
 __global__ void scan_block_sums(int n, const int32_t* __restrict__ in, const int32_t* __restrict__ order,
                                 int32_t* __restrict__ picked, int64_t* __restrict__ sums) {
     chain_wait();
-    __shared__ int ws[32];
+    __shared__ long long part[kScanThreads / 32];
     const int base = blockIdx.x * kScanTile;
-    int s = 0;
+    long long s = 0;  // (a block's counts may pass 31 bits, and the caller has to see it)
 #pragma unroll
     for (int k = 0; k < kScanItems; k++) {
         const unsigned idx = base + k * kScanThreads + threadIdx.x;  // (may pass 31 bits)
@@ -107,9 +107,16 @@ __global__ void scan_block_sums(int n, const int32_t* __restrict__ in, const int
             s += v;
         }
     }
-    int total;
-    block_exclusive_scan(s, ws, total);
-    if (threadIdx.x == 0) sums[blockIdx.x] = total;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        s = 0;
+#pragma unroll
+        for (int w = 0; w < kScanThreads / 32; w++) s += part[w];
+        sums[blockIdx.x] = s;
+    }
 }
 
 // single block: exclusive scan of the block sums (64-bit to detect overflow)
