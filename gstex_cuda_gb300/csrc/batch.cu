@@ -162,10 +162,11 @@ __global__ void gather_counts_kernel(int n, const int32_t* __restrict__ order, c
     if (p < n) out[p] = counts[order[p]];
 }
 
-// The number of slots written, and whether there were more than that.
+// The number of slots written, and whether there were more than that.  From 2^32
+// on the pairs' offsets have wrapped and leave slots unwritten, so none is used.
 __device__ __forceinline__ void clamp_count(const int64_t* total, long long capacity, int64_t* n, int* overflow) {
     const long long t = *total;
-    *n = t < capacity ? t : capacity;
+    *n = t < capacity ? t : t < (1ll << 32) ? capacity : 0;
     if (t > capacity) atomicOr(overflow, 1);
 }
 

@@ -34,3 +34,24 @@ def test_sums_below_that(n):
     total, cum = G.utils.compute_cumulative_intersects(counts.to(DEV))
     want = counts.long().cumsum(0)
     assert total == int(want[-1]) and torch.equal(cum.cpu().long(), want)
+
+
+@pytest.mark.parametrize("total,used", [(5, 5), (64, 64), (65, 64), (2 ** 32 - 1, 64), (2 ** 32, 0), (2 ** 32 + 5, 0)])
+def test_batched_emission_beyond_the_capacity(total, used):
+    """The batched emission uses as many slots as it has, and none once the
+    32-bit offsets of the pairs have wrapped; the overflow is flagged."""
+    from gstex_cuda_gb300 import batch as B
+    L = B._L()
+    cams = [B.Camera(torch.eye(4), 8.0, 8.0, 4.0, 4.0, 8, 8)]
+    r = B.BatchRenderer(cams, 2, capacity=64, block_width=8)
+    # two pairs of one tile each, the second with the rest of the slots
+    r.rects[:] = torch.tensor([[1 << 16, 1 << 16], [1 << 16, 1 << 16]], dtype=torch.int32, device=DEV)
+    r.order[:] = torch.tensor([0, 1], dtype=torch.int32, device=DEV)
+    low = (total + 2 ** 31) % 2 ** 32 - 2 ** 31  # (the offset's 32 bits)
+    r.cum[:] = torch.tensor([1, low], dtype=torch.int64, device=DEV).int()
+    r.total[:] = total
+    rc = L.gstex_batch_emit_sorted(2, 1, r.views_dev.data_ptr(), r.order.data_ptr(), r.cum.data_ptr(),
+                                   r.rects.data_ptr(), r.total.data_ptr(), 64, r.keys.data_ptr(), r.vals.data_ptr(),
+                                   r.count.data_ptr(), r.overflow.data_ptr(),
+                                   torch.cuda.current_stream().cuda_stream)
+    assert rc == 0 and int(r.count) == used and bool(r.overflow) == (total > 64)
