@@ -130,17 +130,26 @@ def stream_of(t: torch.Tensor):
     return torch._C._cuda_getCurrentRawStream(t.get_device())
 
 
+def on_current_device(*tensors) -> bool:
+    """Whether the tensors are on the current CUDA device, the one a kernel
+    launch goes to (a torch operation goes to its tensors')."""
+    current = torch.cuda.current_device()
+    return all(t.get_device() == current for t in tensors)
+
+
 def plain_cuda_f32(*tensors) -> bool:
     """Whether a kernel launch can stand for torch operations on these
-    tensors: float32 CUDA tensors that no gradient, forward-mode tangent,
-    functional transform, tracer, compiler or dispatch mode looks at."""
+    tensors: float32 CUDA tensors of the current device that no gradient,
+    forward-mode tangent, functional transform, tracer, compiler or dispatch
+    mode looks at."""
     grad = torch.is_grad_enabled()
     for t in tensors:
         if type(t) not in (torch.Tensor, torch.nn.Parameter) or not t.is_cuda or t.dtype is not torch.float32 \
                 or (grad and t.requires_grad):
             return False
-    return (torch.autograd.forward_ad._current_level < 0 and torch._C._functorch.peek_interpreter_stack() is None
-            and torch._C._get_tracing_state() is None and not torch.compiler.is_compiling()
+    return (on_current_device(*tensors) and torch.autograd.forward_ad._current_level < 0
+            and torch._C._functorch.peek_interpreter_stack() is None and torch._C._get_tracing_state() is None
+            and not torch.compiler.is_compiling()
             and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0)
 
 

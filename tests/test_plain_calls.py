@@ -1,0 +1,39 @@
+"""Which calls a kernel launch may stand for (no GPU: the tensors' places are
+stood in for)."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from gstex_cuda_gb300 import _lib
+
+
+@pytest.mark.parametrize("places,current,want", [((0,), 0, True), ((1,), 0, False), ((1, 1), 1, True),
+                                                 ((0, 1), 0, False), ((0, 1), 1, False)])
+def test_launches_go_to_the_current_device(places, current, want, monkeypatch):
+    """A launch goes to the current device, so tensors of another one keep the
+    torch operations, which go to theirs."""
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: current)
+    assert _lib.on_current_device(*(SimpleNamespace(get_device=lambda p=p: p) for p in places)) is want
+
+
+def test_projection_asks_for_the_current_device(monkeypatch):
+    """project_points asks before it launches: with CPU tensors that pass for
+    CUDA ones of another device it takes the torch operations."""
+    from gstex_cuda_gb300 import get_aabb_2d as A
+
+    class Elsewhere:
+        """The parts of a tensor that plain_cuda_f32 reads."""
+        is_cuda, dtype, requires_grad = True, torch.float32, False
+
+        def get_device(self):
+            return 1
+
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    monkeypatch.setattr(torch, "Tensor", Elsewhere)
+    assert not _lib.plain_cuda_f32(Elsewhere(), Elsewhere())
+    monkeypatch.undo()
+    seen = []
+    monkeypatch.setattr(_lib, "plain_cuda_f32", lambda *t: seen.append(len(t)))
+    pix, depth = A.project_points(torch.ones(3, 3), torch.eye(4), (1.0, 1.0, 0.0, 0.0))
+    assert seen == [2] and depth.tolist() == [1.0, 1.0, 1.0]
