@@ -137,17 +137,28 @@ def on_current_device(*tensors) -> bool:
     return all(t.get_device() == current for t in tensors)
 
 
+def full_f32_products() -> bool:
+    """Whether torch's float32 matrix products are full float32: no autocast,
+    no reduced precision of products (which raises if it was set through both
+    of torch's interfaces)."""
+    try:
+        return not torch.is_autocast_enabled("cuda") and torch.get_float32_matmul_precision() == "highest"
+    except RuntimeError:
+        return False
+
+
 def plain_cuda_f32(*tensors) -> bool:
     """Whether a kernel launch can stand for torch operations on these
     tensors: float32 CUDA tensors of the current device that no gradient,
     forward-mode tangent, functional transform, tracer, compiler or dispatch
-    mode looks at."""
+    mode looks at, with products in full float32."""
     grad = torch.is_grad_enabled()
     for t in tensors:
         if type(t) not in (torch.Tensor, torch.nn.Parameter) or not t.is_cuda or t.dtype is not torch.float32 \
                 or (grad and t.requires_grad):
             return False
-    return (on_current_device(*tensors) and torch.autograd.forward_ad._current_level < 0
+    return (on_current_device(*tensors) and full_f32_products()
+            and torch.autograd.forward_ad._current_level < 0
             and torch._C._functorch.peek_interpreter_stack() is None and torch._C._get_tracing_state() is None
             and not torch.compiler.is_compiling()
             and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0)

@@ -1,0 +1,40 @@
+"""project_points under autocast and with reduced-precision products: the torch
+operations' results, with and without gradients alike."""
+import contextlib
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+INTR = (400.0, 390.5, 399.5, 300.25)
+
+
+@contextlib.contextmanager
+def _precision(mode):
+    if mode in (torch.float16, torch.bfloat16):
+        with torch.autocast("cuda", dtype=mode):
+            yield
+        return
+    before = torch.get_float32_matmul_precision()
+    torch.set_float32_matmul_precision(mode)
+    try:
+        yield
+    finally:
+        torch.set_float32_matmul_precision(before)
+
+
+@pytest.mark.parametrize("mode", [torch.float16, torch.bfloat16, "high", "highest"])
+def test_the_same_with_and_without_gradients(mode):
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from gstex_cuda_gb300.get_aabb_2d import project_points
+    g = torch.Generator().manual_seed(0)
+    p, vm = (3 * torch.randn(5000, 3, generator=g)).to(DEV), torch.eye(4)
+    vm[:3, :3] = torch.linalg.qr(torch.randn(3, 3, generator=g))[0]
+    vm[:3, 3] = torch.randn(3, generator=g)
+    vm = vm.to(DEV)
+    with _precision(mode):
+        pix, depth = project_points(p, vm, INTR)
+        tp, td = project_points(p.clone().requires_grad_(), vm, INTR)
+    assert pix.dtype == tp.dtype and torch.equal(pix, tp.detach()) and torch.equal(depth, td.detach())

@@ -37,3 +37,22 @@ def test_projection_asks_for_the_current_device(monkeypatch):
     monkeypatch.setattr(_lib, "plain_cuda_f32", lambda *t: seen.append(len(t)))
     pix, depth = A.project_points(torch.ones(3, 3), torch.eye(4), (1.0, 1.0, 0.0, 0.0))
     assert seen == [2] and depth.tolist() == [1.0, 1.0, 1.0]
+
+
+def test_products_in_another_type(monkeypatch):
+    """Autocast and torch's reduced-precision products change the torch
+    operations' results; a launch, which computes in float32, does not stand
+    for them then."""
+    assert _lib.full_f32_products()
+    with monkeypatch.context() as m:
+        m.setattr(torch, "is_autocast_enabled", lambda device: device == "cuda")
+        assert not _lib.full_f32_products()
+    for precision in ("high", "medium"):
+        monkeypatch.setattr(torch, "get_float32_matmul_precision", lambda: precision)
+        assert not _lib.full_f32_products()
+
+    def mixed():
+        raise RuntimeError("set through both interfaces")
+
+    monkeypatch.setattr(torch, "get_float32_matmul_precision", mixed)
+    assert not _lib.full_f32_products()
