@@ -277,7 +277,9 @@ class BatchRenderer:
         self.tile_order = torch.empty(self.total_tiles, **i32) if heavy_first else None
         self.order_ws = (torch.empty(L.gstex_batch_tile_order_workspace_bytes(self.total_tiles), **u8)
                          if heavy_first else None)
-        self._order_groups = self._tile_groups() if heavy_first else None
+        self._order_groups = {}  # of every order_group used: captured graphs keep reading theirs
+        if heavy_first:
+            self._tile_groups()
         self.queue = torch.zeros(1, **i32)
         self.bg = torch.tensor(list(background), **f32)
         # per-pixel outputs of all views
@@ -302,15 +304,18 @@ class BatchRenderer:
 
     def _tile_groups(self):
         """Groups of order_group^2 neighbouring tiles of a view, in tile order
-        ([n, 4]: first tile, tiles per row, width, height), with the
-        order_group they were made for; None in their place if there are too
-        many for the one-launch order."""
+        ([n, 4]: first tile, tiles per row, width, height); None where the
+        one-launch order does not apply: there are too many of them, or they
+        would have to be copied to the device within a capture."""
         G, n = self.order_group, _I(0)
-        rows = torch.empty((self.MAX_SMALL_GROUPS, 4), dtype=torch.int32)
-        if G < 1 or _L().gstex_batch_tile_groups(self.V, self.descs, self.bw, G, self.MAX_SMALL_GROUPS, ptr(rows),
-                                                 ctypes.byref(n)):
-            return G, None
-        return G, rows[:n.value].to(self.dev)
+        if G not in self._order_groups:
+            if torch.cuda.is_current_stream_capturing():
+                return None
+            rows = torch.empty((self.MAX_SMALL_GROUPS, 4), dtype=torch.int32)
+            rc = _L().gstex_batch_tile_groups(self.V, self.descs, self.bw, G, self.MAX_SMALL_GROUPS, ptr(rows),
+                                              ctypes.byref(n))
+            self._order_groups[G] = None if rc else rows[:n.value].to(self.dev)
+        return self._order_groups[G]
 
     def _alloc_isect(self):
         L = _L()
@@ -419,9 +424,7 @@ class BatchRenderer:
                                    self.sort_ws.numel(), st), "sort_pairs32")
         check(L.gstex_get_tile_bin_edges32_dyn(self.capacity, ptr(self.count), ptr(self.keys_sorted), 1,
                                                self.total_tiles, ptr(self.bins), st), "tile_bin_edges32_dyn")
-        if self.tile_order is not None and self._order_groups[0] != self.order_group:
-            self._order_groups = self._tile_groups()
-        groups = self._order_groups[1] if self.tile_order is not None else None
+        groups = self._tile_groups() if self.tile_order is not None else None
         if groups is not None:
             check(L.gstex_batch_tile_order_small(groups.shape[0], ptr(groups), ptr(self.bins), ptr(self.tile_order),
                                                  st), "batch_tile_order_small")
