@@ -455,7 +455,7 @@ extern "C" int gstex_batch_tile_groups(int num_views, const gstex_view_desc* vie
     long long total_pix = 0;
     int rc = gstex_batch_layout(num_views, views, block_width, &total_tiles, &total_pix);
     if (rc) return rc;
-    GSTEX_REQUIRE(group >= 1 && max_groups >= 0 && num_groups && (groups || max_groups == 0));
+    GSTEX_REQUIRE(group >= 1 && group <= 64 && max_groups >= 0 && num_groups && (groups || max_groups == 0));
     long long n = 0;
     int off = 0;
     for (int v = 0; v < num_views; v++) {

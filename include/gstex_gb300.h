@@ -396,8 +396,9 @@ size_t gstex_batch_tile_order_workspace_bytes(int total_tiles);
 int gstex_batch_tile_order(int total_tiles, const int32_t* tile_bins, const int32_t* tile_view,
                            const void* views_dev, int group, int32_t* order, void* workspace,
                            size_t workspace_bytes, gstex_stream_t stream);
-/* Groups for gstex_batch_tile_order_small, in tile order, written to host
- * memory groups [max_groups, 4]; "unsupported" if there are more. */
+/* Groups for gstex_batch_tile_order_small (group: 1 to 64, as in
+ * gstex_batch_tile_order), in tile order, written to host memory groups
+ * [max_groups, 4]; "unsupported" if there are more. */
 int gstex_batch_tile_groups(int num_views, const gstex_view_desc* views, int block_width, int group, int max_groups,
                             int32_t* groups, int* num_groups);
 /* The same order in one launch, for up to 4096 groups given by the caller in

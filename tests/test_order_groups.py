@@ -30,3 +30,14 @@ def test_groups_of_an_earlier_order_group_stay(monkeypatch):
     r.order_group = 3
     monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
     assert r._tile_groups() is None
+
+
+@pytest.mark.parametrize("group,ok", [(-1, False), (0, False), (1, True), (64, True), (65, False), (1000, False)])
+def test_order_groups_that_are_refused(group, ok, monkeypatch):
+    """1 to 64 tiles a side, as gstex_batch_tile_order takes them; others have
+    no groups, and the renderer's step goes on to the refusal there."""
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    r = _renderer(40, 24, group)
+    rows, n = torch.empty((64, 4), dtype=torch.int32), ctypes.c_int(0)
+    rc = B._L().gstex_batch_tile_groups(1, r.descs, 8, group, 64, rows.data_ptr(), ctypes.byref(n))
+    assert rc == (0 if ok else 1) and (r._tile_groups() is not None) is ok
