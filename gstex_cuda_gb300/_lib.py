@@ -58,6 +58,7 @@ _SIGS = {
     "gstex_get_aabb_2d": (_I, [_I, _P, _P, _F, _P, _P, _F, _F, _F, _F, _P, _P, _P]),
     "gstex_project_points": (_I, [_I, _P, _P, _F, _F, _F, _F, _P, _P, _P]),
     "gstex_num_tiles_hit": (_I, [_I, _P, _P, _I, _I, _I, _P, _P]),
+    "gstex_block_kernels": (_I, [_I, _I, _I, _I]),
     "gstex_view_records_bytes": (ctypes.c_size_t, [_I]),
     "gstex_view_records": (_I, [_P, _P, ctypes.c_size_t, _P]),
     "gstex_scan_workspace_bytes": (ctypes.c_size_t, [_I]),

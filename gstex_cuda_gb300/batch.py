@@ -541,9 +541,21 @@ class BatchRenderer:
         return loss
 
     # ------------------------------------------------------------------
+    def takes_knobs(self) -> bool:
+        """Whether this renderer runs the tile kernels, whose launches the tuned
+        knobs shape.  The block kernels (records, tiles of a multiple of 8,
+        no or three channels, no alpha visualisation) take none."""
+        return not _L().gstex_block_kernels(self.bw, self.C, self.settings, self.records is not None)
+
     def tune_key(self) -> str:
-        return autotune_key(self.sizes, self.N, self.C, self.texmode, self.settings, self.bw,
-                            torch.cuda.get_device_name(self.dev))
+        """autotune_key of this renderer, with the kernels it runs where that
+        depends on its records (the block and the tile kernels must not take
+        each other's tunings)."""
+        key = autotune_key(self.sizes, self.N, self.C, self.texmode, self.settings, self.bw,
+                           torch.cuda.get_device_name(self.dev))
+        if _L().gstex_block_kernels(self.bw, self.C, self.settings, 1):
+            key += f";records={int(self.records is not None)}"
+        return key
 
     def autotune(self, s: Scene, tgt_img, tgt_tex, reps: int = 2, use_cache: bool = True) -> dict:
         """Choose pixels-per-thread and Gaussians per batch (64, 128 or one per
@@ -551,6 +563,9 @@ class BatchRenderer:
         walk (32, 16, 8, 4), the resident-CTA variant and Gaussians per batch
         (48, 64, 128 or one per thread) of the backward kernel, by timing each
         candidate on this scene and these cameras (CUDA events).
+        Where the knobs have no effect (takes_knobs) every candidate is the
+        same launch: each kernel is timed once, that time stands for all of
+        them, and the knobs stay as they are.
         The tile width is fixed per renderer (it sets the binning): to tune
         it, build a renderer per block_width and time whole steps.
         With use_cache, a tuning of the same resolution mix, Gaussian count,
@@ -558,17 +573,22 @@ class BatchRenderer:
         named by GSTEX_AUTOTUNE_CACHE) is applied without timing; new tunings
         are stored there."""
         key = self.tune_key()
+        knobs = self.takes_knobs()
+        own = {k: getattr(self, k) for k in TUNED_KNOBS}
         if use_cache:
             hit = autotune_cache_load().get(key)
             if hit is not None:
-                for k in TUNED_KNOBS:
-                    setattr(self, k, int(hit[k]))
+                if knobs:
+                    for k in TUNED_KNOBS:
+                        setattr(self, k, int(hit[k]))
                 self.graph = None
                 return dict(hit, cached=True)
         stream = torch.cuda.current_stream(self.dev)
         self.bin(s)
 
-        def timed(fn):
+        def timed(fn, same_as=None):
+            if same_as is not None and not knobs:
+                return same_as
             fn()
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             e0.record(stream)
@@ -582,14 +602,14 @@ class BatchRenderer:
         best = None
         for ppt in (1, 2):
             self.fwd_ppt, self.fwd_batch = ppt, 0
-            ms = timed(lambda: self.forward(s))
+            ms = timed(lambda: self.forward(s), best and best[0])
             result[f"forward_ppt{ppt}_ms"] = ms
             best = (ms, ppt, 0) if best is None or ms < best[0] else best
         for nb in (64, 128):
             if nb >= self.bw * self.bw:
                 continue  # not below one Gaussian per thread
             self.fwd_ppt, self.fwd_batch = 1, nb
-            ms = timed(lambda: self.forward(s))
+            ms = timed(lambda: self.forward(s), best[0])
             result[f"forward_ppt1_batch{nb}_ms"] = ms
             best = (ms, 1, nb) if ms < best[0] else best
         self.fwd_ppt, self.fwd_batch = best[1], best[2]
@@ -605,17 +625,20 @@ class BatchRenderer:
                 cands += [(1, 32, 10)]
         for ppt, gs, ctas in cands:
             self.bwd_ppt, self.bwd_group, self.bwd_ctas, self.bwd_batch = ppt, gs, ctas, 0
-            ms = timed(lambda: self.backward(s))
+            ms = timed(lambda: self.backward(s), best and best[0])
             result[f"backward_ppt{ppt}_g{gs}" + (f"_ctas{ctas}" if ctas else "") + "_ms"] = ms
             best = (ms, ppt, gs, ctas, 0) if best is None or ms < best[0] else best
         for nb in (48, 64, 128):
             if nb >= self.bw * self.bw // best[1]:
                 continue  # not below one Gaussian per thread
             self.bwd_ppt, self.bwd_group, self.bwd_ctas, self.bwd_batch = best[1], best[2], best[3], nb
-            ms = timed(lambda: self.backward(s))
+            ms = timed(lambda: self.backward(s), best[0])
             result[f"backward_ppt{best[1]}_g{best[2]}" + (f"_ctas{best[3]}" if best[3] else "") + f"_batch{nb}_ms"] = ms
             best = (ms, best[1], best[2], best[3], nb) if ms < best[0] else best
         self.bwd_ppt, self.bwd_group, self.bwd_ctas, self.bwd_batch = best[1], best[2], best[3], best[4]
+        if not knobs:
+            for k, v in own.items():
+                setattr(self, k, v)
         result.update(fwd_ppt=self.fwd_ppt, fwd_batch=self.fwd_batch or "threads", bwd_ppt=self.bwd_ppt,
                       bwd_group=self.bwd_group, bwd_batch=self.bwd_batch or "threads",
                       bwd_ctas=self.bwd_ctas or "default")

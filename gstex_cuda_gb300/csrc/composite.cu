@@ -1016,7 +1016,7 @@ __global__ void __launch_bounds__(32 * kBlockWarps, kBwdCtas)
 // texture or three channels, and prebuilt records; the tile kernels of
 // raster.cu take the rest, and the alpha-visualisation mode.
 bool blocks_apply(int bw, int C, int settings, const RecAll* recs) {
-    return (bw & 7) == 0 && (C == 0 || C == 3) && recs && !(settings & (1 << 16));
+    return gstex_block_kernels(bw, C, settings, recs != nullptr);
 }
 
 int launch_fwd_blocks(const SceneArgs& a, const BlockArgs& ba, const FwdOut& o, int texmode, cudaStream_t stream) {
@@ -1060,3 +1060,7 @@ int launch_bwd_blocks(const SceneArgs& a, const BlockArgs& ba, const BwdArgs& g,
 }
 
 }  // namespace gstex
+
+extern "C" int gstex_block_kernels(int bw, int C, int settings, int with_records) {
+    return (bw & 7) == 0 && (C == 0 || C == 3) && with_records && !(settings & (1 << 16));
+}

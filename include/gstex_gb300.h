@@ -220,6 +220,10 @@ typedef struct gstex_raster_inputs {
     int group_lanes;
 } gstex_raster_inputs;
 
+/* Whether the compositor runs one warp per 8x4 pixels for such a call (1) or
+ * the tile kernels (0), to which alone the launch knobs apply. */
+int gstex_block_kernels(int block_width, int channels, int settings, int with_records);
+
 /* Bytes of the records buffer of one view: 224 per Gaussian plus the list
  * of near-edge-on records solved in double precision. */
 size_t gstex_view_records_bytes(int num_points);
