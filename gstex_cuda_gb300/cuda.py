@@ -206,15 +206,18 @@ def bin_view(centers, extents, depths, num_tiles_hit, tile_bounds, block_width, 
     more = () if texture_dims is None else (texels,)
     if total >= 2 ** 31:
         raise OverflowError(f"{total} intersections exceed the int32 range of the reference's cumsum")
-    if ties:  # depths of +0: the order of the 64-bit keys
+    num_tiles = int(tile_bounds[0]) * int(tile_bounds[1])
+    # depths of +0 have the order of the 64-bit keys; 2^30 tiles or more no 32-bit keys
+    if total > 0 and (ties or num_tiles >= 2 ** 30):
         cum, _ = inclusive_scan(num_tiles_hit)
         keys, ids = map_gaussian_to_intersects(n, total, centers, extents, depths, cum, tile_bounds, block_width)
-        num_tiles = int(tile_bounds[0]) * int(tile_bounds[1])
         keys, ids = sort_pairs(keys, ids, sort_end_bit(num_tiles))
         return (total, ids, get_tile_bin_edges(total, keys, tile_bounds)) + more
     total = max(total, 0)
     gids = torch.empty(total, dtype=torch.int32, device=dev)
-    bins = torch.empty((int(tile_bounds[0]) * int(tile_bounds[1]), 2), dtype=torch.int32, device=dev)
+    if total == 0:
+        return (0, gids, torch.zeros((num_tiles, 2), dtype=torch.int32, device=dev)) + more
+    bins = torch.empty((num_tiles, 2), dtype=torch.int32, device=dev)
     wsb = L.gstex_view_bins_workspace_bytes(total)
     ws = torch.empty(wsb, dtype=torch.uint8, device=dev)
     check(L.gstex_view_bins(n, total, ptr(centers), ptr(extents), ptr(depths), p_order, p_cum,

@@ -116,3 +116,21 @@ def test_binning_up_to_the_last_count(partial):
                                   z(N, 3) + 1, 1.0, quats, z(N, 1, 2), z(N, 1, 3), z(N, 1, 3), z(1, 3), eye, eye,
                                   float(W), float(W), W / 2.0, W / 2.0, 1 << 8, z(3))
     assert bool((outs[5] == 1).all())
+
+
+@pytest.mark.parametrize("n", [2, 5000])
+def test_as_many_tiles_as_64_bit_keys_take(n):
+    """2^30 tiles, which 32-bit keys of a tile and a bit do not hold."""
+    import gstex_cuda_gb300 as G
+    side, bw = 2 ** 15, 2
+    g = torch.Generator().manual_seed(n)
+    at = torch.randint(0, side, (n, 2), generator=g)
+    depths = 1 + torch.randperm(n, generator=g).float() / n
+    tile, order = torch.sort(at[:, 1] * side + at[:, 0])
+    centers = (bw * at + 1).float().to(DEV)
+    extents = torch.full((n, 2), 0.25, device=DEV)
+    counts = torch.ones(n, dtype=torch.int32, device=DEV)
+    total, gids, bins = G.utils.bin_view(centers, extents, depths.to(DEV), counts, (side, side, 1), bw)
+    assert total == n and torch.equal(gids.cpu().long(), order)  # (no two in one tile)
+    assert torch.equal(bins[tile.to(DEV), 0].cpu().long(), torch.arange(n))
+    assert int((bins[:, 1] > bins[:, 0]).sum()) == n
