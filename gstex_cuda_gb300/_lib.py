@@ -150,13 +150,13 @@ def full_f32_products() -> bool:
 
 def plain_cuda_f32(*tensors) -> bool:
     """Whether a kernel launch can stand for torch operations on these
-    tensors: float32 CUDA tensors of the current device that no gradient,
-    forward-mode tangent, functional transform, tracer, compiler or dispatch
-    mode looks at, with products in full float32."""
+    tensors: float32 CUDA tensors of the current device, whose memory holds
+    their values, that no gradient, forward-mode tangent, functional transform,
+    tracer, compiler or dispatch mode looks at, with products in full float32."""
     grad = torch.is_grad_enabled()
     for t in tensors:
         if type(t) not in (torch.Tensor, torch.nn.Parameter) or not t.is_cuda or t.dtype is not torch.float32 \
-                or (grad and t.requires_grad):
+                or (grad and t.requires_grad) or t.is_neg() or t.layout is not torch.strided:
             return False
     return (on_current_device(*tensors) and full_f32_products()
             and torch.autograd.forward_ad._current_level < 0

@@ -1,5 +1,5 @@
-"""project_points under autocast and with reduced-precision products: the torch
-operations' results, with and without gradients alike."""
+"""project_points under autocast, with reduced-precision products and of negated
+views: the torch operations' results, as with gradients."""
 import contextlib
 
 import pytest
@@ -38,3 +38,21 @@ def test_the_same_with_and_without_gradients(mode):
         pix, depth = project_points(p, vm, INTR)
         tp, td = project_points(p.clone().requires_grad_(), vm, INTR)
     assert pix.dtype == tp.dtype and torch.equal(pix, tp.detach()) and torch.equal(depth, td.detach())
+
+
+@pytest.mark.parametrize("n", [5, 3000])
+def test_points_that_are_stored_negated(n):
+    """A view that torch negates as it reads it (the imaginary part of a
+    conjugate is one): its memory holds the opposite of its values."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from gstex_cuda_gb300.get_aabb_2d import project_points
+    g = torch.Generator().manual_seed(n)
+    p, vm = torch.randn(n, 3, generator=g).to(DEV), torch.eye(4, device=DEV)
+    view = torch._neg_view(p)
+    assert view.is_neg()
+    pix, depth = project_points(view, vm, INTR)
+    want, wdepth = project_points(-p, vm, INTR)
+    assert torch.allclose(depth, wdepth, rtol=1e-6, atol=1e-6) and torch.allclose(pix, want, rtol=1e-4)
+    _, moved = project_points(p, torch._neg_view(-vm), INTR)
+    assert torch.allclose(moved, -wdepth, rtol=1e-6, atol=1e-6)

@@ -24,7 +24,10 @@ def test_projection_asks_for_the_current_device(monkeypatch):
 
     class Elsewhere:
         """The parts of a tensor that plain_cuda_f32 reads."""
-        is_cuda, dtype, requires_grad = True, torch.float32, False
+        is_cuda, dtype, requires_grad, layout = True, torch.float32, False, torch.strided
+
+        def is_neg(self):
+            return False
 
         def get_device(self):
             return 1
