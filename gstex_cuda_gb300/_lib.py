@@ -128,7 +128,8 @@ def stream_of(t: torch.Tensor):
     """Handle of the current torch stream on t's device."""
     if not t.is_cuda:
         raise GstexError("gstex_cuda_gb300 operators need CUDA tensors (no CPU implementation)")
-    return torch._C._cuda_getCurrentRawStream(t.get_device())
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)  # (torch's own, without a Stream object)
+    return raw(t.get_device()) if raw is not None else torch.cuda.current_stream(t.device).cuda_stream
 
 
 def on_current_device(*tensors) -> bool:
@@ -148,6 +149,18 @@ def full_f32_products() -> bool:
         return False
 
 
+def unobserved() -> bool:
+    """Whether nothing looks at torch operations as they are called.  A torch
+    that has no answer under these (partly its own) names is taken to look."""
+    try:
+        return (torch.autograd.forward_ad._current_level < 0
+                and torch._C._functorch.peek_interpreter_stack() is None and torch._C._get_tracing_state() is None
+                and not torch.compiler.is_compiling()
+                and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0)
+    except AttributeError:
+        return False
+
+
 def plain_cuda_f32(*tensors) -> bool:
     """Whether a kernel launch can stand for torch operations on these
     tensors: float32 CUDA tensors of the current device, whose memory holds
@@ -158,11 +171,7 @@ def plain_cuda_f32(*tensors) -> bool:
         if type(t) not in (torch.Tensor, torch.nn.Parameter) or not t.is_cuda or t.dtype is not torch.float32 \
                 or (grad and t.requires_grad) or t.is_neg() or t.layout is not torch.strided:
             return False
-    return (on_current_device(*tensors) and full_f32_products()
-            and torch.autograd.forward_ad._current_level < 0
-            and torch._C._functorch.peek_interpreter_stack() is None and torch._C._get_tracing_state() is None
-            and not torch.compiler.is_compiling()
-            and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0)
+    return on_current_device(*tensors) and full_f32_products() and unobserved()
 
 
 def require_cuda(*tensors, names=None):

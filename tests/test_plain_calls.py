@@ -59,3 +59,29 @@ def test_products_in_another_type(monkeypatch):
 
     monkeypatch.setattr(torch, "get_float32_matmul_precision", mixed)
     assert not _lib.full_f32_products()
+
+
+@pytest.mark.parametrize("where,name", [(torch._C, "_functorch"), (torch._C, "_get_tracing_state"),
+                                        (torch._C, "_len_torch_dispatch_stack"),
+                                        (torch._C, "_len_torch_function_stack"),
+                                        (torch.autograd.forward_ad, "_current_level")])
+def test_a_torch_without_one_of_its_private_names(where, name, monkeypatch):
+    """Names that torch does not promise: without one the torch operations are
+    kept."""
+    assert _lib.unobserved()
+    monkeypatch.delattr(where, name)
+    assert not _lib.unobserved()
+
+
+def test_streams_without_the_raw_lookup(monkeypatch):
+    """The current stream's handle through torch's public interface."""
+    asked = []
+
+    def current_stream(device):
+        asked.append(device)
+        return SimpleNamespace(cuda_stream=1234)
+
+    monkeypatch.setattr(torch.cuda, "current_stream", current_stream)
+    monkeypatch.delattr(torch._C, "_cuda_getCurrentRawStream", raising=False)
+    t = SimpleNamespace(is_cuda=True, device="cuda:3", get_device=lambda: 3)
+    assert _lib.stream_of(t) == 1234 and asked == ["cuda:3"]
