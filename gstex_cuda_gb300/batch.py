@@ -20,7 +20,7 @@ import ctypes
 import json
 import os
 from collections import Counter
-from dataclasses import dataclass
+from dataclasses import dataclass, replace
 from typing import List, Optional, Sequence
 
 import torch
@@ -367,8 +367,8 @@ class BatchRenderer:
 
     def activated(self, raw: RawScene) -> Scene:
         """The device buffers that bin_raw fills with the activated parameters
-        of `raw` (allocated once; the texels, SH coefficients and means are
-        raw's own tensors)."""
+        of `raw` (allocated once for its means; the texels, SH coefficients and
+        means are raw's own tensors)."""
         if getattr(self, "_act", None) is None or self._act.means is not raw.means:
             f32 = dict(dtype=torch.float32, device=self.dev)
             N = self.N
@@ -377,6 +377,10 @@ class BatchRenderer:
                               uv0=torch.empty((N, 1, 2), **f32), umap=torch.empty((N, 1, 3), **f32),
                               vmap=torch.empty((N, 1, 3), **f32), texture_dims=raw.texture_dims,
                               texture=raw.texture, channels=raw.channels, glob_scale=raw.glob_scale)
+        own = {k: getattr(raw, k) for k in ("sh_coeffs", "sh_degree", "texture_dims", "texture", "channels",
+                                            "glob_scale")}
+        if any(getattr(self._act, k) is not v for k, v in own.items()):  # another scene over the same means
+            self._act = replace(self._act, **own)
         return self._act
 
     def bin_raw(self, raw: RawScene) -> Scene:
