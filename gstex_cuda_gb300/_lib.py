@@ -136,7 +136,10 @@ def on_current_device(*tensors) -> bool:
     """Whether the tensors are on the current CUDA device, the one a kernel
     launch goes to (a torch operation goes to its tensors')."""
     current = torch.cuda.current_device()
-    return all(t.get_device() == current for t in tensors)
+    for t in tensors:
+        if t.get_device() != current:
+            return False
+    return True
 
 
 def full_f32_products() -> bool:
