@@ -157,7 +157,7 @@ LOSS_WEIGHTS = dict(img=1.0, texture=1.0, reg=100.0, normal=0.05)
 FIXED_BWD_MASK = (1 << 2) | (1 << 8) | (1 << 9) | (1 << 10)
 FIXED_BWD_SETTINGS = 1 << 8
 
-# Launch knobs the autotuner chooses, and its cache: in this process, and in
+# Launch knobs of the tile kernels that the autotuner chooses, and its cache: in this process, and in
 # the JSON file named by GSTEX_AUTOTUNE_CACHE when that is set.
 TUNED_KNOBS = ("fwd_ppt", "fwd_batch", "bwd_ppt", "bwd_group", "bwd_ctas", "bwd_batch")
 _tune_cache: dict = {}

@@ -583,7 +583,7 @@ extern "C" int gstex_batch_tile_order(int total_tiles, const int32_t* tile_bins,
     cudaStream_t st = (cudaStream_t)s;
     const int blocks = ceil_div(total_tiles, 256);
     launch_chained(tile_group_keys_kernel, blocks, 256, 0, st, total_tiles, (const int2*)tile_bins, tile_view,
-                                                   (const BatchView*)views_dev, group, group_key, ids, cost_key);
+                   (const BatchView*)views_dev, group, group_key, ids, cost_key);
     int rc = check_launch("batch_tile_order");
     if (rc) return rc;
     if (group == 1)  // tiles are already in tile order
@@ -620,10 +620,8 @@ extern "C" int gstex_batch_emit_sorted(int N, int V, const void* views_dev, cons
     }
     GSTEX_REQUIRE(order && cum && rects && keys && vals && ((uintptr_t)rects & 7) == 0);
     const int VN = N * V;
-    launch_chained(batch_emit_sorted_kernel, ceil_div(VN, 256), 256, 0, stream,
-                   VN, N, (const BatchView*)views_dev, order, cum,
-                                                                     (const uint2*)rects, total, capacity, keys, vals, count,
-                                                                     overflow);
+    launch_chained(batch_emit_sorted_kernel, ceil_div(VN, 256), 256, 0, stream, VN, N, (const BatchView*)views_dev,
+                   order, cum, (const uint2*)rects, total, capacity, keys, vals, count, overflow);
     return check_launch("batch_emit_sorted");
 }
 
@@ -818,10 +816,8 @@ extern "C" int gstex_batch_image_loss(long long total_pixels, int V, const long 
     if (e != cudaSuccess) { set_cuda_error(e, "batch_image_loss"); return GSTEX_ERR_CUDA; }
     if (total_pixels == 0) return GSTEX_OK;
     const int blocks = (int)std::min<long long>((total_pixels + kLossThreads - 1) / kLossThreads, 152 * kLossCtas);
-    launch_chained(batch_loss_kernel, blocks, kLossThreads, 0, stream,
-                   total_pixels, V, pix_offsets, channels, (const float3*)img, tex,
-                                                  (const float3*)normal, reg, (const float3*)tgt_img, tgt_tex, w_img,
-                                                  w_tex, w_reg, w_normal, (float3*)v_img, v_tex, (float3*)v_normal,
-                                                  v_reg, loss);
+    launch_chained(batch_loss_kernel, blocks, kLossThreads, 0, stream, total_pixels, V, pix_offsets, channels,
+                   (const float3*)img, tex, (const float3*)normal, reg, (const float3*)tgt_img, tgt_tex, w_img, w_tex,
+                   w_reg, w_normal, (float3*)v_img, v_tex, (float3*)v_normal, v_reg, loss);
     return check_launch("batch_image_loss");
 }

@@ -857,7 +857,7 @@ static int sort_impl(int n, const int64_t* n_dev, int end_bit, const K* keys_in,
     const size_t row = (size_t)kRadix * p.blocks;  // counts of one pass
     if (direct) {
         launch_chained(radix_hist_kernel<K>, p.blocks, kSortThreads, 0, stream, ksrc, n, p.chunk, n_dev, first_bit,
-                                                                    (1u << std::min(digit, end_bit)) - 1u, hist, passes);
+                       (1u << std::min(digit, end_bit)) - 1u, hist, passes);
     }
     for (int pass = 0; pass < passes; pass++) {
         const bool to_out = ((passes - 1 - pass) % 2) == 0;
@@ -873,26 +873,23 @@ static int sort_impl(int n, const int64_t* n_dev, int end_bit, const K* keys_in,
                              : dbits == 7 ? radix_scatter_kernel<K, 7, true, VALS> : radix_scatter_kernel<K, 8, true, VALS>;
                 cudaError_t e = cudaFuncSetAttribute(scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
                 if (e != cudaSuccess) { set_cuda_error(e, "sort_pairs"); return GSTEX_ERR_CUDA; }
-                launch_chained(scatter, p.blocks, kSortThreads, smem, stream,
-                               ksrc, vsrc, kdst, vdst, n, p.chunk, n_dev, shift, dbits,
-                                                                  hist + pass * row, nullptr,
-                                                                  left > 0 ? hist + (pass + 1) * row : nullptr, next_mask);
+                launch_chained(scatter, p.blocks, kSortThreads, smem, stream, ksrc, vsrc, kdst, vdst, n, p.chunk,
+                               n_dev, shift, dbits, hist + pass * row, nullptr,
+                               left > 0 ? hist + (pass + 1) * row : nullptr, next_mask);
             }
             ksrc = kdst;
             vsrc = vdst;
             continue;
         }
-        launch_chained(radix_hist_kernel<K>, p.blocks, kSortThreads, 0, stream,
-                       ksrc, n, p.chunk, n_dev, shift, (1u << dbits) - 1u,
-                                                                    hist, 0);
+        launch_chained(radix_hist_kernel<K>, p.blocks, kSortThreads, 0, stream, ksrc, n, p.chunk, n_dev, shift,
+                       (1u << dbits) - 1u, hist, 0);
         launch_chained(radix_scan_rows_kernel, kRadix, kSortThreads, 0, stream, hist, p.blocks, totals);
         auto scatter = dbits <= 5 ? radix_scatter_kernel<K, 5, false, VALS> : dbits == 6 ? radix_scatter_kernel<K, 6, false, VALS>
                      : dbits == 7 ? radix_scatter_kernel<K, 7, false, VALS> : radix_scatter_kernel<K, 8, false, VALS>;
         cudaError_t e = cudaFuncSetAttribute(scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) { set_cuda_error(e, "sort_pairs"); return GSTEX_ERR_CUDA; }
-        launch_chained(scatter, p.blocks, kSortThreads, smem, stream,
-                       ksrc, vsrc, kdst, vdst, n, p.chunk, n_dev, shift, dbits,
-                                                          hist, totals, nullptr, 0u);
+        launch_chained(scatter, p.blocks, kSortThreads, smem, stream, ksrc, vsrc, kdst, vdst, n, p.chunk, n_dev, shift,
+                       dbits, hist, totals, nullptr, 0u);
         ksrc = kdst;
         vsrc = vdst;
     }
@@ -928,9 +925,8 @@ extern "C" int gstex_get_tile_bin_edges(int num_isect, const int64_t* sorted, in
     if (e != cudaSuccess) { set_cuda_error(e, "tile_bin_edges memset"); return GSTEX_ERR_CUDA; }
     if (num_isect == 0) return GSTEX_OK;
     GSTEX_REQUIRE(sorted);
-    launch_chained(bin_edges_kernel<int64_t>, ceil_div(num_isect, 256 * kEdgeItems), 256, 0, stream,
-                   num_isect, nullptr, sorted, 32,
-                                                                             num_tiles, (int2*)bins, nullptr, 0u);
+    launch_chained(bin_edges_kernel<int64_t>, ceil_div(num_isect, 256 * kEdgeItems), 256, 0, stream, num_isect,
+                   nullptr, sorted, 32, num_tiles, (int2*)bins, nullptr, 0u);
     return check_launch("get_tile_bin_edges");
 }
 
@@ -942,9 +938,8 @@ extern "C" int gstex_get_tile_bin_edges_dyn(int capacity, const int64_t* count, 
     if (e != cudaSuccess) { set_cuda_error(e, "tile_bin_edges memset"); return GSTEX_ERR_CUDA; }
     if (capacity == 0) return GSTEX_OK;
     GSTEX_REQUIRE(sorted);
-    launch_chained(bin_edges_kernel<int64_t>, ceil_div(capacity, 256 * kEdgeItems), 256, 0, stream,
-                   capacity, count, sorted, 32, num_tiles,
-                                                                            (int2*)bins, nullptr, 0u);
+    launch_chained(bin_edges_kernel<int64_t>, ceil_div(capacity, 256 * kEdgeItems), 256, 0, stream, capacity, count,
+                   sorted, 32, num_tiles, (int2*)bins, nullptr, 0u);
     return check_launch("get_tile_bin_edges_dyn");
 }
 
@@ -956,9 +951,8 @@ extern "C" int gstex_get_tile_bin_edges32_dyn(int capacity, const int64_t* count
     if (e != cudaSuccess) { set_cuda_error(e, "tile_bin_edges32 memset"); return GSTEX_ERR_CUDA; }
     if (capacity == 0) return GSTEX_OK;
     GSTEX_REQUIRE(sorted);
-    launch_chained(bin_edges_kernel<uint32_t>, ceil_div(capacity, 256 * kEdgeItems), 256, 0, stream,
-                   capacity, count, sorted, shift, num_tiles,
-                                                                             (int2*)bins, nullptr, 0u);
+    launch_chained(bin_edges_kernel<uint32_t>, ceil_div(capacity, 256 * kEdgeItems), 256, 0, stream, capacity, count,
+                   sorted, shift, num_tiles, (int2*)bins, nullptr, 0u);
     return check_launch("get_tile_bin_edges32_dyn");
 }
 
@@ -1058,8 +1052,9 @@ extern "C" int gstex_view_bins(int n, int num_isect, const float* centers, const
                                              sort_bytes, stream, id_bits)
                 : sort_impl<uint32_t>(num_isect, nullptr, end_bit, keys, vals, sorted, gids, w + 3 * a, sort_bytes, stream);
     if (rc) return rc;
-    launch_chained(bin_edges_kernel<uint32_t>, ceil_div(num_isect, 256 * kEdgeItems), 256, 0, stream, num_isect, nullptr,
-                   sorted, id_bits + 1, num_tiles, (int2*)bins, packed ? gids : nullptr, (1u << id_bits) - 1u);
+    launch_chained(bin_edges_kernel<uint32_t>, ceil_div(num_isect, 256 * kEdgeItems), 256, 0, stream, num_isect,
+                   nullptr, sorted, id_bits + 1, num_tiles, (int2*)bins, packed ? gids : nullptr,
+                   (1u << id_bits) - 1u);
     return check_launch("view_bins");
 }
 
@@ -1072,7 +1067,7 @@ extern "C" int gstex_batch_tile_order_small(int num_groups, const int32_t* group
     cudaError_t e = cudaFuncSetAttribute(tile_order_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)sizeof(SmallSort));
     if (e != cudaSuccess) { set_cuda_error(e, "batch_tile_order"); return GSTEX_ERR_CUDA; }
-    launch_chained(tile_order_small_kernel, 1, kSmallThreads, sizeof(SmallSort), (cudaStream_t)s, 
-        num_groups, (const int4*)groups, (const int2*)tile_bins, order);
+    launch_chained(tile_order_small_kernel, 1, kSmallThreads, sizeof(SmallSort), (cudaStream_t)s, num_groups,
+                   (const int4*)groups, (const int2*)tile_bins, order);
     return check_launch("batch_tile_order");
 }

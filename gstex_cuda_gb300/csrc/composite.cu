@@ -560,7 +560,7 @@ __global__ void __launch_bounds__(32 * kBlockWarps, kFwdCtas)
 // reduction by shuffles and 8-lane groups) the scan, staging and ray-plane
 // solves take 6 ms, the adjoint 4, texel reads 3.5, texel atomics 4 and the
 // sums 5.  8 clustered full-HD views: 22.3 -> 13.2 ms; one 800x800 view of 1x1
-// charts 254 -> 108 us; one full-HD view of large splats 36.0 -> 6.9 ms (where
+// charts 254 -> 108 us; one full-HD view of large splats 36.0 -> 7.0 ms (where
 // the list walk also staged every splat behind the last contributor).  The
 // pixels' upstream gradients by shuffles instead of from shared memory in the
 // sums: 23.7 ms.

@@ -239,15 +239,17 @@ def _texture_mode(texture, channels):
     raise _lib.GstexError(f"texture must be float32 or bfloat16, got {texture.dtype}")
 
 
+# The next two shape the tile kernels' launches; calls that the block kernels
+# take (gstex_block_kernels: with PREBUILT_RECORDS the usual ones) have no knobs.
 PIXELS_PER_THREAD = 1  # 1 or 2 (2 halves the threads per tile; even block widths only)
 # Lanes that walk one list of staged splats in texture_backward: 32 (a
 # warp's 8x4 pixel block), 16 (4x4), 8 (4x2) or 4 (2x2); below 32 only for
 # block widths that are multiples of 8, one pixel per thread and 0 or 3
-# channels (else 32).  8 measured fastest on the benchmark scenes.
+# channels (else 32).
 BACKWARD_GROUP_LANES = 8
 # texture_forward / texture_backward build one splat record per Gaussian of the
-# view first (gstex_view_records) and the tiles copy them; False: every tile
-# derives the records of its Gaussians itself.
+# view first (gstex_view_records), which the block kernels need and the tile
+# kernels copy; False: every tile derives the records of its Gaussians itself.
 PREBUILT_RECORDS = True
 
 

@@ -142,7 +142,8 @@ int gstex_get_tile_bin_edges_dyn(int capacity, const int64_t* count, const int64
 /* Stable LSD radix sort of (uint32 key, int32 value) pairs on key bits
  * [0, end_bit); with count non-NULL the number of items is read from device
  * memory (clamped to n) and the call can be captured in a CUDA graph.
- * Workspace: gstex_sort32_workspace_bytes(n).  The two sorts of the
+ * Workspace: gstex_sort32_workspace_bytes(n) (as of the other sorts and of
+ * view binning: never less than for a smaller n).  The two sorts of the
  * depth-first batched binning, which together replace the 64-bit sort of
  * bin_and_sort_gaussians (gstex_cuda/utils.py:159-160). */
 size_t gstex_sort32_workspace_bytes(int n);
