@@ -77,6 +77,7 @@ _SIGS = {
     "gstex_chart_texels": (_I, [_I, _P, _P, _P]),
     "gstex_texture_forward": (_I, [ctypes.POINTER(RasterInputs), ctypes.POINTER(ForwardOutputs), _P]),
     "gstex_texture_edit": (_I, [ctypes.POINTER(RasterInputs), ctypes.POINTER(EditIO), _P]),
+    "gstex_texture_edit_records": (_I, [ctypes.POINTER(RasterInputs), ctypes.POINTER(EditIO), _P, _P]),
     "gstex_preprocess_forward": (_I, [_I, _I] + [_P] * 10 + [_P]),
     "gstex_preprocess_backward": (_I, [_I, _I] + [_P] * 14 + [_P]),
     "gstex_backward_workspace_bytes": (ctypes.c_size_t, [_I]),

@@ -1558,7 +1558,7 @@ extern "C" int gstex_texture_forward(const gstex_raster_inputs* in, const gstex_
     return check_launch("texture_forward");
 }
 
-extern "C" int gstex_texture_edit(const gstex_raster_inputs* in, const gstex_edit_io* io, gstex_stream_t s) {
+static int edit_impl(const gstex_raster_inputs* in, const gstex_edit_io* io, const void* records, gstex_stream_t s) {
     GSTEX_REQUIRE(in && io);
     GSTEX_REQUIRE(in->num_points >= 0 && in->img_width > 0 && in->img_height > 0);
     GSTEX_REQUIRE(in->block_width >= 2 && in->block_width <= kMaxBlockWidth);
@@ -1600,9 +1600,8 @@ extern "C" int gstex_texture_edit(const gstex_raster_inputs* in, const gstex_edi
     va.bins = (const int2*)in->tile_bins;
     EditIO E{ (const float3*)io->updated_img, io->updated_alpha, io->depth_lower, io->depth_upper,
               io->updated_texture };
-    if ((bw & 7) == 0 && in->records) {
-        GSTEX_REQUIRE(((uintptr_t)in->records & 15) == 0);
-        va.recs = (const RecAll*)in->records;
+    if ((bw & 7) == 0 && records) {
+        va.recs = (const RecAll*)records;
         a.settings = (in->settings & 1) << 9;  // the walk's blur bit
         return launch_edit_blocks(a, block_args(va, bw, a.N), E, stream);
     }
@@ -1611,6 +1610,18 @@ extern "C" int gstex_texture_edit(const gstex_raster_inputs* in, const gstex_edi
     if (rc) return rc;
     edit_view_kernel<1><<<dim3(va.tiles_x, ceil_div(va.H, bw)), dim3(bw, bw), smem, stream>>>(a, va, E);
     return check_launch("texture_edit");
+}
+
+// (in->records, which the renderer's calls read, are not editing's: they may have
+// been built for another blur)
+extern "C" int gstex_texture_edit(const gstex_raster_inputs* in, const gstex_edit_io* io, gstex_stream_t s) {
+    return edit_impl(in, io, nullptr, s);
+}
+
+extern "C" int gstex_texture_edit_records(const gstex_raster_inputs* in, const gstex_edit_io* io, const void* records,
+                                          gstex_stream_t s) {
+    GSTEX_REQUIRE(((uintptr_t)records & 15) == 0);
+    return edit_impl(in, io, records, s);
 }
 
 extern "C" size_t gstex_backward_workspace_bytes(int num_points) {

@@ -461,8 +461,8 @@ def texture_edit(tile_bounds, block, img_size, texture_info, texture_total_size,
         rr.channels, rr.num_texels, rr.colors, rr.background = 0, 0, ptr(means), ptr(means)
         rr.settings = (int(settings) & 1) << 9
         recs = _attach_records(rr, means.device)  # (alive until the launch is queued)
-        ri.records = ptr(recs)
     out = torch.empty((T, 5), dtype=torch.float32, device=means.device)
     io = _lib.EditIO(ptr(updated_img), ptr(updated_alpha), ptr(depth_lower), ptr(depth_upper), T, ptr(out))
-    check(_lib.lib().gstex_texture_edit(ctypes.byref(ri), ctypes.byref(io), _lib.stream_of(means)), "texture_edit")
+    check(_lib.lib().gstex_texture_edit_records(ctypes.byref(ri), ctypes.byref(io), ptr(recs), _lib.stream_of(means)),
+          "texture_edit")
     return out

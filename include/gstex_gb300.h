@@ -211,7 +211,8 @@ typedef struct gstex_raster_inputs {
      * of its Gaussians itself.  With records, a block width that is a multiple
      * of 8, 0 or 3 channels and without alpha visualisation the compositor
      * runs one warp per 8x4 pixels, to which pixels_per_thread and
-     * group_lanes do not apply. */
+     * group_lanes do not apply.  Read by texture_forward / texture_backward,
+     * not by texture_edit. */
     const void* records;
     /* texture_backward: lanes that walk one list of staged splats, 32 (a
      * warp's 8x4 pixel block), 16 (4x4), 8 (4x2) or 4 (2x2); 0 = 32.  Values
@@ -262,9 +263,16 @@ typedef struct gstex_edit_io {
 
 /* Replaces _C.texture_edit (csrc/texture_edit.cu:238-346): in->channels must
  * be 5 (texture_info[2]; the reference writes five channels at that stride),
- * in->colors / in->texture / in->background are not read, blur is settings
- * bit 0. */
+ * in->colors / in->texture / in->background / in->records are not read, blur
+ * is settings bit 0. */
 int gstex_texture_edit(const gstex_raster_inputs* in, const gstex_edit_io* io, gstex_stream_t stream);
+/* The same on records of the view (16-byte aligned; NULL: none), which for block
+ * widths that are multiples of 8 runs one warp per 8x4 pixels.  They are built
+ * by gstex_view_records from inputs of the same scene and camera, whose settings
+ * have the blur of this call in bit 9 and alpha visualisation off; colours and
+ * texture do not matter. */
+int gstex_texture_edit_records(const gstex_raster_inputs* in, const gstex_edit_io* io, const void* records,
+                               gstex_stream_t stream);
 
 typedef struct gstex_backward_io {
     /* saved forward state */
