@@ -159,7 +159,6 @@ def unobserved() -> bool:
     try:
         return (torch.autograd.forward_ad._current_level < 0
                 and torch._C._functorch.peek_interpreter_stack() is None and torch._C._get_tracing_state() is None
-                and not torch.compiler.is_compiling()
                 and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0)
     except AttributeError:
         return False
@@ -170,6 +169,8 @@ def plain_cuda_f32(*tensors) -> bool:
     tensors: float32 CUDA tensors of the current device, whose memory holds
     their values, that no gradient, forward-mode tangent, functional transform,
     tracer, compiler or dispatch mode looks at, with products in full float32."""
+    if torch.compiler.is_compiling():  # (first, and alone: a compiler reads this function, too)
+        return False
     grad = torch.is_grad_enabled()
     for t in tensors:
         if type(t) not in (torch.Tensor, torch.nn.Parameter) or not t.is_cuda or t.dtype is not torch.float32 \
