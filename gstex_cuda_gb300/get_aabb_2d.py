@@ -19,7 +19,7 @@ def project_points(points, viewmat, intrins, clip=False):
     """Pixel positions and camera depths of points (gstex_cuda/get_aabb_2d.py:22-32).
     The depths are the per-Gaussian sort keys of the binning stage."""
     if not clip and _lib.plain_cuda_f32(points, viewmat) and points.ndim == 2 and points.shape[-1] == 3 \
-            and viewmat.shape == (4, 4) and all(type(x) in (int, float) for x in intrins) \
+            and viewmat.shape == (4, 4) and len(intrins) == 4 and all(type(x) in (int, float) for x in intrins) \
             and points.device == viewmat.device:
         return _C.project_points(points.detach().contiguous(), viewmat.detach().contiguous(), *intrins)
     view_points = points @ viewmat.T[:3, :3] + viewmat.T[3:, :3]

@@ -56,3 +56,16 @@ def test_points_that_are_stored_negated(n):
     assert torch.allclose(depth, wdepth, rtol=1e-6, atol=1e-6) and torch.allclose(pix, want, rtol=1e-4)
     _, moved = project_points(p, torch._neg_view(-vm), INTR)
     assert torch.allclose(moved, -wdepth, rtol=1e-6, atol=1e-6)
+
+
+@pytest.mark.parametrize("intrinsics", [INTR[:3], INTR[:2], INTR + (1.0,)])
+def test_wrong_numbers_of_intrinsics(intrinsics):
+    """Refused with the error of the torch operations."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from gstex_cuda_gb300.get_aabb_2d import project_points
+    p, vm = torch.randn(20, 3, device=DEV), torch.eye(4, device=DEV)
+    with pytest.raises(ValueError):
+        project_points(p.requires_grad_(), vm, intrinsics)
+    with pytest.raises(ValueError):
+        project_points(p.detach(), vm, intrinsics)
