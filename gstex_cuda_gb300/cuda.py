@@ -288,14 +288,15 @@ def _raster_inputs(img_w, img_h, bw, texture_info, texture_dims, gaussian_ids_so
     return ri, C
 
 
-def _attach_records(ri, device):
+def _attach_records(ri, num_points, device):
     """Builds the view's splat records into a fresh buffer and points `ri` at
     it; returns the buffer (kept alive by the caller until the launch is
-    queued)."""
-    if not PREBUILT_RECORDS or ri.num_points == 0:
+    queued).  (No field of `ri` is read back: torch.compile takes such a read
+    for one of the structure's class.)"""
+    if not PREBUILT_RECORDS or num_points == 0:
         return None
     L = _lib.lib()
-    nb = L.gstex_view_records_bytes(ri.num_points)
+    nb = L.gstex_view_records_bytes(num_points)
     buf = torch.empty(nb, dtype=torch.uint8, device=device)
     check(L.gstex_view_records(ctypes.byref(ri), ptr(buf), nb, _lib.stream_of(buf)), "view_records")
     ri.records = ptr(buf)
@@ -337,7 +338,7 @@ def forward_with_records(tile_bounds, block, img_size, texture_info, texture_dim
     reg_s = torch.empty((H, W, 3), **f32)
     fo = _lib.ForwardOutputs(ptr(out_img), ptr(out_depth), ptr(out_reg), ptr(out_tex), ptr(out_normal), ptr(final_T),
                              ptr(final_idx), ptr(depth_idx), ptr(reg_s))
-    recs = _attach_records(ri, dev)
+    recs = _attach_records(ri, means.shape[0], dev)
     check(_lib.lib().gstex_texture_forward(ctypes.byref(ri), ctypes.byref(fo), _lib.stream_of(means)),
           "texture_forward")
     return (out_img, out_depth, out_reg, out_tex, out_normal, final_T, final_idx, depth_idx, reg_s), recs
@@ -369,7 +370,7 @@ def texture_backward(img_height, img_width, block_width, texture_info, texture_d
     v_uv0 = torch.empty(uv0.shape, dtype=torch.float32, device=dev)
     v_umap = torch.empty(umap.shape, dtype=torch.float32, device=dev)
     v_vmap = torch.empty(vmap.shape, dtype=torch.float32, device=dev)
-    tex_cols = 4 if ri.texture_dtype == TEXTURE_BF16X4 else C
+    tex_cols = 4 if texture.dtype == torch.bfloat16 else C
     v_texture = torch.zeros((texture.shape[0], tex_cols), dtype=torch.float32, device=dev)
     wsb = L.gstex_backward_workspace_bytes(N)
     ws = torch.empty(wsb, dtype=torch.uint8, device=dev)
@@ -378,7 +379,7 @@ def texture_backward(img_height, img_width, block_width, texture_info, texture_d
                           ptr(v_output_normal), ptr(v_colors), ptr(v_opacity), ptr(v_means), ptr(v_scales),
                           ptr(v_quats), ptr(v_uv0), ptr(v_umap), ptr(v_vmap), ptr(v_texture), ptr(ws), wsb)
     if records is None:
-        records = _attach_records(ri, dev)  # (alive until the launch is queued)
+        records = _attach_records(ri, N, dev)  # (alive until the launch is queued)
     else:
         ri.records = ptr(records)
     check(L.gstex_texture_backward(ctypes.byref(ri), ctypes.byref(bio), _lib.stream_of(means)), "texture_backward")
@@ -454,13 +455,13 @@ def texture_edit(tile_bounds, block, img_size, texture_info, texture_total_size,
     ri.fx, ri.fy, ri.cx, ri.cy = float(fx), float(fy), float(cx), float(cy)
     ri.settings = int(settings)
     recs = None
-    if PREBUILT_RECORDS and ri.num_points > 0 and ri.block_width in (8, 16):
+    if PREBUILT_RECORDS and means.shape[0] > 0 and int(block[0]) in (8, 16):
         # the records of the forward walk with editing's blur bit (0) in the
         # renderer's place (9); their colours are not read
         rr = _lib.RasterInputs.from_buffer_copy(ri)
         rr.channels, rr.num_texels, rr.colors, rr.background = 0, 0, ptr(means), ptr(means)
         rr.settings = (int(settings) & 1) << 9
-        recs = _attach_records(rr, means.device)  # (alive until the launch is queued)
+        recs = _attach_records(rr, means.shape[0], means.device)  # (alive until the launch is queued)
     out = torch.empty((T, 5), dtype=torch.float32, device=means.device)
     io = _lib.EditIO(ptr(updated_img), ptr(updated_alpha), ptr(depth_lower), ptr(depth_upper), T, ptr(out))
     check(_lib.lib().gstex_texture_edit_records(ctypes.byref(ri), ctypes.byref(io), ptr(recs), _lib.stream_of(means)),
