@@ -67,6 +67,9 @@ __device__ __forceinline__ float4 quat_axes_vjp(float4 q, float3 c0, float3 c1, 
 }
 
 __device__ __forceinline__ float dot3(float3 a, float3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+__device__ __forceinline__ float3 cross3(float3 a, float3 b) {
+    return make_float3(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x);
+}
 __device__ __forceinline__ float3 operator*(float s, float3 a) { return make_float3(s * a.x, s * a.y, s * a.z); }
 __device__ __forceinline__ float3 operator+(float3 a, float3 b) { return make_float3(a.x + b.x, a.y + b.y, a.z + b.z); }
 __device__ __forceinline__ float3 operator-(float3 a, float3 b) { return make_float3(a.x - b.x, a.y - b.y, a.z - b.z); }
@@ -122,7 +125,8 @@ __device__ __forceinline__ View load_view(const float* viewmat, float fx, float 
 // The record also carries a conservative screen box of the region where the
 // splat can reach alpha >= 1/255: sigma <= ln(255 * opacity) is an ellipse
 // in the splat plane, inside the rectangle +-a*s1*ax1 +-a*s2*ax2 with
-// a = sqrt(2 ln(255 opacity)) (inflated slightly); when all four corners are
+// a = sqrt(2 ln(255 opacity)) (inflated slightly; a parallelogram for a
+// quaternion that is not of unit length); when all four corners are
 // in front of the camera the projected rectangle, hence the box of its
 // projected corners, contains every pixel whose ray meets the ellipse.  A
 // pixel outside the box is a pixel the reference skips (alpha < 1/255).
@@ -294,7 +298,7 @@ __device__ __forceinline__ RecCull cull_box(float x0, float x1, float y0, float 
                      false);
 }
 
-// Image of the plane ellipse mu + e1 cos(t) a1 + e2 sin(t) a2.  With u_i the
+// Image of the plane ellipse mu + e1 cos(t) a1 + e2 sin(t) a2 (for any two a).  With u_i the
 // homogeneous images of the axes relative to the projected centre (px0, py0),
 // its tangent lines satisfy l^T D l = 0, D = e1^2 u1 u1^T + e2^2 u2 u2^T -
 // u0 u0^T, u0 = (0, 0, z); scaled to D_zz = -1, D is [S - c c^T, -c; -c^T, -1]
@@ -376,12 +380,19 @@ __device__ __forceinline__ bool make_record(RecHot& H, RecWarm& Wm, RecCold& Cd,
     if (smax > 0.f) {
         const float a = sqrtf(2.f * smax + 1e-3f) * 1.002f;
         const float e1 = a / is1, e2 = a / is2;
-        bool front = !flags;
+        // The point of the plane with l_k = a_k . delta is delta = l1 b1 + l2 b2, where b is
+        // dual to a in the plane.  b_k = a_k for a rotation; the axes of a quaternion that
+        // is not of unit length are oblique.
+        float3 b1 = cross3(a2c, nc), b2 = cross3(nc, a1c);
+        const float det = dot3(a1c, b1), idet = 1.f / det;
+        b1 = idet * b1;
+        b2 = idet * b2;
+        bool front = !flags && fabsf(det) > 1e-6f;
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             const float s1 = (k & 1) ? -e1 : e1, s2 = (k & 2) ? -e2 : e2;
-            const float3 c = make_float3(mc.x + s1 * a1c.x + s2 * a2c.x, mc.y + s1 * a1c.y + s2 * a2c.y,
-                                         mc.z + s1 * a1c.z + s2 * a2c.z);
+            const float3 c = make_float3(mc.x + s1 * b1.x + s2 * b2.x, mc.y + s1 * b1.y + s2 * b2.y,
+                                         mc.z + s1 * b1.z + s2 * b2.z);
             front = front && c.z > 1e-3f;
             const float iz = 1.f / c.z;
             const float px = V.fx * c.x * iz + V.cx, py = V.fy * c.y * iz + V.cy;
@@ -391,7 +402,7 @@ __device__ __forceinline__ bool make_record(RecHot& H, RecWarm& Wm, RecCold& Cd,
         if (front) {
             const float mx = 1e-2f + 1e-5f * (fabsf(x0) + fabsf(x1)), my = 1e-2f + 1e-5f * (fabsf(y0) + fabsf(y1));
             x0 -= mx; x1 += mx; y0 -= my; y1 += my;
-            if (E && !use_blur && cull) oval = cull_ellipse(*E, V, mc, mc.x / mc.z, mc.y / mc.z, a1c, a2c, e1, e2);
+            if (E && !use_blur && cull) oval = cull_ellipse(*E, V, mc, mc.x / mc.z, mc.y / mc.z, b1, b2, e1, e2);
         } else {
             x0 = y0 = -INFINITY;
             x1 = y1 = INFINITY;
