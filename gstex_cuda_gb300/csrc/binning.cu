@@ -15,7 +15,7 @@ __global__ void emit_kernel(int n, int num_isect, const float2* __restrict__ cen
                             int64_t* __restrict__ keys, int32_t* __restrict__ gids) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const int lo = i == 0 ? 0 : cum[i - 1];
+    const int lo = i == 0 ? 0 : max(cum[i - 1], 0);  // (sums of counts below 0 are, too)
     const int hi = min(cum[i], num_isect);
     int cur = lo;
     const float2 e = extents[i];
