@@ -448,11 +448,12 @@ __global__ void depth_keys_kernel(int n, const float* __restrict__ depths, const
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint32_t k = __float_as_uint(depths[i]);
-    const bool hit = counts[i] > 0;
-    keys[i] = hit ? k : 0xffffffffu;
+    const int count = counts[i];
+    keys[i] = count > 0 ? k : 0xffffffffu;
     ids[i] = i;
-    // a depth of +0 ties with the zero entries, whose order is then their slots'
-    if (hit && k == 0u) info[1] = 1;
+    // a depth of +0 ties with the zero entries, whose order is then their slots';
+    // behind a count below 0 slots overlap
+    if (count < 0 || (count > 0 && k == 0u)) info[1] = 1;
 }
 
 // Key and Gaussian of slot u of the Gaussian gi, whose tile rectangle is
@@ -664,10 +665,10 @@ __global__ void __launch_bounds__(kSmallThreads) view_order_small_kernel(int n, 
     bool zero = false;
     for (int i = threadIdx.x; i < n; i += kSmallThreads) {
         const uint32_t k = __float_as_uint(depths[i]);
-        const bool hit = counts[i] > 0;
-        S.key[0][i] = hit ? k : 0xffffffffu;
+        const int count = counts[i];
+        S.key[0][i] = count > 0 ? k : 0xffffffffu;
         S.val[0][i] = (uint32_t)i;
-        zero = zero || (hit && k == 0u);
+        zero = zero || count < 0 || (count > 0 && k == 0u);
     }
     const int any_zero = __syncthreads_or(zero);
     const int at = small_sort(S, n, 32);

@@ -207,7 +207,7 @@ def bin_view(centers, extents, depths, num_tiles_hit, tile_bounds, block_width, 
     if total >= 2 ** 31:
         raise OverflowError(f"{total} intersections exceed the int32 range of the reference's cumsum")
     num_tiles = int(tile_bounds[0]) * int(tile_bounds[1])
-    # depths of +0 have the order of the 64-bit keys; 2^30 tiles or more no 32-bit keys
+    # depths of +0 and overlapping slots have the order of the 64-bit keys; 2^30 tiles or more no 32-bit keys
     if total > 0 and (ties or num_tiles >= 2 ** 30):
         cum, _ = inclusive_scan(num_tiles_hit)
         keys, ids = map_gaussian_to_intersects(n, total, centers, extents, depths, cum, tile_bounds, block_width)

@@ -161,7 +161,8 @@ int gstex_get_tile_bin_edges32_dyn(int capacity, const int64_t* count, const uin
  *   1. gstex_view_order: the Gaussians in (stable) depth order, the inclusive
  *      sums of their tile counts in that order, and info[0] = their total,
  *      info[1] = 1 if a Gaussian with tiles has depth +0 (such depths tie with
- *      the zero entries of unwritten slots: sort 64-bit keys instead);
+ *      the zero entries of unwritten slots) or a count is below 0 (slots
+ *      overlap): sort 64-bit keys instead;
  *   2. the caller reads info (the total sizes the next step's buffers);
  *   3. gstex_view_bins: emission in that order, a stable sort by tile, ranges.
  * Workspaces 16-byte aligned. */
