@@ -125,58 +125,68 @@ def ptr(t) -> int | None:
     return t.data_ptr()
 
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)  # (without a Stream object)
+
+
 def stream_of(t: torch.Tensor):
     """Handle of the current torch stream on t's device."""
     if not t.is_cuda:
         raise GstexError("gstex_cuda_gb300 operators need CUDA tensors (no CPU implementation)")
-    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)  # (torch's own, without a Stream object)
-    return raw(t.get_device()) if raw is not None else torch.cuda.current_stream(t.device).cuda_stream
+    return torch.cuda.current_stream(t.device).cuda_stream if _raw_stream is None else _raw_stream(t.get_device())
 
 
-def on_current_device(*tensors) -> bool:
-    """Whether the tensors are on the current CUDA device, the one a kernel
-    launch goes to (a torch operation goes to its tensors')."""
-    current = torch.cuda.current_device()
-    for t in tensors:
-        if t.get_device() != current:
-            return False
-    return True
+# Looked up once: a call of project_points takes 50 us of host time with these
+# names bound and one function, 53 with look-ups and a function for every question.
+_is_compiling = torch.compiler.is_compiling
+_current_device = torch.cuda.current_device
+_autocast, _precision = torch.is_autocast_enabled, torch.get_float32_matmul_precision
+_forward_ad = torch.autograd.forward_ad
 
 
-def full_f32_products() -> bool:
-    """Whether torch's float32 matrix products are full float32: no autocast,
-    no reduced precision of products (which raises if it was set through both
-    of torch's interfaces)."""
+def private_questions(c=torch._C):
+    """What only torch's private names tell: the innermost functional transform,
+    the tracer, and the numbers of dispatch and function modes.  None without one
+    of the names, and then something is taken to look."""
     try:
-        return not torch.is_autocast_enabled("cuda") and torch.get_float32_matmul_precision() == "highest"
-    except RuntimeError:
-        return False
-
-
-def unobserved() -> bool:
-    """Whether nothing looks at torch operations as they are called.  A torch
-    that has no answer under these (partly its own) names is taken to look."""
-    try:
-        return (torch.autograd.forward_ad._current_level < 0
-                and torch._C._functorch.peek_interpreter_stack() is None and torch._C._get_tracing_state() is None
-                and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0)
+        if not isinstance(_forward_ad._current_level, int):
+            return None
+        return (c._functorch.peek_interpreter_stack, c._get_tracing_state, c._len_torch_dispatch_stack,
+                c._len_torch_function_stack)
     except AttributeError:
-        return False
+        return None
+
+
+_questions = private_questions()
 
 
 def plain_cuda_f32(*tensors) -> bool:
-    """Whether a kernel launch can stand for torch operations on these
-    tensors: float32 CUDA tensors of the current device, whose memory holds
-    their values, that no gradient, forward-mode tangent, functional transform,
-    tracer, compiler or dispatch mode looks at, with products in full float32."""
-    if torch.compiler.is_compiling():  # (first, and alone: a compiler reads this function, too)
+    """Whether a kernel launch can stand for torch operations on these tensors:
+
+    - float32 CUDA tensors whose memory holds their values, on the current
+      device, to which a launch goes (an operation goes to its tensors');
+    - products in full float32: no autocast, no reduced precision of products
+      (which raises if it was set through both of torch's interfaces);
+    - no gradient, forward-mode tangent, functional transform, tracer, compiler
+      or dispatch mode that looks at the operations.
+    """
+    if _is_compiling():  # (first, and alone: a compiler reads this function, too)
         return False
-    grad = torch.is_grad_enabled()
+    if _questions is None:
+        return False
+    device, grad = _current_device(), torch.is_grad_enabled()
     for t in tensors:
         if type(t) not in (torch.Tensor, torch.nn.Parameter) or not t.is_cuda or t.dtype is not torch.float32 \
-                or (grad and t.requires_grad) or t.is_neg() or t.layout is not torch.strided:
+                or (grad and t.requires_grad) or t.get_device() != device or t.is_neg() \
+                or t.layout is not torch.strided:
             return False
-    return on_current_device(*tensors) and full_f32_products() and unobserved()
+    try:
+        if _precision() != "highest" or _autocast("cuda"):
+            return False
+    except RuntimeError:
+        return False
+    transform, tracer, dispatch_modes, function_modes = _questions
+    return (_forward_ad._current_level < 0 and transform() is None and tracer() is None and dispatch_modes() == 0
+            and function_modes() == 0)
 
 
 def require_cuda(*tensors, names=None):
