@@ -623,7 +623,7 @@ __device__ __forceinline__ void add6(float* dst, float2 a01, float a2, float2 b0
 // as 8 + 4 bytes: second figure): full HD with 48 pixels a texel 8.5 -> 7.3 ->
 // 7.0 ms of backward, a 253x187 view 182 -> 150 -> 132 us, four views with less
 // than two pixels a texel 213 -> 209 -> 211 us.
-template <int TM>
+template <int TM, int FIX>
 __device__ __forceinline__ void add_texel_grads(float* __restrict__ v_texgrad, int T, const Bilerp& B, float2 gv01,
                                                 float gv2) {
     if (gv01.x == 0.f && gv01.y == 0.f && gv2 == 0.f) return;
@@ -633,11 +633,15 @@ __device__ __forceinline__ void add_texel_grads(float* __restrict__ v_texgrad, i
 #pragma unroll
     for (int q = 0; q < 4; q += 2) {
         const float w0 = wts[q], w1 = wts[q + 1];
-        // (a corner without weight adds 0 whatever the gradient: the word it shares
-        // may be another chart's texel, and 0 times infinity is not 0)
-        const float2 z = make_float2(0.f, 0.f);
-        const float2 a01 = w0 != 0.f ? mul2(dup2(w0), gv01) : z, b01 = w1 != 0.f ? mul2(dup2(w1), gv01) : z;
-        const float a2 = w0 != 0.f ? w0 * gv2 : 0.f, b2 = w1 != 0.f ? w1 * gv2 : 0.f;
+        float2 a01 = mul2(dup2(w0), gv01), b01 = mul2(dup2(w1), gv01);
+        float a2 = w0 * gv2, b2 = w1 * gv2;
+        if (TM == 0) {
+            // a corner without weight adds 0 whatever the gradient: the word it shares may
+            // be another chart's texel, and 0 times infinity is not 0 (of two bilinear
+            // weights the first is never the only 0)
+            if (!FIX && w0 == 0.f) { a01 = make_float2(0.f, 0.f); a2 = 0.f; }
+            if (w1 == 0.f) { b01 = make_float2(0.f, 0.f); b2 = 0.f; }
+        }
         if (TM == 1) {
             if (w0 != 0.f) atomicAdd(reinterpret_cast<float4*>(v_texgrad) + rows[q], make_float4(a01.x, a01.y, a2, 0.f));
             if (w1 != 0.f)
@@ -706,7 +710,7 @@ __device__ __forceinline__ void pair_adjoint(BwdState<CT>& S, const SceneArgs& a
         const float2 vs = mul2(val, vt);
         v_vis += vs.x + vs.y + val2 * S.vtex[2];
         // (a coarse chart's are summed over the pixels first, but for pairs in the direct form)
-        if (!is_coarse(nop) || H.direct) add_texel_grads<TM>(g.v_texgrad, a.T, B, gv01, gv2);
+        if (!is_coarse(nop) || H.direct) add_texel_grads<TM, FIX>(g.v_texgrad, a.T, B, gv01, gv2);
     }
     float v_alpha = T * v_vis - T * S.vT_run;
     float vT_cur = alpha * v_vis + (1.f - alpha) * S.vT_run;
